@@ -4,21 +4,35 @@
 //
 //  * gep_inner_kernel: A(i,j) = <Q_j, (HQ)_i>, S(i,j) = <Q_j, Q_i> for j <= i,
 //    full CP inner products in FP64 (one CTA per pair).
-//  * gep_solve_kernel (one CTA): S = L L^T, C = L^-1 A L^-T in FP64;
-//    eigenvectors of C by parallel cyclic Jacobi (round-robin ordering,
-//    disjoint rotations per round), first in FP32 in shared memory, then
-//    refined in FP64: the FP32 vectors V are orthonormalised (two
-//    Newton-Schulz steps), C' = V^T C V is formed and FP64 Jacobi sweeps
-//    diagonalise it (quadratic convergence from the FP32 start: two or three
-//    sweeps), the rotations accumulating into V.  Eigenvalues are the
-//    diagonal of C'.  The FP64 stage matters: the vector updates combine
-//    the block with the eigenvectors, and for nearly degenerate states (the
-//    benchmark block has relative gaps of 4e-5) FP32 eigenvectors are off
-//    by ~1e-7 / gap, which moved the updated vectors by 1e-5 against the
-//    reference's FP64 sygvd.  X = L^-T V with unit columns.  Eigenpairs are
-//    returned in ascending order, each eigenvector with its largest-magnitude
-//    entry positive.
-#include <cfloat>
+//  * gep_solve_launch: the generalised eigenproblem as a short sequence of
+//    phases over a workspace in global memory (L2-resident: 160 vectors at
+//    most).  S = L L^T and C = L^-1 A L^-T in FP64; eigenvectors of C by
+//    parallel cyclic Jacobi in FP32, then refined in FP64 by iterations of
+//    matrix products (Ogita and Aishima, Japan J. Indust. Appl. Math. 35
+//    (2018) 1007-1035): with G = V^T V and S = V^T C V,
+//      lambda_i = S_ii / G_ii,
+//      E_ij = (S_ij - lambda_j G_ij) / (lambda_j - lambda_i),  E_ii = (1 - G_ii) / 2,
+//      V <- V + V E,
+//    which squares the error of V each time.  Pairs whose |E_ij| would pass
+//    1e-3 (levels nearly degenerate on the scale of the FP32 error) are first
+//    separated by FP64 Jacobi rotations of those pairs alone, so three
+//    iterations end at the rounding level for any spectrum.  The FP64 stage
+//    matters: the vector updates combine the block with the eigenvectors,
+//    and for nearly degenerate states (the benchmark block has relative gaps
+//    of 4e-5) FP32 eigenvectors are off by ~1e-7 / gap, which moved the
+//    updated vectors by 1e-5 against the reference's FP64 sygvd.  X = L^-T V
+//    with unit columns of V.  Eigenpairs are returned in ascending order, each
+//    eigenvector with its largest-magnitude entry positive.
+//
+// What bounds it: FP64 issues one warp instruction per SM in 17-19 cycles, so
+// FP64 work has to be spread over the SMs and kept to matrix products; the
+// sequential parts (Cholesky, the Jacobi rounds) are chains of barriers.  One
+// CTA that did everything in global memory, with FP64 Jacobi sweeps (and
+// 16-way bank conflicts in the FP32 ones), took 36.0 ms for 144 vectors and
+// 1.36 ms for 40; the phases take 1.6 ms and 0.39 ms.  Of the 1.6 ms the FP32
+// Jacobi rounds are 0.78, the Cholesky 0.28, the three triangular solves 0.21,
+// the rotation replay 0.10 and the twelve matrix products 0.18.
+#include <algorithm>
 
 #include "common.cuh"
 #include "intertwine.cuh"
@@ -27,7 +41,6 @@ namespace mlcp {
 
 namespace {
 constexpr int kPairThreads = 128;
-constexpr int kSolveThreads = 1024;
 }
 
 __global__ void __launch_bounds__(kPairThreads) gep_inner_kernel(GepParams p) {
@@ -81,8 +94,69 @@ __global__ void __launch_bounds__(kPairThreads) gep_inner_kernel(GepParams p) {
   }
 }
 
+namespace {
+
+constexpr int kMaxB = 160;          // vectors of a block (shared memory of the Cholesky phase)
+constexpr int kMaxQ = kMaxB / 32;   // rows per lane of a warp-held column
+constexpr int kJacobiSweeps = 30;
+constexpr int kVRows = 4;           // rows of V per CTA of the rotation replay
+constexpr int kReplay = 8;          // rounds of rotations loaded together
+constexpr double kUnsafe = 1.0e-3;  // pairs with |E_ij| above this are separated by rotations first
+
+// Workspace of the phases (doubles): L, L^T, C, W, V, V', G, S, E [B][B];
+// invd [B]; the FP32 Jacobi's rotations; counters.
+struct GepWork {
+  double *L, *LT, *C, *W, *V, *V2, *G, *S, *E, *invd;
+  float2* rot;  // [sweeps][Bp - 1][Bp / 2] (c, s)
+  int* cnt;     // [0] Jacobi sweeps, [1] unsafe pairs seen
+};
+
+__host__ __device__ inline int gep_pad(int B) { return (B + 1) / 2 * 2; }
+
+__host__ __device__ inline size_t gep_carve(int B, double* base, GepWork* w) {
+  const size_t bb = (size_t)B * B, Bp = gep_pad(B);
+  size_t o = 0;
+  auto take = [&](size_t n) -> double* {
+    double* r = base ? base + o : nullptr;
+    o += n;
+    return r;
+  };
+  w->L = take(bb);
+  w->LT = take(bb);
+  w->C = take(bb);
+  w->W = take(bb);
+  w->V = take(bb);
+  w->V2 = take(bb);
+  w->G = take(bb);
+  w->S = take(bb);
+  w->E = take(bb);
+  w->invd = take(B);
+  w->rot = reinterpret_cast<float2*>(take((size_t)kJacobiSweeps * (Bp - 1) * (Bp / 2)));
+  w->cnt = reinterpret_cast<int*>(take(1));
+  return o;
+}
+
+// Pair k of round `round` of the round-robin schedule over Bp (even)
+// indices: (Bp-1, round) for k = 0, else ((round+k), (round-k)) mod Bp-1,
+// smaller index first.
+__device__ __forceinline__ void robin_pair(int Bp, int round, int k, int* a, int* b) {
+  const int m = Bp - 1;
+  int x, y;
+  if (k == 0) {
+    x = m;
+    y = round;
+  } else {
+    x = round + k;
+    if (x >= m) x -= m;
+    y = round - k;
+    if (y < 0) y += m;
+  }
+  *a = min(x, y);
+  *b = max(x, y);
+}
+
 // Rotation (c, s) zeroing the (p,q) entry of a symmetric 2x2 block.
-__device__ inline void jacobi_rotation(float app, float aqq, float apq, float* c, float* s) {
+__device__ __forceinline__ void jacobi_rotation(float app, float aqq, float apq, float* c, float* s) {
   if (apq == 0.f) {
     *c = 1.f;
     *s = 0.f;
@@ -94,318 +168,534 @@ __device__ inline void jacobi_rotation(float app, float aqq, float apq, float* c
   *s = t * *c;
 }
 
-__global__ void __launch_bounds__(kSolveThreads) gep_solve_kernel(GepParams p) {
-  const int B = p.nbloc;
-  const int Bp = (B + 1) / 2 * 2;  // even size for the round-robin schedule (padding index is inert)
-  const int tid = threadIdx.x, nt = blockDim.x;
-  double* L = p.work;                        // [B][B] Cholesky factor (lower)
-  double* C = L + (size_t)B * B;             // [B][B]
-  double* Wm = C + (size_t)B * B;            // [B][B]
-  double* lam = Wm + (size_t)B * B;          // [B]
-  double* invd = lam + B;                    // [B]
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float* Cf = reinterpret_cast<float*>(smem_raw);  // [Bp][Bp]
-  float* Vf = Cf + (size_t)Bp * Bp;                // [Bp][Bp]
-  float* rc = Vf + (size_t)Bp * Bp;                // [Bp/2] cosines
-  float* rs = rc + Bp / 2;                         // [Bp/2] sines
-  int* pq = reinterpret_cast<int*>(rs + Bp / 2);   // [Bp] pair members
-  __shared__ double red[32];
-  __shared__ int info;
+// ---- Phases.  Each is run by CTA `cta` of `ncta`; a phase boundary is a
+// kernel boundary, or a block barrier when one CTA runs them all. ----
 
-  // ---- S = L L^T (lower triangle of S) ----
+// S = L L^T (lower triangle of S), one CTA, L in shared memory.  Warp 0 forms
+// the next pivot (FP64 square root and division, ~1300 cycles) while the
+// other warps run the trailing update.
+__device__ void phase_cholesky(const GepParams& p, const GepWork& w, unsigned char* smem) {
+  const int B = p.nbloc, tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+  double* L = reinterpret_cast<double*>(smem);  // [B][B] column-major
+  double* inv_s = L + (size_t)B * B;            // [B]
+  __shared__ int info;
   for (int e = tid; e < B * B; e += nt) {
     const int r = e % B, c = e / B;
     L[e] = (r >= c) ? p.S[e] : 0.0;
   }
   if (tid == 0) info = 0;
+  if (tid < 2) w.cnt[tid] = 0;
+  __syncthreads();
+  auto pivot = [&](int j, double d) {
+    if (!(d > 0.0)) {
+      info = j + 1;
+      d = fabs(d) + 1e-300;
+    }
+    const double l = sqrt(d);
+    L[j + (size_t)j * B] = l;
+    inv_s[j] = 1.0 / l;
+  };
+  if (tid == 0) pivot(0, L[0]);
   __syncthreads();
   for (int j = 0; j < B; ++j) {
-    if (tid == 0) {
-      double d = L[j + (size_t)j * B];
-      if (!(d > 0.0)) { info = j + 1; d = fabs(d) + 1e-300; }
-      const double l = sqrt(d);
-      L[j + (size_t)j * B] = l;
-      invd[j] = 1.0 / l;
-    }
-    __syncthreads();
-    const double inv = invd[j];
+    const double inv = inv_s[j];
     for (int i = j + 1 + tid; i < B; i += nt) L[i + (size_t)j * B] *= inv;
     __syncthreads();
-    const int m = B - j - 1;
-    for (int e = tid; e < m * m; e += nt) {
-      const int c = j + 1 + e / m, i = j + 1 + e % m;
-      if (i >= c) L[i + (size_t)c * B] -= L[i + (size_t)j * B] * L[c + (size_t)j * B];
+    if (j + 1 < B) {
+      if (warp == 0) {
+        if (lane == 0) {
+          const double x = L[j + 1 + (size_t)j * B];
+          pivot(j + 1, fma(-x, x, L[j + 1 + (size_t)(j + 1) * B]));
+        }
+      } else {
+        for (int c = j + warp; c < B; c += nw - 1) {
+          const double x = L[c + (size_t)j * B];
+          for (int i = c + lane; i < B; i += 32)
+            if (i != j + 1) L[i + (size_t)c * B] = fma(-L[i + (size_t)j * B], x, L[i + (size_t)c * B]);
+        }
+      }
     }
     __syncthreads();
   }
-  // ---- C = L^-1 A L^-T (A symmetric from its lower triangle) ----
   for (int e = tid; e < B * B; e += nt) {
     const int r = e % B, c = e / B;
-    C[e] = (r >= c) ? p.A[e] : p.A[c + (size_t)r * B];
+    w.L[e] = L[e];
+    w.LT[e] = L[c + (size_t)r * B];
   }
-  __syncthreads();
-  for (int j = 0; j < B; ++j) {  // C <- L^-1 C (rows)
-    for (int c = tid; c < B; c += nt) C[j + (size_t)c * B] *= invd[j];
-    __syncthreads();
-    for (int e = tid; e < (B - j - 1) * B; e += nt) {
-      const int i = j + 1 + e % (B - j - 1), c = e / (B - j - 1);
-      C[i + (size_t)c * B] -= L[i + (size_t)j * B] * C[j + (size_t)c * B];
-    }
-    __syncthreads();
-  }
-  for (int j = 0; j < B; ++j) {  // C <- C L^-T (columns)
-    for (int r = tid; r < B; r += nt) C[r + (size_t)j * B] *= invd[j];
-    __syncthreads();
-    for (int e = tid; e < (B - j - 1) * B; e += nt) {
-      const int c = j + 1 + e / B, r = e % B;
-      C[r + (size_t)c * B] -= C[r + (size_t)j * B] * L[c + (size_t)j * B];
-    }
-    __syncthreads();
-  }
-  // ---- FP32 cyclic Jacobi (round-robin) ----
-  for (int e = tid; e < Bp * Bp; e += nt) {
-    const int r = e % Bp, c = e / Bp;
-    const bool in = r < B && c < B;
-    Cf[e] = in ? (float)(0.5 * (C[r + (size_t)c * B] + C[c + (size_t)r * B])) : 0.f;
-    Vf[e] = (r == c) ? 1.f : 0.f;
-  }
-  __syncthreads();
-  const int npairs = Bp / 2;
-  for (int sweep = 0; sweep < 30; ++sweep) {
-    // convergence: off-diagonal mass relative to the diagonal
-    double off = 0.0, dia = 0.0;
-    for (int e = tid; e < Bp * Bp; e += nt) {
-      const double v = Cf[e];
-      if (e % Bp == e / Bp) dia += v * v; else off += v * v;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      off += __shfl_xor_sync(0xffffffffu, off, o);
-      dia += __shfl_xor_sync(0xffffffffu, dia, o);
-    }
-    __syncthreads();
-    if (tid % 32 == 0) red[tid / 32] = off;
-    __syncthreads();
-    double offt = 0.0;
-    for (int w = 0; w < nt / 32; ++w) offt += red[w];
-    __syncthreads();
-    if (tid % 32 == 0) red[tid / 32] = dia;
-    __syncthreads();
-    double diat = 0.0;
-    for (int w = 0; w < nt / 32; ++w) diat += red[w];
-    __syncthreads();
-    if (offt <= 1e-12 * diat || offt == 0.0) break;
-    for (int round = 0; round < Bp - 1; ++round) {
-      // pair k: (Bp-1, round) for k = 0, else ((round+k) mod (Bp-1), (round-k) mod (Bp-1))
-      for (int k = tid; k < npairs; k += nt) {
-        int a, b;
-        if (k == 0) {
-          a = Bp - 1;
-          b = round;
-        } else {
-          a = (round + k) % (Bp - 1);
-          b = (round - k + (Bp - 1)) % (Bp - 1);
-        }
-        if (a > b) { const int t = a; a = b; b = t; }
-        pq[2 * k] = a;
-        pq[2 * k + 1] = b;
-        jacobi_rotation(Cf[a + (size_t)a * Bp], Cf[b + (size_t)b * Bp], Cf[a + (size_t)b * Bp], &rc[k], &rs[k]);
-      }
-      __syncthreads();
-      // rows: C <- J^T C
-      for (int e = tid; e < npairs * Bp; e += nt) {
-        const int k = e / Bp, col = e % Bp;
-        const int a = pq[2 * k], b = pq[2 * k + 1];
-        const float c = rc[k], s = rs[k];
-        const float xa = Cf[a + (size_t)col * Bp], xb = Cf[b + (size_t)col * Bp];
-        Cf[a + (size_t)col * Bp] = c * xa - s * xb;
-        Cf[b + (size_t)col * Bp] = s * xa + c * xb;
-      }
-      __syncthreads();
-      // columns: C <- C J, V <- V J
-      for (int e = tid; e < npairs * Bp; e += nt) {
-        const int k = e / Bp, row = e % Bp;
-        const int a = pq[2 * k], b = pq[2 * k + 1];
-        const float c = rc[k], s = rs[k];
-        const float xa = Cf[row + (size_t)a * Bp], xb = Cf[row + (size_t)b * Bp];
-        Cf[row + (size_t)a * Bp] = c * xa - s * xb;
-        Cf[row + (size_t)b * Bp] = s * xa + c * xb;
-        const float va = Vf[row + (size_t)a * Bp], vb = Vf[row + (size_t)b * Bp];
-        Vf[row + (size_t)a * Bp] = c * va - s * vb;
-        Vf[row + (size_t)b * Bp] = s * va + c * vb;
-      }
-      __syncthreads();
-    }
-  }
-  // ---- FP64 refinement of the eigenvectors ----
-  double* V = invd + B;              // [B][B] FP64 eigenvectors (columns)
-  double* C2 = V + (size_t)B * B;    // [B][B] V^T C V, diagonalised in place
-  for (int e = tid; e < B * B; e += nt) {
-    const int r = e % B, c = e / B;
-    V[e] = (double)Vf[r + (size_t)c * Bp];
-  }
-  __syncthreads();
-  for (int ns = 0; ns < 2; ++ns) {  // V <- V (3 I - V^T V) / 2
-    for (int e = tid; e < B * B; e += nt) {  // Wm = V^T V
-      const int r = e % B, c = e / B;
-      double acc = 0.0;
-      for (int k = 0; k < B; ++k) acc += V[k + (size_t)r * B] * V[k + (size_t)c * B];
-      Wm[e] = acc;
-    }
-    __syncthreads();
-    for (int e = tid; e < B * B; e += nt) {  // C2 = V (1.5 I - 0.5 Wm)
-      const int r = e % B, c = e / B;
-      double acc = 1.5 * V[r + (size_t)c * B];
-      for (int k = 0; k < B; ++k) acc -= 0.5 * V[r + (size_t)k * B] * Wm[k + (size_t)c * B];
-      C2[e] = acc;
-    }
-    __syncthreads();
-    for (int e = tid; e < B * B; e += nt) V[e] = C2[e];
-    __syncthreads();
-  }
-  for (int e = tid; e < B * B; e += nt) {  // Wm = C V
-    const int r = e % B, c = e / B;
-    double acc = 0.0;
-    for (int k = 0; k < B; ++k) acc += C[r + (size_t)k * B] * V[k + (size_t)c * B];
-    Wm[e] = acc;
-  }
-  __syncthreads();
-  for (int e = tid; e < B * B; e += nt) {  // C2 = V^T C V, symmetrised
-    const int r = e % B, c = e / B;
-    double a1 = 0.0, a2 = 0.0;
-    for (int k = 0; k < B; ++k) {
-      a1 += V[k + (size_t)r * B] * Wm[k + (size_t)c * B];
-      a2 += V[k + (size_t)c * B] * Wm[k + (size_t)r * B];
-    }
-    C2[e] = 0.5 * (a1 + a2);
-  }
-  __syncthreads();
-  const int npB = B / 2;  // pairs of the odd index padding are skipped below
-  for (int sweep = 0; sweep < 12; ++sweep) {
-    double off = 0.0, dia = 0.0;
-    for (int e = tid; e < B * B; e += nt) {
-      const double v = C2[e];
-      if (e % B == e / B) dia += v * v; else off += v * v;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      off += __shfl_xor_sync(0xffffffffu, off, o);
-      dia += __shfl_xor_sync(0xffffffffu, dia, o);
-    }
-    __syncthreads();
-    if (tid % 32 == 0) red[tid / 32] = off;
-    __syncthreads();
-    double offt = 0.0;
-    for (int w = 0; w < nt / 32; ++w) offt += red[w];
-    __syncthreads();
-    if (tid % 32 == 0) red[tid / 32] = dia;
-    __syncthreads();
-    double diat = 0.0;
-    for (int w = 0; w < nt / 32; ++w) diat += red[w];
-    __syncthreads();
-    if (offt <= 1e-30 * diat || offt == 0.0) break;
-    (void)npB;
-    for (int round = 0; round < Bp - 1; ++round) {
-      double* rcd = Wm;           // [Bp/2] cosines (Wm is free until the back substitution)
-      double* rsd = Wm + Bp / 2;  // [Bp/2] sines
-      for (int k = tid; k < npairs; k += nt) {
-        int a, b;
-        if (k == 0) {
-          a = Bp - 1;
-          b = round;
-        } else {
-          a = (round + k) % (Bp - 1);
-          b = (round - k + (Bp - 1)) % (Bp - 1);
-        }
-        if (a > b) { const int t = a; a = b; b = t; }
-        pq[2 * k] = a;
-        pq[2 * k + 1] = b;
-        double c = 1.0, sn = 0.0;
-        if (b < B) {  // index Bp - 1 = B is padding when B is odd
-          const double app = C2[a + (size_t)a * B], aqq = C2[b + (size_t)b * B], apq = C2[a + (size_t)b * B];
-          if (apq != 0.0) {
-            const double theta = (aqq - app) / (2.0 * apq);
-            const double t = copysign(1.0, theta) / (fabs(theta) + sqrt(theta * theta + 1.0));
-            c = 1.0 / sqrt(t * t + 1.0);
-            sn = t * c;
-          }
-        }
-        rcd[k] = c;
-        rsd[k] = sn;
-      }
-      __syncthreads();
-      for (int e = tid; e < npairs * B; e += nt) {  // rows: C2 <- J^T C2
-        const int k = e / B, col = e % B;
-        const int a = pq[2 * k], b = pq[2 * k + 1];
-        if (b >= B) continue;
-        const double c = rcd[k], sn = rsd[k];
-        const double xa = C2[a + (size_t)col * B], xb = C2[b + (size_t)col * B];
-        C2[a + (size_t)col * B] = c * xa - sn * xb;
-        C2[b + (size_t)col * B] = sn * xa + c * xb;
-      }
-      __syncthreads();
-      for (int e = tid; e < npairs * B; e += nt) {  // columns: C2 <- C2 J, V <- V J
-        const int k = e / B, row = e % B;
-        const int a = pq[2 * k], b = pq[2 * k + 1];
-        if (b >= B) continue;
-        const double c = rcd[k], sn = rsd[k];
-        const double xa = C2[row + (size_t)a * B], xb = C2[row + (size_t)b * B];
-        C2[row + (size_t)a * B] = c * xa - sn * xb;
-        C2[row + (size_t)b * B] = sn * xa + c * xb;
-        const double va = V[row + (size_t)a * B], vb = V[row + (size_t)b * B];
-        V[row + (size_t)a * B] = c * va - sn * vb;
-        V[row + (size_t)b * B] = sn * va + c * vb;
-      }
-      __syncthreads();
-    }
-  }
-  for (int c = tid; c < B; c += nt) {
-    double den = 0.0;
-    for (int k = 0; k < B; ++k) den += V[k + (size_t)c * B] * V[k + (size_t)c * B];
-    lam[c] = C2[c + (size_t)c * B];
-    invd[c] = 1.0 / sqrt(den);  // reuse: column scale
-  }
-  __syncthreads();
-  // X = L^-T V (back substitution per column, columns in parallel through rows)
-  for (int e = tid; e < B * B; e += nt) {
-    const int r = e % B, c = e / B;
-    Wm[e] = V[r + (size_t)c * B] * invd[c];
-  }
-  __syncthreads();
-  for (int jr = B - 1; jr >= 0; --jr) {
-    for (int c = tid; c < B; c += nt) Wm[jr + (size_t)c * B] /= L[jr + (size_t)jr * B];
-    __syncthreads();
-    for (int e = tid; e < jr * B; e += nt) {
-      const int i = e % jr, c = e / jr;
-      Wm[i + (size_t)c * B] -= L[jr + (size_t)i * B] * Wm[jr + (size_t)c * B];
-    }
-    __syncthreads();
-  }
-  // ---- ascending order, sign convention, output ----
-  if (tid == 0) {
-    for (int k = 0; k < B; ++k) pq[k] = k;
-    for (int a = 0; a < B; ++a) {  // selection sort (B <= a few hundred)
-      int m = a;
-      for (int b = a + 1; b < B; ++b)
-        if (lam[pq[b]] < lam[pq[m]]) m = b;
-      const int t = pq[a]; pq[a] = pq[m]; pq[m] = t;
-    }
-  }
-  __syncthreads();
-  for (int c = tid; c < B; c += nt) {
-    const int src = pq[c];
-    int imax = 0;
-    double amax = -1.0;
-    for (int r = 0; r < B; ++r) {
-      const double a = fabs(Wm[r + (size_t)src * B]);
-      if (a > amax) { amax = a; imax = r; }
-    }
-    const double sg = (Wm[imax + (size_t)src * B] < 0.0) ? -1.0 : 1.0;
-    for (int r = 0; r < B; ++r) p.U[r + (size_t)c * B] = sg * Wm[r + (size_t)src * B];
-    p.eigv[c] = lam[src];
-  }
+  for (int i = tid; i < B; i += nt) w.invd[i] = inv_s[i];
   if (tid == 0 && info) atomicOr(p.status, 2);
 }
 
-size_t gep_work_doubles(int nbloc) { return (size_t)5 * nbloc * nbloc + 2 * nbloc; }
+// One column of L^-1 X, held by a warp: lane `lane` has rows lane + 32 q.
+__device__ __forceinline__ void warp_forward(const double* L, const double* invd, int B, double (&x)[kMaxQ],
+                                             int lane) {
+  double l[kMaxQ];
+#pragma unroll
+  for (int q = 0; q < kMaxQ; ++q) l[q] = lane + 32 * q < B ? L[lane + 32 * q] : 0.0;
+#pragma unroll
+  for (int q = 0; q < kMaxQ; ++q) {
+    for (int jj = 0; jj < 32; ++jj) {
+      const int j = 32 * q + jj;
+      if (j >= B) break;
+      double cur[kMaxQ];  // column j of L; the next column is fetched while it is used
+#pragma unroll
+      for (int q2 = 0; q2 < kMaxQ; ++q2) cur[q2] = l[q2];
+      if (j + 1 < B)
+#pragma unroll
+        for (int q2 = q; q2 < kMaxQ; ++q2)
+          if (lane + 32 * q2 < B) l[q2] = L[lane + 32 * q2 + (size_t)(j + 1) * B];
+      const double v = __shfl_sync(0xffffffffu, x[q], jj) * invd[j];
+      if (lane == jj) x[q] = v;
+#pragma unroll
+      for (int q2 = q; q2 < kMaxQ; ++q2)
+        if (lane + 32 * q2 > j) x[q2] = fma(-cur[q2], v, x[q2]);
+    }
+  }
+}
+
+// W = L^-1 A (second = false, A from its lower triangle), then C = W L^-T as
+// the columns of L^-1 W^T (second = true); one warp per column.
+__device__ void phase_reduce(const GepParams& p, const GepWork& w, bool second, int cta, int ncta) {
+  const int B = p.nbloc, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int c = cta * nw + (threadIdx.x >> 5); c < B; c += ncta * nw) {
+    double x[kMaxQ];
+#pragma unroll
+    for (int q = 0; q < kMaxQ; ++q) {
+      const int r = lane + 32 * q;
+      x[q] = 0.0;
+      if (r < B) x[q] = second ? w.W[c + (size_t)r * B] : (r >= c ? p.A[r + (size_t)c * B] : p.A[c + (size_t)r * B]);
+    }
+    warp_forward(w.L, w.invd, B, x, lane);
+    double* out = (second ? w.C : w.W) + (size_t)c * B;
+#pragma unroll
+    for (int q = 0; q < kMaxQ; ++q)
+      if (lane + 32 * q < B) out[lane + 32 * q] = x[q];
+  }
+}
+
+// FP32 cyclic Jacobi on C, one CTA, C in shared memory.  The rotations go to
+// w.rot; the eigenvectors are formed afterwards by phase_replay, whose rows
+// are independent.  A round updates every 2 x 2 block (pair k, pair l) of the
+// upper half and mirrors it, each block owned by one thread, with an odd
+// leading dimension so that neither access conflicts.
+__device__ void phase_jacobi(const GepParams& p, const GepWork& w, unsigned char* smem) {
+  const int B = p.nbloc, Bp = gep_pad(B), ld = Bp + 1, np = Bp / 2, tri = np * (np + 1) / 2;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  float* C = reinterpret_cast<float*>(smem);  // [Bp][ld]
+  float* rc = C + (size_t)Bp * ld;            // [np] cosines, then [np] sines
+  float* rs = rc + np;
+  int* pa = reinterpret_cast<int*>(rs + np);  // [np] pair members
+  int* pb = pa + np;
+  __shared__ float red[2][32];
+  for (int e = tid; e < Bp * Bp; e += nt) {
+    const int r = e % Bp, c = e / Bp;
+    C[r + (size_t)c * ld] =
+        r < B && c < B ? (float)(0.5 * (w.C[r + (size_t)c * B] + w.C[c + (size_t)r * B])) : 0.f;
+  }
+  // the blocks of this thread, the same in every round (pairs k <= l)
+  constexpr int kItems = 4;
+  int ik[kItems], il[kItems];
+#pragma unroll
+  for (int q = 0; q < kItems; ++q) {
+    const int e = tid + q * nt;
+    ik[q] = -1;
+    il[q] = 0;
+    if (e < tri) {
+      int l = (int)((sqrtf(8.f * e + 1.f) - 1.f) * 0.5f);
+      while ((l + 1) * (l + 2) / 2 <= e) ++l;
+      while (l * (l + 1) / 2 > e) --l;
+      il[q] = l;
+      ik[q] = e - l * (l + 1) / 2;
+    }
+  }
+  __syncthreads();
+  int sweep = 0;
+  for (; sweep < kJacobiSweeps; ++sweep) {
+    // until the off-diagonal mass is 1e-12 of the diagonal's
+    float off = 0.f, dia = 0.f;
+    for (int e = tid; e < Bp * Bp; e += nt) {
+      const int r = e % Bp, c = e / Bp;
+      const float v = C[r + (size_t)c * ld];
+      if (r == c) dia = fmaf(v, v, dia); else off = fmaf(v, v, off);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      off += __shfl_xor_sync(0xffffffffu, off, o);
+      dia += __shfl_xor_sync(0xffffffffu, dia, o);
+    }
+    __syncthreads();
+    if (tid % 32 == 0) {
+      red[0][tid / 32] = off;
+      red[1][tid / 32] = dia;
+    }
+    __syncthreads();
+    float offt = 0.f, diat = 0.f;
+    for (int q = 0; q < nt / 32; ++q) {
+      offt += red[0][q];
+      diat += red[1][q];
+    }
+    if (offt <= 1e-12f * diat || offt == 0.f) break;
+    for (int round = 0; round < Bp - 1; ++round) {
+      for (int k = tid; k < np; k += nt) {
+        int a, b;
+        robin_pair(Bp, round, k, &a, &b);
+        float c, s;
+        jacobi_rotation(C[a + (size_t)a * ld], C[b + (size_t)b * ld], C[a + (size_t)b * ld], &c, &s);
+        pa[k] = a;
+        pb[k] = b;
+        rc[k] = c;
+        rs[k] = s;
+        w.rot[((size_t)sweep * (Bp - 1) + round) * np + k] = make_float2(c, s);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < kItems; ++q) {
+        const int k = ik[q], l = il[q];
+        if (k < 0) continue;
+        const int ak = pa[k], bk = pb[k], al = pa[l], bl = pb[l];
+        const float ck = rc[k], sk = rs[k], cl = rc[l], sl = rs[l];
+        const float x00 = C[ak + (size_t)al * ld], x01 = C[ak + (size_t)bl * ld], x10 = C[bk + (size_t)al * ld],
+                    x11 = C[bk + (size_t)bl * ld];
+        const float y00 = ck * x00 - sk * x10, y10 = sk * x00 + ck * x10;  // rows: J_k^T
+        const float y01 = ck * x01 - sk * x11, y11 = sk * x01 + ck * x11;
+        const float z00 = cl * y00 - sl * y01, z01 = sl * y00 + cl * y01;  // columns: J_l
+        const float z10 = cl * y10 - sl * y11, z11 = sl * y10 + cl * y11;
+        C[ak + (size_t)al * ld] = z00;
+        C[bk + (size_t)bl * ld] = z11;
+        if (k == l) {
+          C[ak + (size_t)bl * ld] = 0.f;
+          C[bk + (size_t)al * ld] = 0.f;
+        } else {
+          C[ak + (size_t)bl * ld] = z01;
+          C[bk + (size_t)al * ld] = z10;
+          C[al + (size_t)ak * ld] = z00;
+          C[bl + (size_t)ak * ld] = z01;
+          C[al + (size_t)bk * ld] = z10;
+          C[bl + (size_t)bk * ld] = z11;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  if (tid == 0) w.cnt[0] = sweep;
+}
+
+// V = the product of the recorded rotations, kVRows rows per CTA in shared
+// memory, one (row, pair) per thread; rotations of kReplay rounds are loaded
+// together.
+__device__ void phase_replay(const GepParams& p, const GepWork& w, unsigned char* smem, int cta, int ncta) {
+  const int B = p.nbloc, Bp = gep_pad(B), np = Bp / 2, tid = threadIdx.x, nt = blockDim.x;
+  float* V = reinterpret_cast<float*>(smem);  // [kVRows][Bp]
+  const int rounds = w.cnt[0] * (Bp - 1), k = tid % np, r = tid / np;
+  for (int r0 = cta * kVRows; r0 < B; r0 += ncta * kVRows) {
+    for (int e = tid; e < kVRows * Bp; e += nt) V[e] = (e % Bp == r0 + e / Bp) ? 1.f : 0.f;
+    __syncthreads();
+    for (int base = 0; base < rounds; base += kReplay) {
+      float2 cs[kReplay];
+#pragma unroll
+      for (int u = 0; u < kReplay; ++u)
+        cs[u] = r < kVRows && base + u < rounds ? w.rot[(size_t)(base + u) * np + k] : make_float2(1.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < kReplay; ++u) {
+        if (base + u >= rounds) break;
+        if (r < kVRows) {
+          int a, b;
+          robin_pair(Bp, (base + u) % (Bp - 1), k, &a, &b);
+          const float va = V[r * Bp + a], vb = V[r * Bp + b];
+          V[r * Bp + a] = cs[u].x * va - cs[u].y * vb;
+          V[r * Bp + b] = cs[u].y * va + cs[u].x * vb;
+        }
+        __syncthreads();
+      }
+    }
+    for (int e = tid; e < kVRows * B; e += nt) {
+      const int c = e / kVRows, q = e % kVRows;
+      if (r0 + q < B) w.V[r0 + q + (size_t)c * B] = (double)V[q * Bp + c];
+    }
+    __syncthreads();
+  }
+}
+
+// out = f(op(X) Y), FP64, 8 x 8 tiles of a 64-thread CTA, k in chunks of 32
+// through shared memory.  op: transpose when `tx`.
+//   kPlain: the product;  kNewton: 1.5 Y' - 0.5 (product), Y' = X (so X (3 I - G) / 2);
+//   kAdd: X + product.
+enum : int { kPlain = 0, kNewton = 1, kAdd = 2 };
+constexpr int kTile = 8, kChunk = 32;
+
+__device__ void phase_product(const double* X, const double* Y, double* out, int B, bool tx, int form, int cta,
+                              int ncta, unsigned char* smem) {
+  double(*xs)[kChunk + 1] = reinterpret_cast<double(*)[kChunk + 1]>(smem);  // [row of op(X)][k]
+  double(*ys)[kChunk + 1] = xs + kTile;                                      // [column of Y][k]
+  const int t = threadIdx.x, nb = (B + kTile - 1) / kTile, r = t % kTile, c = t / kTile;
+  for (int tile = cta; tile < nb * nb; tile += ncta) {
+    const int r0 = tile % nb * kTile, c0 = tile / nb * kTile;
+    double acc = 0.0;
+    for (int k0 = 0; k0 < B; k0 += kChunk) {
+#pragma unroll
+      for (int u = 0; u < kTile * kChunk / 64; ++u) {
+        const int e = t + 64 * u;
+        // along the contiguous index of each operand: k (X^T, Y) or the row (X)
+        const int i = tx ? e / kChunk : e % kTile, k = tx ? e % kChunk : e / kTile;
+        xs[i][k] = r0 + i < B && k0 + k < B
+                       ? (tx ? X[k0 + k + (size_t)(r0 + i) * B] : X[r0 + i + (size_t)(k0 + k) * B])
+                       : 0.0;
+        ys[e / kChunk][e % kChunk] = c0 + e / kChunk < B && k0 + e % kChunk < B
+                                         ? Y[k0 + e % kChunk + (size_t)(c0 + e / kChunk) * B]
+                                         : 0.0;
+      }
+      __syncthreads();
+      const int kn = min(kChunk, B - k0);
+      for (int k = 0; k < kn; ++k) acc = fma(xs[r][k], ys[c][k], acc);
+      __syncthreads();
+    }
+    const int row = r0 + r, col = c0 + c;
+    if (row < B && col < B) {
+      const size_t e = row + (size_t)col * B;
+      out[e] = form == kPlain ? acc : form == kNewton ? 1.5 * X[e] - 0.5 * acc : X[e] + acc;
+    }
+  }
+}
+
+// E of one iteration; `first` records pairs that need a rotation instead.
+__device__ void phase_correction(const GepWork& w, int B, bool first, int cta, int ncta) {
+  for (int e = cta * blockDim.x + threadIdx.x; e < B * B; e += ncta * blockDim.x) {
+    const int i = e % B, j = e / B;
+    const double g = w.G[e];
+    double x = 0.5 * ((i == j ? 1.0 : 0.0) - g);
+    if (i != j) {
+      const double sii = w.S[i + (size_t)i * B], sjj = w.S[j + (size_t)j * B];
+      const double li = sii / w.G[i + (size_t)i * B], lj = sjj / w.G[j + (size_t)j * B];
+      const double num = 0.5 * (w.S[e] + w.S[j + (size_t)i * B]) - lj * g, gap = lj - li;
+      if (fabs(num) <= kUnsafe * fabs(gap) && gap != 0.0) {
+        x = num / gap;
+      } else if (first && fabs(num) > 1e-15 * fmax(fabs(li), fabs(lj))) {
+        w.cnt[1] = 1;
+      }
+    }
+    w.E[e] = x;
+  }
+}
+
+// The separation of unsafe pairs (one CTA; nothing to do unless cnt[1]): cyclic
+// Jacobi sweeps in FP64 that rotate only those pairs, S in shared memory,
+// V in global memory; then E from the rotated S (V is orthonormal here, G = I).
+__device__ void phase_separate(const GepWork& w, int B, unsigned char* smem) {
+  if (w.cnt[1] == 0) return;
+  const int Bp = gep_pad(B), np = Bp / 2, tid = threadIdx.x, nt = blockDim.x;
+  double* S = reinterpret_cast<double*>(smem);  // [B][B]
+  double* rc = S + (size_t)B * B;               // [np] cosines, then [np] sines
+  double* rs = rc + np;
+  for (int e = tid; e < B * B; e += nt) {
+    const int i = e % B, j = e / B;
+    S[e] = 0.5 * (w.S[e] + w.S[j + (size_t)i * B]);
+  }
+  __syncthreads();
+  for (int sweep = 0; sweep < 12; ++sweep) {
+    bool any = false;
+    for (int round = 0; round < Bp - 1; ++round) {
+      bool mine = false;
+      for (int k = tid; k < np; k += nt) {
+        int a, b;
+        robin_pair(Bp, round, k, &a, &b);
+        double c = 1.0, s = 0.0;
+        if (b < B) {  // index Bp - 1 = B is padding when B is odd
+          const double app = S[a + (size_t)a * B], aqq = S[b + (size_t)b * B], apq = S[a + (size_t)b * B];
+          if (fabs(apq) > kUnsafe * fabs(aqq - app) && fabs(apq) > 1e-16 * fmax(fabs(app), fabs(aqq))) {
+            const double theta = (aqq - app) / (2.0 * apq);
+            const double t = copysign(1.0, theta) / (fabs(theta) + sqrt(theta * theta + 1.0));
+            c = 1.0 / sqrt(t * t + 1.0);
+            s = t * c;
+            mine = true;
+          }
+        }
+        rc[k] = c;
+        rs[k] = s;
+      }
+      if (!__syncthreads_or(mine)) continue;
+      any = true;
+      for (int e = tid; e < np * B; e += nt) {  // rows: S <- J^T S
+        const int k = e / B, col = e % B;
+        int a, b;
+        robin_pair(Bp, round, k, &a, &b);
+        const double c = rc[k], s = rs[k];
+        if (b >= B || s == 0.0) continue;
+        const double xa = S[a + (size_t)col * B], xb = S[b + (size_t)col * B];
+        S[a + (size_t)col * B] = c * xa - s * xb;
+        S[b + (size_t)col * B] = s * xa + c * xb;
+      }
+      __syncthreads();
+      for (int e = tid; e < np * B; e += nt) {  // columns: S <- S J, V <- V J
+        const int k = e / B, row = e % B;
+        int a, b;
+        robin_pair(Bp, round, k, &a, &b);
+        const double c = rc[k], s = rs[k];
+        if (b >= B || s == 0.0) continue;
+        const double xa = S[row + (size_t)a * B], xb = S[row + (size_t)b * B];
+        S[row + (size_t)a * B] = c * xa - s * xb;
+        S[row + (size_t)b * B] = s * xa + c * xb;
+        const double va = w.V[row + (size_t)a * B], vb = w.V[row + (size_t)b * B];
+        w.V[row + (size_t)a * B] = c * va - s * vb;
+        w.V[row + (size_t)b * B] = s * va + c * vb;
+      }
+      __syncthreads();
+    }
+    if (!any) break;
+  }
+  for (int e = tid; e < B * B; e += nt) {
+    const int i = e % B, j = e / B;
+    const double gap = S[j + (size_t)j * B] - S[i + (size_t)i * B];
+    w.E[e] = (i != j && fabs(S[e]) <= kUnsafe * fabs(gap) && gap != 0.0) ? S[e] / gap : 0.0;
+  }
+}
+
+// X = L^-T V with unit columns of V; eigenvalues; ascending order; signs.  One
+// warp per column.
+__device__ void phase_finish(const GepParams& p, const GepWork& w, int cta, int ncta) {
+  const int B = p.nbloc, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int c = cta * nw + (threadIdx.x >> 5); c < B; c += ncta * nw) {
+    const double lam = w.S[c + (size_t)c * B] / w.G[c + (size_t)c * B];
+    int pos = 0;  // place of this eigenvalue, ties by column
+    for (int k = lane; k < B; k += 32) {
+      const double o = w.S[k + (size_t)k * B] / w.G[k + (size_t)k * B];
+      pos += (o < lam) || (o == lam && k < c);
+    }
+    for (int o = 16; o > 0; o >>= 1) pos += __shfl_xor_sync(0xffffffffu, pos, o);
+    double x[kMaxQ], den = 0.0;
+#pragma unroll
+    for (int q = 0; q < kMaxQ; ++q) {
+      x[q] = lane + 32 * q < B ? w.V[lane + 32 * q + (size_t)c * B] : 0.0;
+      den = fma(x[q], x[q], den);
+    }
+    for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
+    const double sc = 1.0 / sqrt(den);
+#pragma unroll
+    for (int q = 0; q < kMaxQ; ++q) x[q] *= sc;
+    // back substitution: row j of L is column j of L^T
+#pragma unroll
+    for (int q = kMaxQ - 1; q >= 0; --q) {
+      for (int jj = 31; jj >= 0; --jj) {
+        const int j = 32 * q + jj;
+        if (j >= B) continue;
+        double l[kMaxQ];
+#pragma unroll
+        for (int q2 = 0; q2 <= q; ++q2) l[q2] = lane + 32 * q2 < j ? w.LT[lane + 32 * q2 + (size_t)j * B] : 0.0;
+        const double v = __shfl_sync(0xffffffffu, x[q], jj) * w.invd[j];
+        if (lane == jj) x[q] = v;
+#pragma unroll
+        for (int q2 = 0; q2 <= q; ++q2) x[q2] = fma(-l[q2], v, x[q2]);
+      }
+    }
+    double amax = -1.0, at = 0.0;  // the first largest magnitude and its value
+    int imax = 0;
+#pragma unroll
+    for (int q = 0; q < kMaxQ; ++q)
+      if (lane + 32 * q < B && fabs(x[q]) > amax) {
+        amax = fabs(x[q]);
+        at = x[q];
+        imax = lane + 32 * q;
+      }
+    for (int o = 16; o > 0; o >>= 1) {
+      const double a2 = __shfl_xor_sync(0xffffffffu, amax, o), t2 = __shfl_xor_sync(0xffffffffu, at, o);
+      const int i2 = __shfl_xor_sync(0xffffffffu, imax, o);
+      if (a2 > amax || (a2 == amax && i2 < imax)) {
+        amax = a2;
+        at = t2;
+        imax = i2;
+      }
+    }
+    const double sg = at < 0.0 ? -1.0 : 1.0;
+#pragma unroll
+    for (int q = 0; q < kMaxQ; ++q)
+      if (lane + 32 * q < B) p.U[lane + 32 * q + (size_t)pos * B] = sg * x[q];
+    if (lane == 0) p.eigv[pos] = lam;
+  }
+}
+
+// The refinement iterations, in order: G = V^T V and W = C V; S = V^T W; E;
+// (first: the separation); V' = V + V E.  V and V' alternate, starting
+// from V2 after the Newton step.
+enum Phase : int {
+  kCholesky, kReduce1, kReduce2, kJacobi, kReplayV, kGram0, kNewtonV, kGramApply, kProject, kCorrect1, kSeparate,
+  kCorrect, kUpdate, kFinish
+};
+
+__device__ void run_phase(const GepParams& p, const GepWork& w, int ph, unsigned char* smem, int cta, int ncta) {
+  const int B = p.nbloc, nb = (B + kTile - 1) / kTile;
+  switch (ph) {
+    case kCholesky: phase_cholesky(p, w, smem); break;
+    case kReduce1: phase_reduce(p, w, false, cta, ncta); break;
+    case kReduce2: phase_reduce(p, w, true, cta, ncta); break;
+    case kJacobi: phase_jacobi(p, w, smem); break;
+    case kReplayV: phase_replay(p, w, smem, cta, ncta); break;
+    case kGram0: phase_product(w.V, w.V, w.G, B, true, kPlain, cta, ncta, smem); break;
+    case kNewtonV: phase_product(w.V, w.G, w.V2, B, false, kNewton, cta, ncta, smem); break;
+    case kGramApply:  // two products of V over twice the tiles
+      if (ncta == 1 || cta < nb * nb) phase_product(w.V, w.V, w.G, B, true, kPlain, cta, ncta == 1 ? 1 : nb * nb, smem);
+      if (ncta == 1 || cta >= nb * nb)
+        phase_product(w.C, w.V, w.W, B, false, kPlain, ncta == 1 ? 0 : cta - nb * nb, ncta == 1 ? 1 : nb * nb, smem);
+      break;
+    case kProject: phase_product(w.V, w.W, w.S, B, true, kPlain, cta, ncta, smem); break;
+    case kCorrect1: phase_correction(w, B, true, cta, ncta); break;
+    case kSeparate: phase_separate(w, B, smem); break;
+    case kCorrect: phase_correction(w, B, false, cta, ncta); break;
+    case kUpdate: phase_product(w.V, w.E, w.V2, B, false, kAdd, cta, ncta, smem); break;
+    case kFinish: phase_finish(p, w, cta, ncta); break;
+  }
+}
+
+// The sequence of phases; `swap` after a phase exchanges V and V'.
+struct Step {
+  Phase phase;
+  bool swap;
+};
+constexpr int kNumSteps = 21;
+__host__ __device__ inline Step step_at(int q) {
+  constexpr Step seq[kNumSteps] = {
+      {kCholesky, false}, {kReduce1, false}, {kReduce2, false}, {kJacobi, false}, {kReplayV, false},
+      {kGram0, false}, {kNewtonV, true},
+      {kGramApply, false}, {kProject, false}, {kCorrect1, false}, {kSeparate, false}, {kUpdate, true},
+      {kGramApply, false}, {kProject, false}, {kCorrect, false}, {kUpdate, true},
+      {kGramApply, false}, {kProject, false}, {kCorrect, false}, {kUpdate, true},
+      {kFinish, false}};
+  return seq[q];
+}
+
+__device__ inline void swap_v(GepWork& w) {
+  double* t = w.V;
+  w.V = w.V2;
+  w.V2 = t;
+}
+
+}  // namespace
+
+// One phase per launch (swapped: V and V' exchanged).
+template <int kPhase>
+__global__ void __launch_bounds__(1024) gep_phase_kernel(GepParams p, int swapped) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  GepWork w;
+  gep_carve(p.nbloc, p.work, &w);
+  if (swapped) swap_v(w);
+  run_phase(p, w, kPhase, smem_raw, blockIdx.x, gridDim.x);
+}
+
+// Every phase in one CTA of 64 threads, for blocks so small that the
+// launches would cost more than the work.
+__global__ void __launch_bounds__(64) gep_small_kernel(GepParams p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  GepWork w;
+  gep_carve(p.nbloc, p.work, &w);
+  for (int q = 0; q < kNumSteps; ++q) {
+    const Step st = step_at(q);
+    run_phase(p, w, st.phase, smem_raw, 0, 1);
+    __syncthreads();
+    if (st.swap) swap_v(w);
+  }
+}
+
+size_t gep_work_doubles(int nbloc) {
+  GepWork w;
+  return gep_carve(nbloc, nullptr, &w);
+}
 
 int gep_launch(const GepParams& p, cudaStream_t st) {
   const int B = p.nbloc;
@@ -415,14 +705,60 @@ int gep_launch(const GepParams& p, cudaStream_t st) {
   return gep_solve_launch(p, st);
 }
 
-int gep_solve_launch(const GepParams& p, cudaStream_t st) {
-  const int B = p.nbloc;
-  const int Bp = (B + 1) / 2 * 2;
-  const size_t smem = sizeof(float) * ((size_t)2 * Bp * Bp + Bp) + sizeof(int) * Bp + 64;
-  MLCP_CUDA_TRY(cudaFuncSetAttribute(gep_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  gep_solve_kernel<<<1, kSolveThreads, smem, st>>>(p);
+namespace {
+
+template <int kPhase>
+int launch_phase(const GepParams& p, int swapped, int grid, int threads, size_t smem, cudaStream_t st) {
+  if (smem > 48 * 1024)
+    MLCP_CUDA_TRY(
+        cudaFuncSetAttribute(gep_phase_kernel<kPhase>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  gep_phase_kernel<kPhase><<<grid, threads, smem, st>>>(p, swapped);
   MLCP_CUDA_TRY(cudaGetLastError());
   return kOk;
+}
+
+// Blocks of at most this many vectors run in gep_small_kernel: a whole
+// diagonalizecpp_ call with it takes 160 us for 4 vectors, 214 for 8, 382 for
+// 12 and 458 for 16; with one launch per phase about 290 us at each of these
+// sizes (297 for 17).
+constexpr int kSmallBlock = 8;
+
+}  // namespace
+
+int gep_solve_launch(const GepParams& p, cudaStream_t st) {
+  const int B = p.nbloc, Bp = gep_pad(B), np = Bp / 2, nb = (B + kTile - 1) / kTile;
+  const size_t s_chol = sizeof(double) * ((size_t)B * B + Bp), s_prod = sizeof(double) * 2 * kTile * (kChunk + 1),
+               s_jac = sizeof(float) * ((size_t)Bp * (Bp + 1) + 4 * np), s_rep = sizeof(float) * kVRows * Bp;
+  if (B <= kSmallBlock) {
+    const size_t smem = std::max(std::max(s_chol, s_prod), std::max(s_jac, s_rep));
+    gep_small_kernel<<<1, 64, smem, st>>>(p);
+    MLCP_CUDA_TRY(cudaGetLastError());
+    return kOk;
+  }
+  int swapped = 0, rc = kOk;
+  for (int q = 0; q < kNumSteps && rc == kOk; ++q) {
+    const Step step = step_at(q);
+    switch (step.phase) {
+      case kCholesky: rc = launch_phase<kCholesky>(p, swapped, 1, 1024, s_chol, st); break;
+      case kReduce1: rc = launch_phase<kReduce1>(p, swapped, B, 32, 0, st); break;
+      case kReduce2: rc = launch_phase<kReduce2>(p, swapped, B, 32, 0, st); break;
+      case kJacobi: rc = launch_phase<kJacobi>(p, swapped, 1, 1024, s_jac, st); break;
+      case kReplayV:
+        rc = launch_phase<kReplayV>(p, swapped, (B + kVRows - 1) / kVRows, round_up(kVRows * np, 32), s_rep, st);
+        break;
+      case kGram0: rc = launch_phase<kGram0>(p, swapped, nb * nb, 64, s_prod, st); break;
+      case kNewtonV: rc = launch_phase<kNewtonV>(p, swapped, nb * nb, 64, s_prod, st); break;
+      case kGramApply: rc = launch_phase<kGramApply>(p, swapped, 2 * nb * nb, 64, s_prod, st); break;
+      case kProject: rc = launch_phase<kProject>(p, swapped, nb * nb, 64, s_prod, st); break;
+      case kCorrect1: rc = launch_phase<kCorrect1>(p, swapped, (B * B + 127) / 128, 128, 0, st); break;
+      case kSeparate: rc = launch_phase<kSeparate>(p, swapped, 1, 1024, s_chol, st); break;
+      case kCorrect: rc = launch_phase<kCorrect>(p, swapped, (B * B + 127) / 128, 128, 0, st); break;
+      case kUpdate: rc = launch_phase<kUpdate>(p, swapped, nb * nb, 64, s_prod, st); break;
+      case kFinish: rc = launch_phase<kFinish>(p, swapped, B, 32, 0, st); break;
+    }
+    if (step.swap) swapped ^= 1;
+  }
+  return rc;
 }
 
 // ---------------------------------------------------------------------------

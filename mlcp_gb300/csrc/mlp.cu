@@ -8,18 +8,27 @@
 //
 // GEMM on the 5th-generation tensor cores: C[M x N] = A[M x K] B[N x K]^T
 // with A and B BF16, K-major (row-major, K contiguous), one CTA of 4 warps
-// per 128 x BN output tile (BN <= 256).  Per 64-wide K slice the operands
-// are copied into shared memory in the canonical no-swizzle K-major layout
+// per 128 x BN output tile.  Per 64-wide K slice the operands are copied with
+// cp.async into shared memory in the canonical no-swizzle K-major layout
 // (8-row x 16-byte core matrices: core (r/8, k/8) at ((r/8) 8 + k/8) 128
 // bytes, so the core-matrix stride is 128 B along K and 1024 B along M/N),
-// two stages deep; one elected thread issues four tcgen05.mma (kind::f16,
-// M = 128, K = 16 each) into a TMEM accumulator and commits them to the
-// stage's mbarrier, which the copies into that stage wait on (bounded
-// waits: on expiry the kernel records status bit 1, stops issuing and
-// still frees its tensor memory).  The epilogue reads the accumulator with
-// tcgen05.ld (warp w: rows 32w..32w+31) and applies bias, ReLU or the ReLU
-// derivative, writing FP32 and/or BF16 and a transposed BF16 copy (the
-// operand layouts of the backward GEMMs).
+// through a ring of up to eight stages; one elected thread issues four
+// tcgen05.mma (kind::f16, M = 128, K = 16 each) into a TMEM accumulator and
+// commits them to the stage's mbarrier, which the copies into that stage
+// wait on (bounded waits: on expiry the kernel records status bit 1, stops
+// issuing and still frees its tensor memory).  The epilogue reads the
+// accumulator with tcgen05.ld (warp w: rows 32w..32w+31) and applies bias,
+// ReLU or the ReLU derivative, writing FP32 and/or BF16 (16 bytes at a time)
+// and a transposed BF16 copy (coalesced along the rows; the operand layouts
+// of the backward GEMMs).
+//
+// What bounds it: the network's GEMMs (768 x 256 x 576 and smaller) are 0.1 us
+// of tensor work; their time is the latency of the first operand slices, the
+// epilogue and the launch.  So the tile width BN is the widest that still
+// gives every SM a tile, the whole K range is in flight at once when it fits
+// the ring, and no lane writes single elements across rows.  With 256-wide
+// tiles (six CTAs), two stages and element-wise stores the five shapes of a
+// training step took 51-77 us each.
 #include <cuda_bf16.h>
 
 #include <cstdint>
@@ -35,8 +44,8 @@ constexpr int kGemmThreads = 128;
 constexpr int kBM = 128;
 constexpr int kBK = 64;
 constexpr int kMaxBN = 256;
+constexpr int kMinBN = 32;
 constexpr int kStageA = kBM * kBK * 2;       // bytes
-constexpr int kStageB = kMaxBN * kBK * 2;    // bytes
 constexpr int kWaitLimit = 1 << 22;
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -67,7 +76,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(saddr(dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// All but the latest N committed groups of this thread have landed.
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -134,27 +148,58 @@ __device__ __forceinline__ void stage_tile(unsigned char* dst, const __nv_bfloat
   }
 }
 
+// Ring stages for tiles of BN columns.
+__host__ __device__ constexpr int gemm_stages(int bn) { return bn <= 64 ? 8 : 4; }
+
+// Eight consecutive BF16 values as 16 bytes.
+__device__ __forceinline__ uint4 pack8(const __nv_bfloat16 (&x)[8]) {
+  uint32_t w[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    w[q] = (uint32_t)__bfloat16_as_ushort(x[2 * q]) | ((uint32_t)__bfloat16_as_ushort(x[2 * q + 1]) << 16);
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Whether rows of `ld` elements of `size` bytes at `ptr` start on 16-byte
+// boundaries (their 8-element groups then do too).
+__device__ __forceinline__ bool rows_aligned(const void* ptr, int ld, int size) {
+  return ((reinterpret_cast<uintptr_t>(ptr) | (uintptr_t)((size_t)ld * size)) & 15u) == 0;
+}
+
 }  // namespace
 
+// BN: the tile width (32, 64, 128 or 256); S = gemm_stages(BN).
+template <int BN>
 __global__ void __launch_bounds__(kGemmThreads, 1) mlp_gemm_kernel(MlpGemm p) {
+  constexpr int S = gemm_stages(BN), kStageB = BN * kBK * 2;
   extern __shared__ __align__(1024) unsigned char gsm[];
-  unsigned char* sA = gsm;                        // [2][kStageA]
-  unsigned char* sB = gsm + 2 * kStageA;          // [2][kStageB]
-  __shared__ __align__(8) uint64_t bar[2];
+  unsigned char* sA = gsm;                 // [S][kStageA]
+  unsigned char* sB = gsm + S * kStageA;   // [S][kStageB]
+  __shared__ __align__(8) uint64_t bar[S];
   __shared__ uint32_t tmem_base;
-  __shared__ int abort_flag;
-  const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * kMaxBN;
-  const int bn = min(kMaxBN, p.N - n0);
+  const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
+  const int bn = min(BN, p.N - n0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int KT = p.K / kBK;
+  auto load = [&](int kt) {
+    const int st = kt % S;
+    stage_tile(sA + st * kStageA, p.A, p.lda, m0, kBM, kt * kBK);
+    stage_tile(sB + st * kStageB, p.B, p.ldb, n0, bn, kt * kBK);
+  };
+  // one group per slice, empty ones past the end, so that the wait below
+  // always means "slice kt has landed"
+#pragma unroll
+  for (int kt = 0; kt < S - 1; ++kt) {
+    if (kt < KT) load(kt);
+    cp_async_commit();
+  }
   if (threadIdx.x == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    abort_flag = 0;
+    for (int s = 0; s < S; ++s) mbar_init(&bar[s], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&tmem_base)),
-                 "r"(kMaxBN)
+                 "r"(BN)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -163,21 +208,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) mlp_gemm_kernel(MlpGemm p) {
   tc_fence_after();
   const uint32_t tmem = tmem_base;
   const uint32_t idesc = idesc_bf16(bn);
-  const int KT = p.K / kBK;
-  uint32_t phase[2] = {0u, 0u};
+  bool failed = false, aborted = false;
   for (int kt = 0; kt < KT; ++kt) {
-    const int st = kt & 1;
-    if (kt >= 2) {  // the MMAs of slice kt - 2 have finished reading this stage
-      if (!abort_flag && !mbar_wait(&bar[st], phase[st])) atomicExch(&abort_flag, 1);
-      phase[st] ^= 1u;
-    }
-    __syncthreads();
-    if (abort_flag) break;
-    stage_tile(sA + st * kStageA, p.A, p.lda, m0, kBM, kt * kBK);
-    stage_tile(sB + st * kStageB, p.B, p.ldb, n0, bn, kt * kBK);
-    cp_async_wait_all();
+    cp_async_wait<S - 2>();
     fence_proxy_async();
-    __syncthreads();
+    aborted = __syncthreads_or(failed);
+    if (aborted) break;
+    const int st = kt % S;
     if (threadIdx.x == 0) {
       tc_fence_after();
       const uint32_t a0 = saddr(sA + st * kStageA), b0 = saddr(sB + st * kStageB);
@@ -186,74 +223,159 @@ __global__ void __launch_bounds__(kGemmThreads, 1) mlp_gemm_kernel(MlpGemm p) {
         mma_bf16(tmem, smem_desc(a0 + kk * 256), smem_desc(b0 + kk * 256), idesc, (kt > 0 || kk > 0) ? 1u : 0u);
       mma_commit(&bar[st]);
     }
+    if (kt + S - 1 < KT) {  // into the stage whose MMAs were committed in the previous iteration
+      if (kt > 0 && !mbar_wait(&bar[(kt - 1) % S], (uint32_t)((kt - 1) / S) & 1u)) failed = true;
+      if (!failed) load(kt + S - 1);
+    }
+    cp_async_commit();
   }
   // the last commit covers every MMA issued before it
-  if (!abort_flag && KT > 0) {
-    const int st = (KT - 1) & 1;
-    if (!mbar_wait(&bar[st], phase[st])) atomicExch(&abort_flag, 1);
-  }
+  if (!aborted && !failed && !mbar_wait(&bar[(KT - 1) % S], (uint32_t)((KT - 1) / S) & 1u)) failed = true;
   tc_fence_before();
-  __syncthreads();
+  aborted = __syncthreads_or(failed) || aborted;
   tc_fence_after();
-  if (!abort_flag) {
+  if (!aborted) {
     const int row = m0 + warp * 32 + lane;
     const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
+    const bool live = row < p.valid_m;
+    const bool vc = p.C && rows_aligned(p.C, p.ldc, 4), vb = p.Cb && rows_aligned(p.Cb, p.ldcb, 2),
+               vm = p.act == 2 && rows_aligned(p.mask, p.ldm, 2);
     for (int c0 = 0; c0 < bn; c0 += 32) {
       float v[32];
       tmem_ld32(trow + (uint32_t)c0, v);
 #pragma unroll
-      for (int q = 0; q < 32; ++q) {
-        const int col = n0 + c0 + q;
-        if (c0 + q >= bn) break;
-        float x = v[q];
-        if (p.bias) x += p.bias[col];
-        if (p.act == 1) x = fmaxf(x, 0.f);
-        if (p.act == 2) x = (__bfloat162float(p.mask[(size_t)row * p.ldm + col]) > 0.f) ? x : 0.f;
-        if (row >= p.valid_m) x = 0.f;
-        if (p.C) p.C[(size_t)row * p.ldc + col] = x;
-        const __nv_bfloat16 xb = __float2bfloat16_rn(x);
-        if (p.Cb) p.Cb[(size_t)row * p.ldcb + col] = xb;
-        if (p.Ct) p.Ct[(size_t)col * p.ldct + row] = xb;
+      for (int g = 0; g < 4; ++g) {  // eight columns at a time (bn is a multiple of 16)
+        if (c0 + 8 * g >= bn) break;
+        const int col = n0 + c0 + 8 * g;
+        float x[8];
+        __nv_bfloat16 xb[8], mk[8];
+        if (p.act == 2) {
+          if (vm) {
+            *reinterpret_cast<uint4*>(mk) = *reinterpret_cast<const uint4*>(p.mask + (size_t)row * p.ldm + col);
+          } else {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) mk[q] = p.mask[(size_t)row * p.ldm + col + q];
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          x[q] = v[8 * g + q];
+          if (p.bias) x[q] += p.bias[col + q];
+          if (p.act == 1) x[q] = fmaxf(x[q], 0.f);
+          if (p.act == 2) x[q] = (__bfloat162float(mk[q]) > 0.f) ? x[q] : 0.f;
+          if (!live) x[q] = 0.f;
+          xb[q] = __float2bfloat16_rn(x[q]);
+        }
+        if (p.C) {
+          float* o = p.C + (size_t)row * p.ldc + col;
+          if (vc) {
+            reinterpret_cast<float4*>(o)[0] = make_float4(x[0], x[1], x[2], x[3]);
+            reinterpret_cast<float4*>(o)[1] = make_float4(x[4], x[5], x[6], x[7]);
+          } else {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) o[q] = x[q];
+          }
+        }
+        if (p.Cb) {
+          __nv_bfloat16* o = p.Cb + (size_t)row * p.ldcb + col;
+          if (vb) {
+            *reinterpret_cast<uint4*>(o) = pack8(xb);
+          } else {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) o[q] = xb[q];
+          }
+        }
+        if (p.Ct)
+#pragma unroll
+          for (int q = 0; q < 8; ++q) p.Ct[(size_t)(col + q) * p.ldct + row] = xb[q];
       }
     }
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kMaxBN) : "memory");
-  if (threadIdx.x == 0 && abort_flag && p.status) atomicOr(p.status, 2);
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN) : "memory");
+  if (threadIdx.x == 0 && aborted && p.status) atomicOr(p.status, 2);
 }
 
-size_t mlp_gemm_smem_bytes() { return 2 * (size_t)kStageA + 2 * (size_t)kStageB; }
+namespace {
+
+template <int BN>
+int gemm_launch_bn(const MlpGemm& g, cudaStream_t st) {
+  constexpr size_t smem = (size_t)gemm_stages(BN) * (kStageA + BN * kBK * 2);
+  MLCP_CUDA_TRY(cudaFuncSetAttribute(mlp_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  mlp_gemm_kernel<BN><<<dim3(g.M / kBM, (g.N + BN - 1) / BN), kGemmThreads, smem, st>>>(g);
+  MLCP_CUDA_TRY(cudaGetLastError());
+  return kOk;
+}
+
+}  // namespace
 
 int mlp_gemm_launch(const MlpGemm& g, cudaStream_t st) {
   if (g.M % kBM || g.K % kBK || g.N % 16 || g.N <= 0 || g.K <= 0 || g.lda % 8 || g.ldb % 8) {
     set_error("mlp gemm: unsupported shape M=%d N=%d K=%d (M multiple of 128, N of 16, K of 64)", g.M, g.N, g.K);
     return kBadArgument;
   }
-  const size_t smem = mlp_gemm_smem_bytes();
-  MLCP_CUDA_TRY(cudaFuncSetAttribute(mlp_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid(g.M / kBM, (g.N + kMaxBN - 1) / kMaxBN);
-  mlp_gemm_kernel<<<grid, kGemmThreads, smem, st>>>(g);
-  MLCP_CUDA_TRY(cudaGetLastError());
-  return kOk;
+  // the widest tile that still makes a tile for every SM (wider tiles re-read
+  // less of A), else the narrowest: one 768 x 256 x 576 GEMM takes 13.9 us
+  // with 32-wide tiles (48 CTAs), and took 76.4 with 256-wide ones (6 CTAs,
+  // two stages, element-wise stores; launch list, cold)
+  int dev = 0, nsm = 0;
+  MLCP_CUDA_TRY(cudaGetDevice(&dev));
+  MLCP_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  int bn = kMaxBN;
+  while (bn > kMinBN && (long long)(g.M / kBM) * ((g.N + bn - 1) / bn) < nsm) bn /= 2;
+  switch (bn) {
+    case 256: return gemm_launch_bn<256>(g, st);
+    case 128: return gemm_launch_bn<128>(g, st);
+    case 64: return gemm_launch_bn<64>(g, st);
+    default: return gemm_launch_bn<32>(g, st);
+  }
 }
 
 // ---------------------------------------------------------------------------
 // Loss, bias gradients, optimiser
 // ---------------------------------------------------------------------------
 
+constexpr int kTileDim = 32;    // tiles of the kernels that also write a transposed copy
+constexpr int kTileThreads = 256;
+
+inline unsigned tile_count(int rows, int cols) {
+  return (unsigned)((long long)((rows + kTileDim - 1) / kTileDim) * ((cols + kTileDim - 1) / kTileDim));
+}
+
+// Sum over the block (warp order; every thread of the block calls it); valid in thread 0.
+__device__ float block_sum_f32(float v) {
+  __shared__ float red[32];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  float s = 0.f;
+  if (threadIdx.x == 0)
+    for (int w = 0; w < (int)blockDim.x / 32; ++w) s += red[w];
+  return s;
+}
+
 // Mean squared error over the valid block (rows < m, cols < n) of Y against
-// T (both [rows][ld] FP32); dY = 2 (Y - T) / (m n) as BF16 [rows][ld] and
-// transposed [ld][rows_p]; loss accumulated into *loss.
-__global__ void mlp_loss_kernel(const float* Y, const float* T, int m, int n, int ld, int rows_p,
-                                __nv_bfloat16* dY, __nv_bfloat16* dYt, float* loss) {
-  const long long total = (long long)rows_p * ld;
+// T (both [rows_p][ld] FP32); dY = 2 (Y - T) / (m n) as BF16 [rows_p][ld] and
+// transposed [ld][rows_p]; loss accumulated into *loss, one atomic per CTA.
+// One 32 x 32 tile per CTA, transposed through shared memory so that both
+// copies are written in rows (13 us -> 5.0 us for 768 x 256: element-wise
+// transposed stores touched a sector per two bytes).
+__global__ void __launch_bounds__(kTileThreads) mlp_loss_kernel(const float* Y, const float* T, int m, int n, int ld,
+                                                                int rows_p, __nv_bfloat16* dY, __nv_bfloat16* dYt,
+                                                                float* loss) {
+  __shared__ __nv_bfloat16 tile[kTileDim][kTileDim + 2];
+  const int tx = threadIdx.x % kTileDim, ty = threadIdx.x / kTileDim;
+  const int across = (ld + kTileDim - 1) / kTileDim;
+  const int r0 = blockIdx.x / across * kTileDim, c0 = blockIdx.x % across * kTileDim;
   const float scale = 2.f / ((float)m * (float)n);
   float part = 0.f;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int r = (int)(e / ld), c = (int)(e - (long long)r * ld);
+#pragma unroll
+  for (int u = 0; u < kTileDim; u += kTileThreads / kTileDim) {
+    const int r = r0 + ty + u, c = c0 + tx;
+    if (r >= rows_p || c >= ld) continue;
+    const size_t e = (size_t)r * ld + c;
     float g = 0.f;
     if (r < m && c < n) {
       const float d = Y[e] - T[e];
@@ -262,29 +384,53 @@ __global__ void mlp_loss_kernel(const float* Y, const float* T, int m, int n, in
     }
     const __nv_bfloat16 gb = __float2bfloat16_rn(g);
     dY[e] = gb;
-    dYt[(size_t)c * rows_p + r] = gb;
+    tile[ty + u][tx] = gb;
   }
-  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(loss, part / ((float)m * (float)n));
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < kTileDim; u += kTileThreads / kTileDim) {
+    const int c = c0 + ty + u, r = r0 + tx;
+    if (r < rows_p && c < ld) dYt[(size_t)c * rows_p + r] = tile[tx][ty + u];
+  }
+  part = block_sum_f32(part);
+  if (threadIdx.x == 0) atomicAdd(loss, part / ((float)m * (float)n));
 }
 
-// db[c] = sum over rows of G[r][c] (BF16 [rows][ld]); one thread per column.
-__global__ void mlp_colsum_kernel(const __nv_bfloat16* G, int rows, int n, int ld, float* db) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
+// db[c] = sum over rows of G[r][c] (BF16 [rows][ld]): a CTA per 32 columns,
+// each warp every 32nd row, the warps' sums added in order (one thread per
+// column walked its rows alone: 45 us -> 5.1 us for 768 x 256).
+__global__ void __launch_bounds__(1024) mlp_colsum_kernel(const __nv_bfloat16* G, int rows, int n, int ld, float* db) {
+  __shared__ float red[32][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int r = 0; r < rows; ++r) s += __bfloat162float(G[(size_t)r * ld + c]);
-  db[c] = s;
+  if (c < n)
+#pragma unroll 8
+    for (int r = warp; r < rows; r += 32) s += __bfloat162float(G[(size_t)r * ld + c]);
+  red[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && c < n) {
+    float t = 0.f;
+    for (int w = 0; w < 32; ++w) t += red[w][lane];
+    db[c] = t;
+  }
 }
 
 // Adam step on FP32 master parameters [rows][cols]; writes the BF16 copy
-// and, when wt is given, the transposed BF16 copy [cols][rows].
-__global__ void mlp_adam_kernel(float* w, const float* g, float* m1, float* m2, int rows, int cols, float lr,
-                                float b1, float b2, float eps, float c1, float c2, __nv_bfloat16* wb,
-                                __nv_bfloat16* wt) {
-  const long long total = (long long)rows * cols;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
+// and, when wt is given, the transposed BF16 copy [cols][rows] (32 x 32
+// tiles, as in the loss kernel).
+__global__ void __launch_bounds__(kTileThreads) mlp_adam_kernel(float* w, const float* g, float* m1, float* m2,
+                                                                int rows, int cols, float lr, float b1, float b2,
+                                                                float eps, float c1, float c2, __nv_bfloat16* wb,
+                                                                __nv_bfloat16* wt) {
+  __shared__ __nv_bfloat16 tile[kTileDim][kTileDim + 2];
+  const int tx = threadIdx.x % kTileDim, ty = threadIdx.x / kTileDim;
+  const int across = (cols + kTileDim - 1) / kTileDim;
+  const int r0 = blockIdx.x / across * kTileDim, x0 = blockIdx.x % across * kTileDim;
+#pragma unroll
+  for (int u = 0; u < kTileDim; u += kTileThreads / kTileDim) {
+    const int r = r0 + ty + u, c = x0 + tx;
+    if (r >= rows || c >= cols) continue;
+    const size_t e = (size_t)r * cols + c;
     const float gv = g[e];
     const float a = b1 * m1[e] + (1.f - b1) * gv;
     const float b = b2 * m2[e] + (1.f - b2) * gv * gv;
@@ -294,24 +440,26 @@ __global__ void mlp_adam_kernel(float* w, const float* g, float* m1, float* m2, 
     w[e] = x;
     const __nv_bfloat16 xb = __float2bfloat16_rn(x);
     if (wb) wb[e] = xb;
-    if (wt) {
-      const int r = (int)(e / cols), c = (int)(e - (long long)r * cols);
-      wt[(size_t)c * rows + r] = xb;
-    }
+    tile[ty + u][tx] = xb;
+  }
+  if (!wt) return;
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < kTileDim; u += kTileThreads / kTileDim) {
+    const int c = x0 + ty + u, r = r0 + tx;
+    if (r < rows && c < cols) wt[(size_t)c * rows + r] = tile[tx][ty + u];
   }
 }
 
 int mlp_loss_launch(const float* Y, const float* T, int m, int n, int ld, int rows_p, __nv_bfloat16* dY,
                     __nv_bfloat16* dYt, float* loss, cudaStream_t st) {
-  const long long total = (long long)rows_p * ld;
-  mlp_loss_kernel<<<(int)std::min<long long>((total + 255) / 256, 1024), 256, 0, st>>>(Y, T, m, n, ld, rows_p, dY,
-                                                                                       dYt, loss);
+  mlp_loss_kernel<<<tile_count(rows_p, ld), kTileThreads, 0, st>>>(Y, T, m, n, ld, rows_p, dY, dYt, loss);
   MLCP_CUDA_TRY(cudaGetLastError());
   return kOk;
 }
 
 int mlp_colsum_launch(const __nv_bfloat16* G, int rows, int n, int ld, float* db, cudaStream_t st) {
-  mlp_colsum_kernel<<<(n + 127) / 128, 128, 0, st>>>(G, rows, n, ld, db);
+  mlp_colsum_kernel<<<(n + 31) / 32, 1024, 0, st>>>(G, rows, n, ld, db);
   MLCP_CUDA_TRY(cudaGetLastError());
   return kOk;
 }
@@ -319,9 +467,8 @@ int mlp_colsum_launch(const __nv_bfloat16* G, int rows, int n, int ld, float* db
 int mlp_adam_launch(float* w, const float* g, float* m1, float* m2, int rows, int cols, float lr, float b1, float b2,
                     float eps, int step, __nv_bfloat16* wb, __nv_bfloat16* wt, cudaStream_t st) {
   const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
-  const long long total = (long long)rows * cols;
-  mlp_adam_kernel<<<(int)std::min<long long>((total + 255) / 256, 2048), 256, 0, st>>>(w, g, m1, m2, rows, cols, lr,
-                                                                                       b1, b2, eps, c1, c2, wb, wt);
+  mlp_adam_kernel<<<tile_count(rows, cols), kTileThreads, 0, st>>>(w, g, m1, m2, rows, cols, lr, b1, b2, eps, c1, c2,
+                                                                   wb, wt);
   MLCP_CUDA_TRY(cudaGetLastError());
   return kOk;
 }

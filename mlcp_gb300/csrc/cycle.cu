@@ -59,6 +59,7 @@ struct HopCache {
   void* dev = nullptr;
   size_t bytes = 0;
   OpTable tab{};
+  std::vector<int> nbas, uoff;  // host copies behind tab.h_nbas, tab.h_uoff
 };
 
 std::mutex g_hop_mu;
@@ -189,6 +190,11 @@ int get_optable(Context* ctx, const Layout& Ly, const int* nbas, int R, int T, c
     std::vector<int> pos(cnt.begin(), cnt.end() - 1);
     for (int t = 0; t < T; ++t) order[(size_t)j * T + pos[uid[(size_t)t * D + j]]++] = t;
   }
+  std::vector<int> slot((size_t)T * D);
+  for (int t = 0; t < T; ++t)
+    for (int d = 0; d < D; ++d) slot[(size_t)t * D + d] = uoff[d] + uid[(size_t)t * D + d];
+  std::vector<dw> alphadw(T);
+  for (int t = 0; t < T; ++t) alphadw[t] = dw_from_double(Hcoef[t]);
   // one device allocation for the whole table
   size_t bytes = 0;
   auto reserve = [&](size_t b) { size_t o = align256(bytes); bytes = o + b; return o; };
@@ -197,7 +203,8 @@ int get_optable(Context* ctx, const Layout& Ly, const int* nbas, int R, int T, c
                o_uid = reserve(sizeof(int) * uid.size()), o_ident = reserve(utot),
                o_h = reserve(sizeof(dw) * hmat.size()), o_h64 = reserve(sizeof(double) * hmat64.size()),
                o_alpha = reserve(sizeof(double) * T),
-               o_order = reserve(sizeof(int) * order.size()), o_gs = reserve(sizeof(int) * gstart.size());
+               o_order = reserve(sizeof(int) * order.size()), o_gs = reserve(sizeof(int) * gstart.size()),
+               o_slot = reserve(sizeof(int) * slot.size()), o_adw = reserve(sizeof(dw) * T);
   std::vector<char> host(bytes);
   std::memcpy(&host[o_nbas], nbas, sizeof(int) * D);
   std::memcpy(&host[o_off], Ly.off.data(), sizeof(int) * (D + 1));
@@ -210,6 +217,8 @@ int get_optable(Context* ctx, const Layout& Ly, const int* nbas, int R, int T, c
   std::memcpy(&host[o_alpha], Hcoef, sizeof(double) * T);
   std::memcpy(&host[o_order], order.data(), sizeof(int) * order.size());
   std::memcpy(&host[o_gs], gstart.data(), sizeof(int) * gstart.size());
+  std::memcpy(&host[o_slot], slot.data(), sizeof(int) * slot.size());
+  std::memcpy(&host[o_adw], alphadw.data(), sizeof(dw) * T);
   if (hc.dev) {
     MLCP_CUDA_TRY(cudaStreamSynchronize(st));
     MLCP_CUDA_TRY(cudaFree(hc.dev));
@@ -225,6 +234,10 @@ int get_optable(Context* ctx, const Layout& Ly, const int* nbas, int R, int T, c
   t.ident = (const unsigned char*)(b + o_ident); t.hdw = (const dw*)(b + o_h);
   t.hmat64 = (const double*)(b + o_h64);
   t.alpha = (const double*)(b + o_alpha); t.order = (const int*)(b + o_order); t.gstart = (const int*)(b + o_gs);
+  t.slot = (const int*)(b + o_slot); t.alphadw = (const dw*)(b + o_adw);
+  hc.nbas.assign(nbas, nbas + D);
+  hc.uoff = uoff;
+  t.h_nbas = hc.nbas.data(); t.h_uoff = hc.uoff.data();
   hc.key = key;
   hc.R = R;
   hc.bytes = bytes;
@@ -245,7 +258,7 @@ __global__ void update_weights_kernel(int B, int R, const double* qcoef, const d
 
 struct CycleBuffers {
   double *q, *qc, *hq, *hqc, *qn, *qnc, *shift;
-  dw *mscr, *wscr, *zscr, *uwork, *qdw;
+  dw *mscr, *wscr, *zscr, *ogscr, *uwork, *qdw;
   double *g64, *gsw, *A, *S, *U, *eigv, *gwork, *wts;
   int *meta, *status;
 };
@@ -262,7 +275,8 @@ size_t plan_cycle(const Layout& Ly, const OpTable& t, int R, int B, CycleBuffers
   cb->qnc = (double*)take(sizeof(double) * vec);
   cb->mscr = (dw*)take(sizeof(dw) * (size_t)B * t.utot * R * R);
   cb->wscr = (dw*)take(sizeof(dw) * (size_t)B * t.umax * R * R);
-  cb->zscr = (dw*)take(sizeof(dw) * (size_t)B * t.umax * R * t.npmax);
+  cb->zscr = (dw*)take(sizeof(dw) * (size_t)B * t.utot * R * t.npmax);
+  cb->ogscr = (dw*)take(sizeof(dw) * opals_grid_dw(t, B));
   cb->g64 = (double*)take(sizeof(double) * (size_t)B * Ly.D * R * R);
   cb->gsw = (double*)take(sizeof(double) * gs_work_doubles(B, R, Ly.nD, Ly.D, Ly.npmax));
   cb->A = (double*)take(sizeof(double) * (size_t)B * B);
@@ -424,7 +438,7 @@ int intertwine_cycle(Context* ctx, double* base, double* coef, const int* nbas, 
       p.ops = tab; p.nvec = B; p.nD = Ly.nD; p.mode = 0; p.nsweeps = npow; p.ishift = ishift; p.eshift = Eshift;
       p.pen_factor = kPen;
       p.fo_base = cb.q; p.fo_coef = cb.qc; p.f_base = cb.q; p.f_coef = cb.qc;
-      p.mscr = cb.mscr; p.wscr = cb.wscr; p.zscr = cb.zscr; p.g64 = cb.g64; p.status = cb.status;
+      p.mscr = cb.mscr; p.wscr = cb.wscr; p.zscr = cb.zscr; p.gscr = cb.ogscr; p.g64 = cb.g64; p.status = cb.status;
       p.rank_v = d_rank;
       if (int r = opals_launch(p, st)) return r;
     }
@@ -444,7 +458,7 @@ int intertwine_cycle(Context* ctx, double* base, double* coef, const int* nbas, 
         p.ops = tab; p.nvec = B; p.nD = Ly.nD; p.mode = 1; p.nsweeps = nals; p.ishift = 0; p.eshift = 0.0;
         p.pen_factor = kPen;
         p.fo_base = cb.q; p.fo_coef = cb.qc; p.f_base = cb.hq; p.f_coef = cb.hqc;
-        p.mscr = cb.mscr; p.wscr = cb.wscr; p.zscr = cb.zscr; p.g64 = cb.g64; p.status = cb.status;
+        p.mscr = cb.mscr; p.wscr = cb.wscr; p.zscr = cb.zscr; p.gscr = cb.ogscr; p.g64 = cb.g64; p.status = cb.status;
         p.rank_v = d_rank;
         if (int r = opals_launch(p, st)) return r;
       } else {
@@ -932,7 +946,7 @@ int spectral_range(Context* ctx, double* base, double* coef, const int* nbas, in
       p.eshift_v = shift;
       p.pen_factor = kPen;
       p.fo_base = cb.q; p.fo_coef = cb.qc; p.f_base = cb.q; p.f_coef = cb.qc;
-      p.mscr = cb.mscr; p.wscr = cb.wscr; p.zscr = cb.zscr; p.g64 = cb.g64; p.status = cb.status;
+      p.mscr = cb.mscr; p.wscr = cb.wscr; p.zscr = cb.zscr; p.gscr = cb.ogscr; p.g64 = cb.g64; p.status = cb.status;
       if ((rc = opals_launch(p, st))) return rc;
     }
     if ((rc = rq_launch(q, st))) return rc;

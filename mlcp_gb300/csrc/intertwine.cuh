@@ -30,6 +30,10 @@ struct OpTable {
   const double* alpha;      // [T] term coefficients
   const int* order;         // [D][T] terms grouped by their operator at mode j
   const int* gstart;        // [D][umax+1] group starts in order[j]
+  const int* slot;          // [T][D] global operator slot of term t at mode d (uoff[d] + uid)
+  const dw* alphadw;        // [T] term coefficients in double-word
+  const int* h_nbas;        // [D] and [D+1]: nbas and uoff in host memory, for the launch planners
+  const int* h_uoff;
 };
 
 // Ragged ranks (an extension; the reference requires equal ranks in a block,
@@ -57,16 +61,19 @@ struct OpAlsParams {
   double* f_coef;
   dw* mscr;               // [nvec][utot][R][R] operator Grams M = Fo^T h F
   dw* wscr;               // [nvec][umax][R][R] grouped term products W
-  dw* zscr;               // [nvec][umax][R][npmax] h Fo_j
+  dw* zscr;               // [nvec][utot][R][npmax] h Fo_d
   double* g64;            // [nvec][D][R][R] FP64 Grams of F
   int* status;            // [nvec]
+  dw* gscr;               // opals_grid_dw(ops, nvec): scratch of the grid form
   const int* rank_v;      // [nvec] ranks <= R (terms beyond carry zero weight), or null: all R
-  int tabulate;           // set by opals_launch: term/operator tables copied to shared memory
 };
 
 int opals_launch(const OpAlsParams& p, cudaStream_t st);
-// Smallest shared-memory footprint of the kernel (no resident operators, no tables).
+// Shared-memory footprint that a shape may not exceed.
 size_t opals_smem_bytes(const OpTable& t);
+// The grid form (opals_grid.cu) and its scratch entries.
+int opals_grid_launch(const OpAlsParams& p, cudaStream_t st);
+size_t opals_grid_dw(const OpTable& t, int nvec);
 
 // ALS-guided Gram-Schmidt over a block (reference src/intertw_lcv.cu:131).
 struct GsParams {

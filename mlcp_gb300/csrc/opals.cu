@@ -1,4 +1,5 @@
-// ALS-fitted Hamiltonian applications, one persistent CTA per vector.
+// ALS-fitted Hamiltonian applications, one persistent CTA per vector (small
+// nodes; opals_grid.cu has the form for larger ones).
 //
 // Reference: POW_ALS (src/intertw_mvp.cu:452-497) and PRODHV_ALS (:501-549)
 // with mvp_build_linear_system (:380-448).  For mode j the reference builds,
@@ -34,51 +35,42 @@
 #include "dword.cuh"
 #include "dwsolve.cuh"
 #include "intertwine.cuh"
+#include "opstep.cuh"
 
 namespace mlcp {
 
 namespace {
 
-constexpr int kThreads = 256;
-
-constexpr int kWarps = kThreads / 32;
+constexpr int kThreads = kStepThreads;
 
 struct OpSmem {
+  StepSmem st;    // the step from the normal equations on
   dw* f;          // [R][nDp] current F
   dw* fo;         // [R][nDp] Fo; aliases f for POW
   dw* y;          // [R][npmax] temporary h Fo_r
-  dw* X;          // [R][npmax] solution (column-major, ld R)
-  dw* b0;         // [R][npmax] right-hand side
-  dw* res;        // [R][npmax] refinement residual
-  dw* BB;         // [R][R] normal equations
-  float* gi;      // [2][R][R] FP32 inverse of BB
-  dw* cf;         // [R] weights of F
   dw* cfo;        // [R] weights of Fo
-  dw* red;        // [kWarps] reduction scratch
-  dw* dinv;       // [R] LDL^T reciprocal pivots
-  dw* u;          // [R] LDL^T scratch column
-  dw* misc;       // [2] penalty, norm
-  float* rred;    // [4] refinement scratch
-  dwsolve::ColScratch cs;
-  int* moff;      // [T][D] offset of each term's operator Gram per mode (null when T D is large)
-  int* ord;       // [D][T] terms grouped by their operator at each mode (with moff)
-  int* gst;       // [D][umax+1] group starts (with moff)
-  dw* alpha;      // [T] term coefficients (with moff)
-  dw *Ms, *Ws, *Zs;  // operator Grams, term products, h_u Fo_j when resident in shared memory
-  dw* hs;         // [utot][npmax][npmax] the operators when resident
-  int* flags;     // [4]
+  int* moff;      // [T][D] offset of each term's operator Gram per mode
+  int* ord;       // [D][T] terms grouped by their operator at each mode
+  int* gst;       // [D][umax+1] group starts
+  dw* alpha;      // [T] term coefficients
+  dw *Ms, *Ws, *Zs;  // operator Grams, term products, h_u Fo_j
+  dw* hs;         // [utot][npmax][npmax] the operators
 };
 
-// Terms x modes up to which the Gram offsets are tabulated in shared memory.
+// Terms x modes up to which the one-CTA form tabulates the Gram offsets.
 constexpr int kMoffMax = 8192;
+// Multiply-adds per mode step and vector up to which the one-CTA form is
+// taken: a grid step costs four launches (24 us at least, whatever the block),
+// a step of the one-CTA form what its one CTA takes.  Measured steps, one CTA
+// against grid: 6 modes of 10, rank 16 (41 k) 18.5 against 24.5 us; 4 of 6,
+// rank 8, 40 terms (29 k) 22 against 33; 8 of 10, rank 20 (82 k) 35 against
+// 38; 3 of 30, rank 16 (150 k) 105 against 34; 2 of 24, rank 24 (170 k) 121
+// against 80.
+constexpr double kOneCtaWork = 1.0e5;
 
 // Carves the shared memory (null base: sizes only); returns the bytes.
-// tabulate: copy the term tables (Gram offsets, operator groups, term
-// coefficients) into shared memory when T D <= kMoffMax; without them the
-// kernel reads the same tables from the global operator table.
-__host__ __device__ inline size_t carve(OpSmem& s, unsigned char* base, const OpTable& t, bool separate_fo,
-                                        bool resident, bool tabulate) {
-  size_t o = 0;
+__host__ __device__ inline size_t carve(OpSmem& s, unsigned char* base, const OpTable& t, bool separate_fo) {
+  size_t o = (step_carve(s.st, base, t.R, t.npmax) + 15) / 16 * 16;
   auto take = [&](size_t bytes) -> unsigned char* {
     const size_t r = o;
     o += (bytes + 15) / 16 * 16;
@@ -88,64 +80,16 @@ __host__ __device__ inline size_t carve(OpSmem& s, unsigned char* base, const Op
   s.f = (dw*)take(sizeof(dw) * t.R * t.nDp);
   s.fo = separate_fo ? (dw*)take(sizeof(dw) * t.R * t.nDp) : s.f;
   s.y = (dw*)take(sizeof(dw) * Rn);
-  s.X = (dw*)take(sizeof(dw) * Rn);
-  s.b0 = (dw*)take(sizeof(dw) * Rn);
-  s.res = (dw*)take(sizeof(dw) * Rn);
-  s.BB = (dw*)take(sizeof(dw) * RR);
-  s.gi = (float*)take(sizeof(float) * 2 * RR);
-  s.cf = (dw*)take(sizeof(dw) * t.R);
   s.cfo = (dw*)take(sizeof(dw) * t.R);
-  s.red = (dw*)take(sizeof(dw) * kWarps);
-  s.dinv = (dw*)take(sizeof(dw) * t.R);
-  s.u = (dw*)take(sizeof(dw) * t.R);
-  s.misc = (dw*)take(sizeof(dw) * 2);
-  s.rred = (float*)take(sizeof(float) * 4);
-  s.cs.conv = (float*)take(sizeof(float) * 64);
-  s.cs.rmax = (float*)take(sizeof(float) * 16 * 32);
-  s.cs.rsum = (dw*)take(sizeof(dw) * 16 * 32);
-  const bool tab = tabulate && t.T * t.D <= kMoffMax;
-  s.moff = tab ? (int*)take(sizeof(int) * t.T * t.D) : nullptr;
-  s.ord = tab ? (int*)take(sizeof(int) * t.T * t.D) : nullptr;
-  s.gst = tab ? (int*)take(sizeof(int) * t.D * (t.umax + 1)) : nullptr;
-  s.alpha = tab ? (dw*)take(sizeof(dw) * t.T) : nullptr;
-  s.hs = resident ? (dw*)take(sizeof(dw) * t.utot * t.npmax * t.npmax) : nullptr;
-  s.Ms = resident ? (dw*)take(sizeof(dw) * t.utot * RR) : nullptr;
-  s.Ws = resident ? (dw*)take(sizeof(dw) * t.umax * RR) : nullptr;
-  s.Zs = resident ? (dw*)take(sizeof(dw) * t.umax * Rn) : nullptr;
-  s.flags = (int*)take(sizeof(int) * 4);
+  s.moff = (int*)take(sizeof(int) * t.T * t.D);
+  s.ord = (int*)take(sizeof(int) * t.T * t.D);
+  s.gst = (int*)take(sizeof(int) * t.D * (t.umax + 1));
+  s.alpha = (dw*)take(sizeof(dw) * t.T);
+  s.hs = (dw*)take(sizeof(dw) * t.utot * t.npmax * t.npmax);
+  s.Ms = (dw*)take(sizeof(dw) * t.utot * RR);
+  s.Ws = (dw*)take(sizeof(dw) * t.umax * RR);
+  s.Zs = (dw*)take(sizeof(dw) * t.umax * Rn);
   return o;
-}
-
-// Sum over the block; thread 0 gets the result (fixed order).
-__device__ dw block_sum_dw(dw v, dw* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int o = 16; o > 0; o >>= 1) v = dw_add(v, dwsolve::dw_shfl_xor(v, o));
-  __syncthreads();
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  dw s = dw_make(0.f);
-  if (threadIdx.x == 0)
-    for (int w = 0; w < kWarps; ++w) s = dw_add(s, red[w]);
-  return s;
-}
-
-// In-place POW applies (H - E) once per mode step, so within a sweep the
-// weights grow (or shrink) by about ||H - E|| per step: a 12-mode quartic
-// force field in cm^-1 passes the FP32 exponent range after nine steps, and a
-// 400-term random Hamiltonian over 24 modes overflows the squared row norms
-// (weights above 1.8e19).  The end-of-sweep renormalisation divides out any
-// common factor, so after each step the weights are multiplied by the power
-// of two that brings the largest into [0.5, 1): exact, and the solve is linear
-// in the weights, so the sweep's result is unchanged.  Warp 0 only; each lane
-// rescales the entries it read.
-__device__ void rescale_weights_warp(dw* cf, int R) {
-  float m = 0.f;
-  for (int i = threadIdx.x; i < R; i += 32) m = fmaxf(m, fabsf(cf[i].hi));
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (!(m > 0.f && m <= 3.4028235e38f)) return;  // zero, or non-finite (reported by the next solve)
-  int e;
-  frexpf(m, &e);
-  for (int i = threadIdx.x; i < R; i += 32) cf[i] = dw_make(ldexpf(cf[i].hi, -e), ldexpf(cf[i].lo, -e));
 }
 
 // M(r,i) = sum_n (h Fo_r^d)(n) F_i^d(n); identity operators skip the product.
@@ -189,9 +133,6 @@ __device__ void f_gram_from64(const OpTable& t, int d, const double* fb, int nD,
 
 }  // namespace
 
-// kResident: the operator Grams, term products, h_u Fo_j and the operators in
-// shared memory (else in the per-vector global scratch of p and the table).
-template <bool kResident>
 __global__ void __launch_bounds__(kThreads, 1) opals_kernel(OpAlsParams p) {
   const OpTable& t = p.ops;
   const int v = blockIdx.x;
@@ -199,27 +140,24 @@ __global__ void __launch_bounds__(kThreads, 1) opals_kernel(OpAlsParams p) {
   const bool pow_mode = (p.mode == 0);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   OpSmem s;
-  carve(s, smem_raw, t, !pow_mode, kResident, p.tabulate != 0);
+  carve(s, smem_raw, t, !pow_mode);
 
   const double* fob = p.fo_base + (size_t)v * R * nD;
   const double* foc = p.fo_coef + (size_t)v * R;
   double* fb = p.f_base + (size_t)v * R * nD;
   double* fc = p.f_coef + (size_t)v * R;
-  dw* M = kResident ? s.Ms : p.mscr + (size_t)v * t.utot * R * R;
-  dw* W = kResident ? s.Ws : p.wscr + (size_t)v * t.umax * R * R;
-  dw* Z = kResident ? s.Zs : p.zscr + (size_t)v * t.umax * R * npm;
+  dw* M = s.Ms;
+  dw* W = s.Ws;
+  dw* Z = s.Zs;
   const int* moff = s.moff;
-  if (moff) {
-    for (int e = threadIdx.x; e < T * D; e += blockDim.x) {
-      s.moff[e] = (t.uoff[e % D] + t.uid[e]) * RR;
-      s.ord[e] = t.order[e];
-    }
-    for (int e = threadIdx.x; e < D * (t.umax + 1); e += blockDim.x) s.gst[e] = t.gstart[e];
-    for (int e = threadIdx.x; e < T; e += blockDim.x) s.alpha[e] = dw_from_double(t.alpha[e]);
+  for (int e = threadIdx.x; e < T * D; e += blockDim.x) {
+    s.moff[e] = t.slot[e] * RR;
+    s.ord[e] = t.order[e];
   }
-  const dw* hmat = kResident ? s.hs : t.hdw;
-  if (kResident)
-    for (int e = threadIdx.x; e < t.utot * npm * npm; e += blockDim.x) s.hs[e] = t.hdw[e];
+  for (int e = threadIdx.x; e < D * (t.umax + 1); e += blockDim.x) s.gst[e] = t.gstart[e];
+  for (int e = threadIdx.x; e < T; e += blockDim.x) s.alpha[e] = t.alphadw[e];
+  const dw* hmat = s.hs;
+  for (int e = threadIdx.x; e < t.utot * npm * npm; e += blockDim.x) s.hs[e] = t.hdw[e];
   dw* G = reinterpret_cast<dw*>(p.g64) + (size_t)v * D * R * R;  // double-word F Grams per mode
 
   // ---- set-up: F (= Fo for PRODHV), double-word copies, Grams, penalty ----
@@ -238,20 +176,20 @@ __global__ void __launch_bounds__(kThreads, 1) opals_kernel(OpAlsParams p) {
     if (!pow_mode) s.fo[e] = x;
   }
   for (int e = threadIdx.x; e < R; e += blockDim.x) {
-    s.cf[e] = dw_from_double(fc[e]);
+    s.st.cf[e] = dw_from_double(fc[e]);
     s.cfo[e] = dw_from_double(foc[e]);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     double pen = foc[0];
     for (int i = 1; i < R; ++i) pen = foc[i] > pen ? foc[i] : pen;
-    s.misc[0] = dw_from_double(pen * p.pen_factor);
-    s.flags[0] = 0;
-    s.flags[1] = 0;
+    s.st.misc[0] = dw_from_double(pen * p.pen_factor);
+    s.st.flags[0] = 0;
+    s.st.flags[1] = 0;
   }
   for (int d = 0; d < D; ++d) f_gram_from64(t, d, fb, nD, G + (size_t)d * R * R);
   __syncthreads();
-  const dw pen = s.misc[0];
+  const dw pen = s.st.misc[0];
   const int rv = p.rank_v ? p.rank_v[v] : R;  // ragged: this vector's rank
   for (int d = 0; d < D; ++d)
     for (int u = 0; u < t.uoff[d + 1] - t.uoff[d]; ++u)
@@ -262,37 +200,17 @@ __global__ void __launch_bounds__(kThreads, 1) opals_kernel(OpAlsParams p) {
     for (int j = 0; j < D; ++j) {
       const int nj = t.nbas[j], opj = t.offp[j];
       const int nu = t.uoff[j + 1] - t.uoff[j];
-      const int* ord = (moff ? s.ord : t.order) + (size_t)j * T;
-      const int* gs = (moff ? s.gst : t.gstart) + (size_t)j * (t.umax + 1);
+      const int* ord = s.ord + (size_t)j * T;
+      const int* gs = s.gst + (size_t)j * (t.umax + 1);
       // -- normal equations from the Grams of the previous step:
       //    prod_{d != j} G_d + pen I --
-      for (int e = threadIdx.x; e < RR; e += blockDim.x) {
-        dw bb = dw_make(1.f);
-        for (int d = 0; d < D; ++d)
-          if (d != j) bb = dw_mul(bb, G[(size_t)d * RR + e]);
-        if (e % R == e / R) bb = dw_add(bb, pen);
-        if (e % R >= rv || e / R >= rv) bb = dw_make(e % R == e / R ? 1.f : 0.f);  // ragged: decoupled padding
-        s.BB[e] = bb;
-      }
+      for (int e = threadIdx.x; e < RR; e += blockDim.x) s.st.BB[e] = normal_equation(G, D, j, e, R, rv, pen);
       __syncthreads();
       // -- their FP32 inverse (warp 0 in registers for R <= 32, else warps
       //    0-3) while the other warps form the right-hand side --
-      const int w0 = R <= 32 ? 32 : dwsolve::kSolverThreads;
+      const int w0 = step_invert_threads(R);
       if (threadIdx.x < w0) {
-        if (R <= 32) {
-          const bool g = dwsolve::gj_inverse_warp(s.BB, R, s.gi);
-          if (threadIdx.x == 0) {
-            s.flags[2] = g;
-            s.flags[0] = 0;
-          }
-        } else {
-          bool ok;
-          const float* iv = dwsolve::gj_inverse(s.BB, R, s.gi, &ok);
-          if (threadIdx.x == 0) {
-            s.flags[2] = ok;
-            s.flags[0] = iv == s.gi ? 0 : 1;
-          }
-        }
+        step_invert(s.st, R);
       } else {
         const int wt = threadIdx.x - w0, nw = kThreads - w0;
         // grouped term products W_u(r,i) = sum_{t in group u} alpha_t prod_{d != j} M[d][op(t,d)](r,i),
@@ -307,14 +225,14 @@ __global__ void __launch_bounds__(kThreads, 1) opals_kernel(OpAlsParams p) {
             for (int k = 0; k < 4; ++k) {
               const bool live = q + k < gs[u + 1];
               const int term = ord[live ? q + k : q];
-              pr[k] = live ? (moff ? s.alpha[term] : dw_from_double(t.alpha[term])) : dw_make(0.f);
+              pr[k] = live ? s.alpha[term] : dw_make(0.f);
               tb[k] = term * D;
             }
             for (int d = 0; d < D; ++d) {
               if (d == j) continue;
 #pragma unroll
               for (int k = 0; k < 4; ++k)
-                pr[k] = dw_mul(pr[k], M[(moff ? moff[tb[k] + d] : (t.uoff[d] + t.uid[tb[k] + d]) * RR) + e]);
+                pr[k] = dw_mul(pr[k], M[moff[tb[k] + d] + e]);
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k) acc_add(acc, pr[k]);
@@ -344,7 +262,7 @@ __global__ void __launch_bounds__(kThreads, 1) opals_kernel(OpAlsParams p) {
         }
         asm volatile("bar.sync 2, %0;" ::"r"(nw) : "memory");
         // right-hand side b(i,n) = sum_u sum_r W_u(r,i) c_r Z_u(r,n)
-        const dw* cg = pow_mode ? s.cf : s.cfo;
+        const dw* cg = pow_mode ? s.st.cf : s.cfo;
         for (int e = wt; e < R * nj; e += nw) {
           const int i = e % R, m = e / R;
           dw_acc acc = acc_zero();
@@ -352,60 +270,14 @@ __global__ void __launch_bounds__(kThreads, 1) opals_kernel(OpAlsParams p) {
             for (int r = 0; r < R; ++r)
               acc_fma(acc, dw_mul(W[(size_t)u * RR + r * R + i], cg[r]), Z[(size_t)u * R * npm + r * npm + m]);
           const dw b = acc_value(acc);
-          s.b0[i + m * R] = i >= rv ? dw_make(m == 0 ? 1.f : 0.f) : (p.ishift < 0 ? dw_neg(b) : b);
+          s.st.b0[i + m * R] = i >= rv ? dw_make(m == 0 ? 1.f : 0.f) : (p.ishift < 0 ? dw_neg(b) : b);
         }
       }
       __syncthreads();
-      bool gj_ok = s.flags[2] != 0;
-      const float* inv = s.gi + (size_t)s.flags[0] * RR;
-      bool solved = false;
-      const int nsw = dwsolve::solve_cols_warps(R, nj);
-      if (gj_ok && R <= 32 && nj <= 16 && nsw <= kWarps) {
-        if (threadIdx.x < nsw * 32) {
-          const bool ok = dwsolve::solve_cols_any(s.BB, R, s.b0, s.X, nj, inv, s.cf, s.cs);
-          if (threadIdx.x == 0) s.flags[3] = ok;
-        }
-        __syncthreads();
-        solved = s.flags[3] != 0;
-        gj_ok = false;  // not converged: straight to the LDL^T
-      }
-      if (!solved) {
-        if (threadIdx.x < dwsolve::kSolverThreads) {
-          int bad = 0;
-          if (!(gj_ok && dwsolve::refine_solve(s.BB, R, s.b0, s.X, nj, inv, s.res, s.rred))) {
-            for (int e = threadIdx.x; e < R * nj; e += dwsolve::kSolverThreads) s.X[e] = s.b0[e];
-            bad = dwsolve::dw_ldlt(s.BB, R, s.dinv, s.u);
-            dwsolve::dw_ldlt_solve(s.BB, R, s.dinv, s.X, nj);
-          }
-          dwsolve::dw_normalise_rows(s.X, R, nj, s.cf);
-          if (threadIdx.x == 0 && bad) s.flags[1] = 1;
-        }
-        __syncthreads();
-      }
-      // -- the new factor: FP64 output, double-word copy and Gram (warp 0
-      //    rescales the POW weights first; no other thread reads them before
-      //    the next barrier) --
-      if (threadIdx.x < 32) {
-        for (int i = rv + threadIdx.x; i < R; i += 32) s.cf[i] = dw_make(0.f);  // ragged: padding stays weightless
-        __syncwarp();
-        if (pow_mode) rescale_weights_warp(s.cf, R);
-        for (int i = threadIdx.x; i < R; i += 32) fc[i] = dw_to_double(s.cf[i]);
-      }
-      for (int e = threadIdx.x; e < R * nj; e += blockDim.x) {
-        const int i = e / nj, m = e % nj;
-        const dw x = s.X[i + m * R];
-        fb[(size_t)i * nD + t.off[j] + m] = dw_to_double(x);
-        s.f[i * t.nDp + opj + m] = x;
-      }
-      for (int e = threadIdx.x; e < R * R; e += blockDim.x) {
-        const int i = e % R, i2 = e / R;
-        if (i > i2) continue;
-        dw_acc acc = acc_zero();
-        for (int m = 0; m < nj; ++m) acc_fma(acc, s.X[i + m * R], s.X[i2 + m * R]);
-        const dw g = acc_value(acc);
-        G[(size_t)j * R * R + i + i2 * R] = g;
-        G[(size_t)j * R * R + i2 + i * R] = g;
-      }
+      step_solve(s.st, R, nj);
+      // -- the new factor: FP64 output, double-word copy and Gram --
+      step_weights(s.st, R, rv, pow_mode, fc);
+      step_factor(s.st, R, nj, fb + t.off[j], nD, s.f + opj, t.nDp, G + (size_t)j * RR);
       __syncthreads();
       // -- operator Grams of mode j with the new factor: h_u F_j for every
       //    operator (POW; PRODHV keeps h_u Fo_j in Z), then M_u = (h_u F_j) F_j^T --
@@ -434,62 +306,34 @@ __global__ void __launch_bounds__(kThreads, 1) opals_kernel(OpAlsParams p) {
       }
       __syncthreads();
     }
-    if (pow_mode) {
-      // weight renormalisation after each sweep (src/intertw_mvp.cu:491-494)
-      dw part = dw_make(0.f);
-      for (int e = threadIdx.x; e < R * R; e += blockDim.x) {
-        dw prod = dw_mul(s.cf[e % R], s.cf[e / R]);
-        for (int d = 0; d < D; ++d) prod = dw_mul(prod, G[(size_t)d * R * R + e]);
-        part = dw_add(part, prod);
-      }
-      const dw tot = block_sum_dw(part, s.red);
-      if (threadIdx.x == 0) s.misc[1] = dw_sqrt(dw_abs(tot));
-      __syncthreads();
-      const dw q = s.misc[1];
-      for (int i = threadIdx.x; i < R; i += blockDim.x) {
-        s.cf[i] = dw_div(s.cf[i], q);
-        fc[i] = dw_to_double(s.cf[i]);
-      }
-      __syncthreads();
-    }
+    if (pow_mode) step_renormalise(s.st, R, D, G, fc);
   }
-  if (threadIdx.x == 0 && s.flags[1]) atomicOr(&p.status[v], 1);
+  if (threadIdx.x == 0 && s.st.flags[1]) atomicOr(&p.status[v], 1);
 }
 
+// F, Fo and one mode step: what both forms' callers check against the
+// device's limit (the grid form alone would need less).
 size_t opals_smem_bytes(const OpTable& t) {
-  OpSmem s;
-  return carve(s, nullptr, t, true, false, false);
+  StepSmem m;
+  return step_carve(m, nullptr, t.R, t.npmax) +
+         sizeof(dw) * ((size_t)2 * t.R * t.nDp + (size_t)t.R * t.npmax + (size_t)t.R);
 }
 
-// Largest layout that fits: operators and Grams resident with the tables,
-// then the tables alone, then neither (wide top-layer vectors, e.g. rank 30
-// over 6 x 48 basis functions, where F and Fo take 138 KB).
-int opals_launch(const OpAlsParams& p0, cudaStream_t st) {
+int opals_launch(const OpAlsParams& p, cudaStream_t st) {
   int dev = 0, limit = 0;
   MLCP_CUDA_TRY(cudaGetDevice(&dev));
   MLCP_CUDA_TRY(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  OpAlsParams p = p0;
   OpSmem s;
-  p.tabulate = 1;
-  const size_t res = carve(s, nullptr, p.ops, p.mode != 0, true, true);
-  if (res <= (size_t)limit) {
-    MLCP_CUDA_TRY(cudaFuncSetAttribute(opals_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)res));
-    opals_kernel<true><<<p.nvec, kThreads, res, st>>>(p);
-    MLCP_CUDA_TRY(cudaGetLastError());
-    return kOk;
-  }
-  size_t smem = carve(s, nullptr, p.ops, p.mode != 0, false, true);
-  if (smem > (size_t)limit) {
-    p.tabulate = 0;
-    smem = carve(s, nullptr, p.ops, p.mode != 0, false, false);
-  }
-  if (smem > (size_t)limit) {
-    set_error("ALS-fitted products: rank %d over %d padded basis functions needs %zu bytes of shared memory (limit %d)",
-              p.ops.R, p.ops.nDp, smem, limit);
-    return kTooLarge;
-  }
-  MLCP_CUDA_TRY(cudaFuncSetAttribute(opals_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  opals_kernel<false><<<p.nvec, kThreads, smem, st>>>(p);
+  const size_t res = carve(s, nullptr, p.ops, p.mode != 0);
+  // multiply-adds of one mode step of one vector: term products, operators
+  // applied, operator Grams and right-hand side (mean over the modes)
+  const OpTable& t = p.ops;
+  const double R = t.R, nu = (double)t.utot / t.D, n = (double)t.nDp / t.D;
+  const double work = (double)t.T * R * R * (t.D - 1) + nu * R * n * (n + 2.0 * R);
+  const bool one = t.T * t.D <= kMoffMax && res <= (size_t)limit && work <= kOneCtaWork;
+  if (!one) return opals_grid_launch(p, st);
+  MLCP_CUDA_TRY(cudaFuncSetAttribute(opals_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)res));
+  opals_kernel<<<p.nvec, kThreads, res, st>>>(p);
   MLCP_CUDA_TRY(cudaGetLastError());
   return kOk;
 }

@@ -16,8 +16,13 @@ namespace dwsolve {
 constexpr int kSolverWarps = 4;
 constexpr int kSolverThreads = kSolverWarps * 32;
 
-// Barrier among the solver warps only (named barrier 1).
-__device__ __forceinline__ void solver_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kSolverThreads) : "memory"); }
+// Barrier among the solver warps only (named barrier 1): threads 0 .. NT-1 of
+// the block.
+template <int NT>
+__device__ __forceinline__ void team_sync() {
+  asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
+}
+__device__ __forceinline__ void solver_sync() { team_sync<kSolverThreads>(); }
 
 // In-place LDL^T of the symmetric A (lower triangle): afterwards A(i,j) =
 // L(i,j) for i > j and dinv[j] = 1/D(j).  The next pivot is formed first so
@@ -123,13 +128,14 @@ __device__ __forceinline__ dw dw_shfl_xor(dw v, int o) {
 }
 
 // dw_normalise_row for all nr rows of X (column-major, ld nr, n columns) by
-// the solver team, G lanes of one warp per row (G the largest power of two
-// <= 32 with G nr <= 128); norms to nrm[i].  The lanes of a row combine
+// threads 0 .. NT-1, G lanes of one warp per row (G the largest power of two
+// <= 32 with G nr <= NT); norms to nrm[i].  The lanes of a row combine
 // their maxima and sums of squares by butterflies, so all of them hold the
 // same norm.  Ends without a barrier.
+template <int NT = kSolverThreads>
 __device__ inline void dw_normalise_rows(dw* X, int nr, int n, dw* nrm) {
   int G = 32;
-  while (G > 1 && G * nr > kSolverThreads) G >>= 1;
+  while (G > 1 && G * nr > NT) G >>= 1;
   const int t = threadIdx.x, row = t / G, sub = t - row * G;
   const bool live = row < nr;
   dw* x = X + (live ? row : 0);
@@ -163,13 +169,14 @@ __device__ inline void dw_normalise_rows(dw* X, int nr, int n, dw* nrm) {
   if (sub == 0) nrm[row] = r;
 }
 
-// Walk over the entries e = tid, tid + 128, ... of a matrix with n rows
+// Walk over the entries e = tid, tid + NT, ... of a matrix with n rows
 // (column-major), tracking (row, column) = (e mod n, e div n) without dividing.
 struct Walk {
   int i, j, di, dj, n;
 };
+template <int NT = kSolverThreads>
 __device__ __forceinline__ Walk walk_start(int t, int n) {
-  return Walk{t % n, t / n, kSolverThreads % n, kSolverThreads / n, n};
+  return Walk{t % n, t / n, NT % n, NT / n, n};
 }
 __device__ __forceinline__ void walk_next(Walk& w) {
   w.i += w.di;
@@ -281,11 +288,131 @@ __device__ inline bool gj_inverse_warp_n(const dw* A, int n, float* inv) {
   return good;
 }
 
+// The same for n <= 16 with the rows split over the half-warps: lane (h, j)
+// holds rows 8 h .. 8 h + 7 of column j, so that a step costs half the
+// instructions (it is bound by one warp's issue); the same operations on
+// every entry, so the same bits as gj_inverse_warp_n<16>.
+__device__ inline bool gj_inverse_half(const dw* A, int n, float* inv) {
+  const int lane = threadIdx.x & 31, j = lane & 15, h = lane >> 4;
+  float a[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) a[q] = (j < n && 8 * h + q < n) ? A[8 * h + q + j * n].hi : 0.f;
+  bool good = true;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    if (k >= n) break;
+    const int kh = k >> 3, kq = k & 7;  // row k: register kq of half kh
+    const float piv = __shfl_sync(0xffffffffu, a[kq], 16 * kh + k);
+    good = good && piv > 0.f;
+    float pk = f_rcp_approx(piv);
+    pk = pk * fmaf(-piv, pk, 2.0f);
+    const float rk = __shfl_sync(0xffffffffu, a[kq], 16 * kh + j) * pk;  // row k of this column, scaled
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const float ci = __shfl_sync(0xffffffffu, a[q], 16 * h + k);  // column k, before the step
+      const float v = j == k ? -ci * pk : fmaf(-ci, rk, a[q]);
+      a[q] = q == kq && h == kh ? (j == k ? pk : rk) : v;
+    }
+  }
+  if (j < n)
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (8 * h + q < n) inv[8 * h + q + j * n] = a[q];
+  return good;
+}
+
 // Register Gauss-Jordan for n <= 32, by the calling warp.
 __device__ inline bool gj_inverse_warp(const dw* A, int n, float* inv) {
   if (n <= 8) return gj_inverse_warp_n<8>(A, n, inv);
-  if (n <= 16) return gj_inverse_warp_n<16>(A, n, inv);
+  if (n <= 16) return gj_inverse_half(A, n, inv);
   return gj_inverse_warp_n<32>(A, n, inv);
+}
+
+// The FP32 inverses above by NW warps (threads 0 .. 32 NW - 1, named barrier
+// 1) in registers: warp w holds rows w, w + NW, ... (ROWS of them), lane l
+// columns l and, when COLS is 2, l + 32.  A step's pivot row goes through
+// shared memory (row: [2][72] floats, two buffers so that a step needs one
+// barrier); a row's own multiplier is a shuffle from the pivot column's lane.
+// kColumn picks whose rounding is kept: the pivot column scaled first, as in
+// gj_inverse, or the pivot row, as in gj_inverse_warp; entries are then the
+// same bits as there.  What it replaces is bound by latency: one warp takes
+// ~15 cycles per row and step (15.7 k cycles for n = 32), four warps through
+// two shared-memory matrices ~1600 cycles per step (100 k for n = 64); this
+// takes ~200 per step with four warps at n = 32 and eight at n = 64.  Writes
+// inv (column-major, ld n); *flag (set by the caller before a barrier) becomes 0
+// when a pivot is not positive.  Ends without a barrier.
+template <int NW, int ROWS, int COLS, bool kColumn>
+__device__ inline void team_inverse(const dw* A, int n, float* inv, float* row, int* flag) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  float a[ROWS][COLS];
+#pragma unroll
+  for (int q = 0; q < ROWS; ++q)
+#pragma unroll
+    for (int c = 0; c < COLS; ++c) {
+      const int i = w + NW * q, j = lane + 32 * c;
+      a[q][c] = i < n && j < n ? A[i + j * n].hi : 0.f;
+    }
+  float* buf = row;
+#pragma unroll
+  for (int q = 0; q < ROWS; ++q) {
+    for (int wk = 0; wk < NW; ++wk) {
+      const int k = NW * q + wk;
+      if (k >= n) break;
+      const int kl = k & 31, kc = k >> 5;
+      if (w == wk) {
+        const float piv = __shfl_sync(0xffffffffu, COLS > 1 && kc ? a[q][COLS - 1] : a[q][0], kl);
+        if (!(piv > 0.f) && lane == 0) *flag = 0;
+        float pk = f_rcp_approx(piv);
+        pk = pk * fmaf(-piv, pk, 2.0f);
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) {
+          const float rk = a[q][c] * pk;
+          buf[lane + 32 * c] = kColumn ? a[q][c] : rk;
+          a[q][c] = lane + 32 * c == k ? pk : rk;
+        }
+        if (lane == 0) buf[64] = pk;
+      }
+      team_sync<32 * NW>();
+      float r[COLS];
+#pragma unroll
+      for (int c = 0; c < COLS; ++c) r[c] = buf[lane + 32 * c];
+      const float pk = buf[64];
+#pragma unroll
+      for (int p = 0; p < ROWS; ++p) {
+        const float ci = __shfl_sync(0xffffffffu, COLS > 1 && kc ? a[p][COLS - 1] : a[p][0], kl);
+        if (p == q && w == wk) continue;
+        const float cp = ci * pk;
+#pragma unroll
+        for (int c = 0; c < COLS; ++c)
+          a[p][c] = lane + 32 * c == k ? -cp : fmaf(kColumn ? -cp : -ci, r[c], a[p][c]);
+      }
+      buf = buf == row ? row + 72 : row;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < ROWS; ++q)
+#pragma unroll
+    for (int c = 0; c < COLS; ++c) {
+      const int i = w + NW * q, j = lane + 32 * c;
+      if (i < n && j < n) inv[i + j * n] = a[q][c];
+    }
+}
+
+// Warps that invert an n x n matrix (n <= 64) beside other work.
+__host__ __device__ constexpr int invert_warps(int n) { return n <= 16 ? 1 : n <= 32 ? 4 : 8; }
+
+// The inverse by threads 0 .. 32 invert_warps(n) - 1; row: [2][72] floats.
+// *flag must be 1 on entry (ordered before the call); 0 on return when a pivot
+// was not positive.
+__device__ inline void invert_any(const dw* A, int n, float* inv, float* row, int* flag) {
+  if (n <= 16) {
+    const bool good = gj_inverse_warp(A, n, inv);
+    if (threadIdx.x == 0 && !good) *flag = 0;
+  } else if (n <= 32) {
+    team_inverse<4, 8, 1, false>(A, n, inv, row, flag);
+  } else {
+    team_inverse<8, 8, 2, true>(A, n, inv, row, flag);
+  }
 }
 
 // Refinement rounds before falling back to the double-word LDL^T.
@@ -297,13 +424,16 @@ constexpr int kRefineMax = 4;
 // correction is below 1e-10 of max |X| (or the first is below 1e-5, which
 // bounds the remaining error by 1e-10).  Returns whether that happened within
 // kRefineMax rounds.  Each thread computes up to four entries in registers
-// before storing them.
+// before storing them.  Threads 0 .. NT-1; every entry is the same chain
+// whatever NT (128 where other warps work beside it, the whole block where
+// they would wait: 30 x 48 entries take ~12 us with 128 threads and ~4 with 512).
+template <int NT = kSolverThreads>
 __device__ inline bool refine_solve(const dw* A, int n, const dw* B, dw* X, int nrhs, const float* inv, dw* R, float* red) {
   const int t = threadIdx.x, nr = n * nrhs;
   // X = inv * B
   {
-    Walk w = walk_start(t, n);
-    for (int e0 = t; e0 < nr; e0 += kSolveBatch * kSolverThreads) {
+    Walk w = walk_start<NT>(t, n);
+    for (int e0 = t; e0 < nr; e0 += kSolveBatch * NT) {
       int ii[kSolveBatch], jj[kSolveBatch];
       float acc[kSolveBatch];
 #pragma unroll
@@ -316,21 +446,21 @@ __device__ inline bool refine_solve(const dw* A, int n, const dw* B, dw* X, int 
       for (int j = 0; j < n; ++j)
 #pragma unroll
         for (int q = 0; q < kSolveBatch; ++q)
-          if (e0 + q * kSolverThreads < nr) acc[q] = fmaf(inv[ii[q] + j * n], B[j + jj[q] * n].hi, acc[q]);
+          if (e0 + q * NT < nr) acc[q] = fmaf(inv[ii[q] + j * n], B[j + jj[q] * n].hi, acc[q]);
 #pragma unroll
       for (int q = 0; q < kSolveBatch; ++q)
-        if (e0 + q * kSolverThreads < nr) X[e0 + q * kSolverThreads] = dw_make(acc[q]);
+        if (e0 + q * NT < nr) X[e0 + q * NT] = dw_make(acc[q]);
     }
   }
   bool ok = false;
   for (int round = 0; round < kRefineMax && !ok; ++round) {
     float* rd = red + 2 * (round & 1);
     if (t == 0) rd[0] = rd[1] = 0.f;
-    solver_sync();
+    team_sync<NT>();
     // R = B - A X, compensated accumulation (two entries per thread)
     {
-      Walk w = walk_start(t, n);
-      for (int e0 = t; e0 < nr; e0 += 2 * kSolverThreads) {
+      Walk w = walk_start<NT>(t, n);
+      for (int e0 = t; e0 < nr; e0 += 2 * NT) {
         int ii[2], jj[2];
         dw_acc acc[2];
 #pragma unroll
@@ -338,24 +468,24 @@ __device__ inline bool refine_solve(const dw* A, int n, const dw* B, dw* X, int 
           ii[q] = w.i;
           jj[q] = w.j;
           acc[q] = acc_zero();
-          if (e0 + q * kSolverThreads < nr) acc_add(acc[q], B[e0 + q * kSolverThreads]);
+          if (e0 + q * NT < nr) acc_add(acc[q], B[e0 + q * NT]);
           walk_next(w);
         }
-        const bool two = e0 + kSolverThreads < nr;
+        const bool two = e0 + NT < nr;
         for (int j = 0; j < n; ++j) {
           acc_fma(acc[0], dw_neg(A[ii[0] + j * n]), X[j + jj[0] * n]);
           if (two) acc_fma(acc[1], dw_neg(A[ii[1] + j * n]), X[j + jj[1] * n]);
         }
         R[e0] = acc_value(acc[0]);
-        if (two) R[e0 + kSolverThreads] = acc_value(acc[1]);
+        if (two) R[e0 + NT] = acc_value(acc[1]);
       }
     }
-    solver_sync();
+    team_sync<NT>();
     // X += inv * R
     float mdx = 0.f, mx = 0.f;
     {
-      Walk w = walk_start(t, n);
-      for (int e0 = t; e0 < nr; e0 += kSolveBatch * kSolverThreads) {
+      Walk w = walk_start<NT>(t, n);
+      for (int e0 = t; e0 < nr; e0 += kSolveBatch * NT) {
         int ii[kSolveBatch], jj[kSolveBatch];
         float acc[kSolveBatch];
         dw xv[kSolveBatch];
@@ -364,18 +494,18 @@ __device__ inline bool refine_solve(const dw* A, int n, const dw* B, dw* X, int 
           ii[q] = w.i;
           jj[q] = w.j;
           acc[q] = 0.f;
-          if (e0 + q * kSolverThreads < nr) xv[q] = X[e0 + q * kSolverThreads];
+          if (e0 + q * NT < nr) xv[q] = X[e0 + q * NT];
           walk_next(w);
         }
         for (int j = 0; j < n; ++j)
 #pragma unroll
           for (int q = 0; q < kSolveBatch; ++q)
-            if (e0 + q * kSolverThreads < nr) acc[q] = fmaf(inv[ii[q] + j * n], R[j + jj[q] * n].hi, acc[q]);
+            if (e0 + q * NT < nr) acc[q] = fmaf(inv[ii[q] + j * n], R[j + jj[q] * n].hi, acc[q]);
 #pragma unroll
         for (int q = 0; q < kSolveBatch; ++q) {
-          if (e0 + q * kSolverThreads >= nr) continue;
+          if (e0 + q * NT >= nr) continue;
           const dw xn = dw_add_f(xv[q], acc[q]);
-          X[e0 + q * kSolverThreads] = xn;
+          X[e0 + q * NT] = xn;
           mdx = fmaxf(mdx, (fabsf(acc[q]) <= FLT_MAX) ? fabsf(acc[q]) : INFINITY);
           mx = fmaxf(mx, fabsf(xn.hi));
         }
@@ -384,7 +514,7 @@ __device__ inline bool refine_solve(const dw* A, int n, const dw* B, dw* X, int 
     // non-negative floats order like their bit patterns
     atomicMax(reinterpret_cast<int*>(rd), __float_as_int(mdx));
     atomicMax(reinterpret_cast<int*>(rd + 1), __float_as_int(mx));
-    solver_sync();
+    team_sync<NT>();
     // converged when the correction just applied is negligible, or when the
     // contraction it shows (rho ~ |dX|/|X|) leaves an error of rho^2 |X| <=
     // 1e-10 |X| (refinement converges linearly with rate rho), far below the
@@ -394,6 +524,119 @@ __device__ inline bool refine_solve(const dw* A, int n, const dw* B, dw* X, int 
   return ok;
 }
 
+
+// refine_solve with the entries of a thread fixed at compile time: NQ of them
+// (NT NQ >= n nrhs), the right-hand sides in registers, the products over j
+// unrolled by four so that their shared-memory loads are in flight together.
+// Every entry is the same chain as in refine_solve, and the maxima that
+// decide convergence are the same numbers: the same bits.  Rh: [n nrhs]
+// floats (the corrections read the residuals' high parts only).
+template <int NT, int NQ>
+__device__ inline bool refine_solve_q(const dw* __restrict__ A, int n, const dw* __restrict__ B, dw* X, int nrhs,
+                                      const float* __restrict__ inv, float* Rh, float* red) {
+  const int t = threadIdx.x, nr = n * nrhs;
+  int i[NQ], mo[NQ];  // row, offset of the column
+  dw b[NQ], x[NQ];
+  {
+    Walk w = walk_start<NT>(t, n);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      const bool live = t + q * NT < nr;
+      i[q] = live ? w.i : 0;
+      mo[q] = live ? w.j * n : 0;
+      walk_next(w);
+      b[q] = B[live ? t + q * NT : 0];
+    }
+  }
+  // acc[q] = sum_j inv(i, j) v(j), v the high parts of column mo[q] of a dw
+  // matrix (stride 2 floats) or a float matrix (stride 1)
+  auto apply = [&](const float* v, int stride, float(&acc)[NQ]) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) acc[q] = 0.f;
+    int j = 0;
+    for (; j + 4 <= n; j += 4)
+#pragma unroll
+      for (int q = 0; q < NQ; ++q)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[q] = fmaf(inv[i[q] + (j + u) * n], v[(j + u + mo[q]) * stride], acc[q]);
+    for (; j < n; ++j)
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) acc[q] = fmaf(inv[i[q] + j * n], v[(j + mo[q]) * stride], acc[q]);
+  };
+  {
+    float acc[NQ];
+    apply(reinterpret_cast<const float*>(B), 2, acc);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      x[q] = dw_make(acc[q]);
+      if (t + q * NT < nr) X[t + q * NT] = x[q];
+    }
+  }
+  bool ok = false;
+  for (int round = 0; round < kRefineMax && !ok; ++round) {
+    float* rd = red + 2 * (round & 1);
+    if (t == 0) rd[0] = rd[1] = 0.f;
+    team_sync<NT>();
+    {  // residuals B - A X, compensated
+      dw_acc acc[NQ];
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        acc[q] = acc_zero();
+        acc_add(acc[q], b[q]);
+      }
+      int j = 0;
+      for (; j + 4 <= n; j += 4)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) acc_fma(acc[q], dw_neg(A[i[q] + (j + u) * n]), X[j + u + mo[q]]);
+      for (; j < n; ++j)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) acc_fma(acc[q], dw_neg(A[i[q] + j * n]), X[j + mo[q]]);
+#pragma unroll
+      for (int q = 0; q < NQ; ++q)
+        if (t + q * NT < nr) Rh[t + q * NT] = acc_value(acc[q]).hi;
+    }
+    team_sync<NT>();
+    float d[NQ], mdx = 0.f, mx = 0.f;
+    apply(Rh, 1, d);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      if (t + q * NT >= nr) continue;
+      x[q] = dw_add_f(x[q], d[q]);
+      X[t + q * NT] = x[q];
+      mdx = fmaxf(mdx, (fabsf(d[q]) <= FLT_MAX) ? fabsf(d[q]) : INFINITY);
+      mx = fmaxf(mx, fabsf(x[q].hi));
+    }
+    // non-negative floats order like their bit patterns
+    const int wd = __reduce_max_sync(0xffffffffu, __float_as_int(mdx)),
+              wx = __reduce_max_sync(0xffffffffu, __float_as_int(mx));
+    if ((t & 31) == 0) {
+      atomicMax(reinterpret_cast<int*>(rd), wd);
+      atomicMax(reinterpret_cast<int*>(rd + 1), wx);
+    }
+    team_sync<NT>();
+    // the convergence rule of refine_solve
+    ok = rd[0] <= 1e-10f * rd[1] || (round == 0 && rd[0] <= 1e-5f * rd[1]);
+  }
+  return ok;
+}
+
+// refine_solve by threads 0 .. NT-1 for n, nrhs <= 64 (res: [n nrhs] dw).  The
+// Gram-Schmidt of a 3 x 30 node (40 vectors, rank 16, 234 solves of 16 x 30
+// entries) takes 4.57 ms with refine_solve<512>, whose entries are found at run
+// time with an atomic per thread, and 4.00 with refine_solve_q.
+template <int NT>
+__device__ inline bool refine_any(const dw* A, int n, const dw* B, dw* X, int nrhs, const float* inv, dw* res,
+                                  float* red) {
+  const int nr = n * nrhs;
+  float* Rh = reinterpret_cast<float*>(res);
+  if (nr <= NT) return refine_solve_q<NT, 1>(A, n, B, X, nrhs, inv, Rh, red);
+  if (nr <= 2 * NT) return refine_solve_q<NT, 2>(A, n, B, X, nrhs, inv, Rh, red);
+  if (nr <= 4 * NT) return refine_solve_q<NT, 4>(A, n, B, X, nrhs, inv, Rh, red);
+  if (nr <= 8 * NT) return refine_solve_q<NT, 8>(A, n, B, X, nrhs, inv, Rh, red);
+  return refine_solve<NT>(A, n, B, X, nrhs, inv, res, red);
+}
 
 __device__ __forceinline__ dw dw_shfl(dw v, int src) {
   return dw{__shfl_sync(0xffffffffu, v.hi, src), __shfl_sync(0xffffffffu, v.lo, src)};

@@ -68,7 +68,7 @@ struct GsArrays {
                                // and over d not in {j, next mode}; [nkmax+1][2][R*npm] partial dot products
   dw *fb, *g;              // [R][nD] vector being fitted; [D][R*R] its Grams
   dw *fcs, *wf, *Gp, *pGp, *BB, *gpart, *gco, *bpart, *X, *b0, *res, *dinv, *u, *red, *misc;
-  float *gi, *rred;
+  float *gi, *rred, *prow;  // prow: [2][72] pivot rows of the inverse
   dwsolve::ColScratch cs;
   int *nb, *off, *flags;
   FastDiv* fd;  // divisors of the step's index splits: R, R*R, RRp, then R*n_d per mode
@@ -123,6 +123,7 @@ __host__ __device__ inline size_t gs_carve(const GsDims& m, GsArrays* a, unsigne
   a->misc = (dw*)take_s(sizeof(dw) * 4);
   a->gi = (float*)take_s(sizeof(float) * 2 * RR);
   a->rred = (float*)take_s(sizeof(float) * 4);
+  a->prow = (float*)take_s(sizeof(float) * 2 * 72);
   a->cs.conv = (float*)take_s(sizeof(float) * 64);
   a->cs.rmax = (float*)take_s(sizeof(float) * 16 * 32);
   a->cs.rsum = (dw*)take_s(sizeof(dw) * 16 * 32);
@@ -137,8 +138,6 @@ __host__ __device__ inline size_t gs_carve(const GsDims& m, GsArrays* a, unsigne
 __device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-// Threads outside the solver team (warps 4-15).
-constexpr int kWorkerThreads = kGsThreads - dwsolve::kSolverThreads;
 // Barrier of the threads w0..511 (named barrier 2).
 __device__ __forceinline__ void worker_sync(int w0) {
   asm volatile("bar.sync 2, %0;" ::"r"(kGsThreads - w0) : "memory");
@@ -449,18 +448,21 @@ __device__ void step_grid_sum(const Gs& c, const GsParams& p, int j, int step, c
   __syncthreads();
 }
 
-// Step phase 5 (solver warps): X = BB^-1 b0 from the FP32 inverse formed
-// during phases 2-4, rows normalised, norms as the new weights.
+// Step phase 5 (every thread): X = BB^-1 b0 from the FP32 inverse formed
+// during phases 2-4 (the solver warps' LDL^T when that fails), rows
+// normalised, norms as the new weights.  Ends without a barrier.
 __device__ void step_solve(const Gs& c, int j, const float* inv, bool gj_ok) {
   const int R = c.R, nj = c.a.nb[j];
-  int bad = 0;
-  if (!(gj_ok && dwsolve::refine_solve(c.a.BB, R, c.a.b0, c.a.X, nj, inv, c.a.res, c.a.rred))) {
-    for (int e = c.tid; e < R * nj; e += dwsolve::kSolverThreads) c.a.X[e] = c.a.b0[e];
-    bad = dwsolve::dw_ldlt(c.a.BB, R, c.a.dinv, c.a.u);
-    dwsolve::dw_ldlt_solve(c.a.BB, R, c.a.dinv, c.a.X, nj);
+  if (!(gj_ok && dwsolve::refine_any<kGsThreads>(c.a.BB, R, c.a.b0, c.a.X, nj, inv, c.a.res, c.a.rred))) {
+    if (c.tid < dwsolve::kSolverThreads) {
+      for (int e = c.tid; e < R * nj; e += dwsolve::kSolverThreads) c.a.X[e] = c.a.b0[e];
+      const int bad = dwsolve::dw_ldlt(c.a.BB, R, c.a.dinv, c.a.u);
+      dwsolve::dw_ldlt_solve(c.a.BB, R, c.a.dinv, c.a.X, nj);
+      if (c.tid == 0 && bad) c.a.flags[1] = 1;
+    }
+    __syncthreads();
   }
-  dwsolve::dw_normalise_rows(c.a.X, R, nj, c.a.fcs);
-  if (c.tid == 0 && bad) c.a.flags[1] = 1;
+  dwsolve::dw_normalise_rows<kGsThreads>(c.a.X, R, nj, c.a.fcs);
 }
 
 // When another step of this vector follows (mode jn): the products over d
@@ -571,7 +573,10 @@ __global__ void __launch_bounds__(kGsThreads, 1) gs_kernel(GsParams p) {
   }
   for (int q = c.tid; q < c.D + 3; q += kGsThreads)
     c.a.fd[q] = FastDiv((unsigned)(q == 0 ? c.R : q == 1 ? c.RR : q == 2 ? c.RRp : c.R * p.nbas[q - 3]));
-  if (c.tid == 0) c.a.flags[1] = 0;
+  if (c.tid == 0) {
+    c.a.flags[1] = 0;
+    c.a.flags[2] = 1;
+  }
   __syncthreads();
 
   load_vector(c, p, 0);
@@ -593,24 +598,15 @@ __global__ void __launch_bounds__(kGsThreads, 1) gs_kernel(GsParams p) {
         dw* bp = c.a.bpart + (size_t)(step & 1) * c.R * c.npm;
         const bool more = it + 1 < p.nals || j + 1 < c.D;  // another step of this vector follows
         const int jn = j + 1 < c.D ? j + 1 : 0, nj = c.a.nb[j];
-        // FP32 inverse of BB (warp 0 in registers for R <= 32, else the
-        // solver warps) concurrently with the right-hand side (threads w0..);
-        // when the previous update already formed BB, also concurrently with
-        // the products
-        bool gj_ok = false;
-        const float* inv = c.a.gi;
-        const int w0 = c.R <= 32 ? 32 : dwsolve::kSolverThreads;
-        const bool early = pre && c.R <= 32;
-        if (!early) step_products(c, j, nk, pre, 0, qinv);
+        // FP32 inverse of BB (the first invert_warps(R) warps) concurrently
+        // with the right-hand side (threads w0..); when the previous update
+        // already formed BB, also concurrently with the products
+        const int w0 = 32 * dwsolve::invert_warps(c.R);
+        if (!pre) step_products(c, j, nk, pre, 0, qinv);
         if (c.tid < w0) {
-          if (c.R > 32) {
-            inv = dwsolve::gj_inverse(c.a.BB, c.R, c.a.gi, &gj_ok);
-          } else {
-            const bool good = dwsolve::gj_inverse_warp(c.a.BB, c.R, c.a.gi);
-            if (c.tid == 0) c.a.flags[2] = good;
-          }
+          dwsolve::invert_any(c.a.BB, c.R, c.a.gi, c.a.prow, c.a.flags + 2);
         } else {
-          if (early) step_products(c, j, nk, pre, w0, qinv);
+          if (pre) step_products(c, j, nk, pre, w0, qinv);
           step_dots(c, j, nk, w0);
           step_rhs_part(c, j, nk, bp, w0);
         }
@@ -629,18 +625,18 @@ __global__ void __launch_bounds__(kGsThreads, 1) gs_kernel(GsParams p) {
             step_grid_sum(c, p, j, step, xs);
           }
         }
-        if (c.R <= 32) gj_ok = c.a.flags[2] != 0;
+        bool gj_ok = c.a.flags[2] != 0;
         // the solve: refinement in registers (warps 0..nsw-1, one or two
-        // right-hand-side columns each), or the solver warps' refinement /
-        // LDL^T fallback; the next step's partial products on the other warps
+        // right-hand-side columns each) with the next step's partial products
+        // on the other warps, or the whole block's refinement / LDL^T
         bool solved = false, pre_done = !more;
         if (gj_ok && c.R <= 32 && nj <= 16) {
           // rank <= 16: one column per warp, sums split over the half-warps
           const bool split = c.R <= 16;
           const int nsw = (split ? nj : dwsolve::solve_cols_warps(c.R, nj)) * 32;
           if (c.tid < nsw) {
-            const bool ok = split ? dwsolve::solve_cols_split(c.a.BB, c.R, c.a.b0, c.a.X, nj, inv, c.a.fcs, c.a.cs)
-                                  : dwsolve::solve_cols_any(c.a.BB, c.R, c.a.b0, c.a.X, nj, inv, c.a.fcs, c.a.cs);
+            const bool ok = split ? dwsolve::solve_cols_split(c.a.BB, c.R, c.a.b0, c.a.X, nj, c.a.gi, c.a.fcs, c.a.cs)
+                                  : dwsolve::solve_cols_any(c.a.BB, c.R, c.a.b0, c.a.X, nj, c.a.gi, c.a.fcs, c.a.cs);
             if (c.tid == 0) c.a.flags[3] = ok;
           } else if (more) {
             step_preproducts(c, j, jn, nk, c.tid - nsw, kGsThreads - nsw);
@@ -650,16 +646,10 @@ __global__ void __launch_bounds__(kGsThreads, 1) gs_kernel(GsParams p) {
           pre_done = pre_done || nsw < kGsThreads;
           gj_ok = false;  // not converged: straight to the LDL^T
         }
-        if (!solved) {
-          if (c.tid < dwsolve::kSolverThreads) step_solve(c, j, inv, gj_ok);
-          else if (!pre_done) step_preproducts(c, j, jn, nk, c.tid - dwsolve::kSolverThreads, kWorkerThreads);
-          __syncthreads();
-          pre_done = true;
-        }
-        if (!pre_done) {
-          step_preproducts(c, j, jn, nk, c.tid, kGsThreads);
-          __syncthreads();
-        }
+        if (!solved) step_solve(c, j, c.a.gi, gj_ok);
+        if (!pre_done) step_preproducts(c, j, jn, nk, c.tid, kGsThreads);
+        if (!solved || !pre_done) __syncthreads();
+        if (c.tid == 0) c.a.flags[2] = 1;
         if (c.rv < c.R) {  // ragged: the padded terms keep zero weight
           for (int i = c.rv + c.tid; i < c.R; i += kGsThreads) c.a.fcs[i] = dw_make(0.f);
           __syncthreads();

@@ -240,9 +240,12 @@ __global__ void __launch_bounds__(kSolveThreads, 1) og_solve_kernel(OpAlsParams 
   og_carve(t, p.nvec, p.gscr, &s);
   for (int e = threadIdx.x; e < RR; e += kSolveThreads) m.BB[e] = s.bb[(size_t)v * RR + e];
   for (int e = threadIdx.x; e < R * nj; e += kSolveThreads) m.b0[e] = s.b0[(size_t)v * R * npm + e];
-  if (threadIdx.x == 0) m.flags[1] = 0;
+  if (threadIdx.x == 0) {
+    m.flags[0] = m.flags[1] = 0;
+    m.flags[2] = 1;
+  }
   __syncthreads();
-  step_invert(m, R);
+  if (threadIdx.x < 32 * dwsolve::invert_warps(R)) dwsolve::invert_any(m.BB, R, m.gi, m.prow, m.flags + 2);
   __syncthreads();
   step_solve(m, R, nj);
   const int rv = p.rank_v ? p.rank_v[v] : R;

@@ -26,6 +26,7 @@ struct StepSmem {
   dw* u;      // [R] LDL^T scratch column
   dw* misc;   // [2] penalty, norm
   float* rred;  // [4] refinement scratch
+  float* prow;  // [2][72] pivot rows of the inverse
   dwsolve::ColScratch cs;
   int* flags;  // [4] [0] buffer of the inverse, [1] non-positive pivot seen, [2] inverse usable, [3] solved
 };
@@ -50,6 +51,7 @@ __host__ __device__ inline size_t step_carve(StepSmem& s, unsigned char* base, i
   s.u = (dw*)take(sizeof(dw) * R);
   s.misc = (dw*)take(sizeof(dw) * 2);
   s.rred = (float*)take(sizeof(float) * 4);
+  s.prow = (float*)take(sizeof(float) * 2 * 72);
   s.cs.conv = (float*)take(sizeof(float) * 64);
   s.cs.rmax = (float*)take(sizeof(float) * 16 * 32);
   s.cs.rsum = (dw*)take(sizeof(dw) * 16 * 32);
@@ -93,6 +95,7 @@ __device__ inline void step_invert(const StepSmem& s, int R) {
 }
 
 // X = BB^-1 b0 with unit rows, their norms to cf; ends with a block barrier.
+// (Norms by 128 threads: their partial sums depend on how many share a row.)
 __device__ inline void step_solve(const StepSmem& s, int R, int nj) {
   bool gj_ok = s.flags[2] != 0;
   const float* inv = s.gi + (size_t)s.flags[0] * R * R;
@@ -108,16 +111,16 @@ __device__ inline void step_solve(const StepSmem& s, int R, int nj) {
     gj_ok = false;  // not converged: straight to the LDL^T
   }
   if (!solved) {
-    if (threadIdx.x < dwsolve::kSolverThreads) {
-      int bad = 0;
-      if (!(gj_ok && dwsolve::refine_solve(s.BB, R, s.b0, s.X, nj, inv, s.res, s.rred))) {
+    if (!(gj_ok && dwsolve::refine_any<kStepThreads>(s.BB, R, s.b0, s.X, nj, inv, s.res, s.rred))) {
+      if (threadIdx.x < dwsolve::kSolverThreads) {
         for (int e = threadIdx.x; e < R * nj; e += dwsolve::kSolverThreads) s.X[e] = s.b0[e];
-        bad = dwsolve::dw_ldlt(s.BB, R, s.dinv, s.u);
+        const int bad = dwsolve::dw_ldlt(s.BB, R, s.dinv, s.u);
         dwsolve::dw_ldlt_solve(s.BB, R, s.dinv, s.X, nj);
+        if (threadIdx.x == 0 && bad) s.flags[1] = 1;
       }
-      dwsolve::dw_normalise_rows(s.X, R, nj, s.cf);
-      if (threadIdx.x == 0 && bad) s.flags[1] = 1;
+      __syncthreads();
     }
+    if (threadIdx.x < dwsolve::kSolverThreads) dwsolve::dw_normalise_rows(s.X, R, nj, s.cf);
     __syncthreads();
   }
 }

@@ -63,6 +63,7 @@ struct UpdSmem {
   dw* misc;   // [2] penalty, norm
   dw* red;    // [kWarps]
   float* rred;
+  float* prow;  // [2][72] pivot rows of the inverse
   dwsolve::ColScratch cs;
   dw* P;      // [R][TL] products of one tile of block terms
   dw* Qt;     // [TL][npmax] mode-k factors of the tile
@@ -93,6 +94,7 @@ __host__ __device__ inline size_t upd_carve(UpdSmem& s, unsigned char* base, int
   s.misc = (dw*)take(sizeof(dw) * 2);
   s.red = (dw*)take(sizeof(dw) * kWarps);
   s.rred = (float*)take(sizeof(float) * 4);
+  s.prow = (float*)take(sizeof(float) * 2 * 72);
   s.cs.conv = (float*)take(sizeof(float) * 64);
   s.cs.rmax = (float*)take(sizeof(float) * 16 * 32);
   s.cs.rsum = (dw*)take(sizeof(dw) * 16 * 32);
@@ -173,6 +175,7 @@ __global__ void __launch_bounds__(kThreads, 1) upd_kernel(UpdParams p) {
     for (int r = 1; r < R; ++r) pen = p.qc[(size_t)i * R + r] > pen ? p.qc[(size_t)i * R + r] : pen;
     s.misc[0] = dw_from_double(pen * p.pen_factor);
     s.flags[1] = 0;
+    s.flags[2] = 1;
   }
   for (int d = 0; d < D; ++d) {
     const int nd = p.nbas[d], od = p.off[d];
@@ -211,22 +214,9 @@ __global__ void __launch_bounds__(kThreads, 1) upd_kernel(UpdParams p) {
         s.BB[e] = bb;
       }
       __syncthreads();
-      const int w0 = R <= 32 ? 32 : dwsolve::kSolverThreads;
+      const int w0 = 32 * dwsolve::invert_warps(R);
       if (threadIdx.x < w0) {
-        if (R <= 32) {
-          const bool g = dwsolve::gj_inverse_warp(s.BB, R, s.gi);
-          if (threadIdx.x == 0) {
-            s.flags[2] = g;
-            s.flags[0] = 0;
-          }
-        } else {
-          bool ok2;
-          const float* iv = dwsolve::gj_inverse(s.BB, R, s.gi, &ok2);
-          if (threadIdx.x == 0) {
-            s.flags[2] = ok2;
-            s.flags[0] = iv == s.gi ? 0 : 1;
-          }
-        }
+        dwsolve::invert_any(s.BB, R, s.gi, s.prow, s.flags + 2);
       } else {
         // -- this CTA's part of the right-hand side, tile by tile over its block terms --
         const int wt = threadIdx.x - w0, nw = kThreads - w0;
@@ -299,12 +289,11 @@ __global__ void __launch_bounds__(kThreads, 1) upd_kernel(UpdParams p) {
       __syncthreads();
       // -- solve (as in the power sweep) --
       bool gj_ok = s.flags[2] != 0;
-      const float* inv = s.gi + (size_t)s.flags[0] * RR;
       bool solved = false;
       const int nsw = dwsolve::solve_cols_warps(R, nk);
       if (gj_ok && R <= 32 && nk <= 16 && nsw <= kWarps) {
         if (threadIdx.x < nsw * 32) {
-          const bool ok2 = dwsolve::solve_cols_any(s.BB, R, s.b0, s.X, nk, inv, s.cf, s.cs);
+          const bool ok2 = dwsolve::solve_cols_any(s.BB, R, s.b0, s.X, nk, s.gi, s.cf, s.cs);
           if (threadIdx.x == 0) s.flags[3] = ok2;
         }
         __syncthreads();
@@ -312,18 +301,19 @@ __global__ void __launch_bounds__(kThreads, 1) upd_kernel(UpdParams p) {
         gj_ok = false;
       }
       if (!solved) {
-        if (threadIdx.x < dwsolve::kSolverThreads) {
-          int bad = 0;
-          if (!(gj_ok && dwsolve::refine_solve(s.BB, R, s.b0, s.X, nk, inv, s.res, s.rred))) {
+        if (!(gj_ok && dwsolve::refine_any<kThreads>(s.BB, R, s.b0, s.X, nk, s.gi, s.res, s.rred))) {
+          if (threadIdx.x < dwsolve::kSolverThreads) {
             for (int e = threadIdx.x; e < R * nk; e += dwsolve::kSolverThreads) s.X[e] = s.b0[e];
-            bad = dwsolve::dw_ldlt(s.BB, R, s.dinv, s.u);
+            const int bad = dwsolve::dw_ldlt(s.BB, R, s.dinv, s.u);
             dwsolve::dw_ldlt_solve(s.BB, R, s.dinv, s.X, nk);
+            if (threadIdx.x == 0 && bad) s.flags[1] = 1;
           }
-          dwsolve::dw_normalise_rows(s.X, R, nk, s.cf);
-          if (threadIdx.x == 0 && bad) s.flags[1] = 1;
+          __syncthreads();
         }
+        dwsolve::dw_normalise_rows<kThreads>(s.X, R, nk, s.cf);
         __syncthreads();
       }
+      if (threadIdx.x == 0) s.flags[2] = 1;
       for (int r = rv + threadIdx.x; r < R; r += kThreads) s.cf[r] = dw_make(0.f);  // ragged: weightless padding
       // -- the new factor: FP64 output (rank 0), its Gram, the own block overlaps of mode k --
       if (rank == 0)

@@ -844,5 +844,140 @@ __device__ inline bool solve_cols_split(const dw* A, int n, const dw* B, dw* X, 
   return true;
 }
 
+
+// ---------------------------------------------------------------------------
+// Systems of up to 16 rows by a dense double-word inverse
+// ---------------------------------------------------------------------------
+constexpr int kRowRank = 16;
+
+// Sum over `lanes` (a power of two) neighbouring lanes, in all of them: compensated
+// pairs merged without normalising in between (half the chain of dw_add).
+template <int lanes>
+__device__ __forceinline__ dw lane_sum(dw v) {
+  dw_acc a{v.hi, v.lo};
+#pragma unroll
+  for (int o = lanes / 2; o > 0; o >>= 1)
+    a = acc_merge(a, dw_acc{__shfl_xor_sync(0xffffffffu, a.s, o), __shfl_xor_sync(0xffffffffu, a.c, o)});
+  return acc_value(a);
+}
+
+// One correction of correct_inverse: *big = n max |I - Iv A| before it.
+template <int RT, bool kFirst>
+__device__ __forceinline__ bool correct_round(const dw* A, int n_, const float* gi, dw* Iv, float* Ef, float* emax,
+                                              float* big) {
+  constexpr int NE = kRowRank * kRowRank / kSolverThreads;
+  const int n = RT ? RT : n_, nn = n * n, t = threadIdx.x, lane = t & 31;
+  int i[NE], k[NE];
+  dw_acc acc[NE];
+#pragma unroll
+  for (int q = 0; q < NE; ++q) {
+    const int p = t + q * kSolverThreads, pl = p < nn ? p : 0;
+    k[q] = (unsigned)pl / (unsigned)n;
+    i[q] = pl - k[q] * n;
+    acc[q] = dw_acc{i[q] == k[q] ? 1.f : 0.f, 0.f};
+  }
+#pragma unroll 4
+  for (int l = 0; l < n; ++l)
+#pragma unroll
+    for (int q = 0; q < NE; ++q) {
+      const dw v = kFirst ? dw_make(-gi[i[q] + l * n]) : dw_neg(Iv[i[q] + l * n]);
+      acc_fma(acc[q], v, A[l + k[q] * n]);
+    }
+  int mx = 0;  // non-negative floats order like their bit patterns, NaN above all
+#pragma unroll
+  for (int q = 0; q < NE; ++q) {
+    const float ev = acc_value(acc[q]).hi;
+    if (t + q * kSolverThreads < nn) Ef[i[q] + k[q] * n] = ev;
+    mx = max(mx, __float_as_int(fabsf(ev)));
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if (lane == 0) emax[t >> 5] = __int_as_float(mx);
+  solver_sync();
+  *big = n * __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(emax[lane & (kSolverWarps - 1)])));
+  if (!(*big <= (kFirst ? 3e-3f : 1e-5f))) return false;
+  float d[NE] = {};
+#pragma unroll 4
+  for (int l = 0; l < n; ++l)
+#pragma unroll
+    for (int q = 0; q < NE; ++q) d[q] = fmaf(Ef[i[q] + l * n], kFirst ? gi[l + k[q] * n] : Iv[l + k[q] * n].hi, d[q]);
+  dw v[NE];
+#pragma unroll
+  for (int q = 0; q < NE; ++q) v[q] = dw_add_f(kFirst ? dw_make(gi[i[q] + k[q] * n]) : Iv[i[q] + k[q] * n], d[q]);
+  if (!kFirst) solver_sync();
+#pragma unroll
+  for (int q = 0; q < NE; ++q)
+    if (t + q * kSolverThreads < nn) Iv[i[q] + k[q] * n] = v[q];
+  return true;
+}
+
+// Iv = A^-1 in double-word (threads 0 .. 127, n <= 16; RT: n when known at compile
+// time, else 0): the FP32 inverse gi corrected by Iv += (I - Iv A) Iv (Schulz's iteration, the
+// residual in double-word) until n max |I - Iv A| was at most 1e-5 before a
+// correction, so 1e-10 after it (what refine_solve reaches for its right-hand sides), in
+// two corrections at most; false when that does not suffice.  The left residual is taken
+// so that a solution Iv b has an error of (residual)^2 |x| and (rounding) cond |x|.
+// Ef: [n n], emax: [4] floats.  Ends without a barrier.
+template <int RT>
+__device__ inline bool correct_inverse(const dw* A, int n, const float* gi, dw* Iv, float* Ef, float* emax) {
+  float big;
+  if (!correct_round<RT, true>(A, n, gi, Iv, Ef, emax, &big)) return false;
+  if (big <= 1e-5f) return true;
+  solver_sync();
+  return correct_round<RT, false>(A, n, gi, Iv, Ef, emax, &big);
+}
+
+// A row of X = Iv B by one warp: iv points at the row (entries ld apart), B is [n][nj].
+// NC columns per lane, or (NC = 0, nj <= 16) one column with its sum split over the
+// half-warps; columns beyond nj are 0.  Without `solved` the row is read from xr (entries
+// ld apart) instead.
+template <int RT, int NC>
+__device__ __forceinline__ void row_product(const dw* iv, int ld, const dw* B, int nj, bool solved, const dw* xr, dw* x) {
+  constexpr bool split = NC == 0;
+  const int lane = threadIdx.x & 31, h = split ? lane >> 4 : 0, m0 = split ? lane & 15 : lane;
+#pragma unroll
+  for (int q = 0; q < (split ? 1 : NC); ++q) {
+    const int m = m0 + 32 * q, ml = m < nj ? m : 0;
+    if (solved) {
+      dw_acc acc = acc_zero();
+#pragma unroll
+      for (int u = 0; u < (split ? kRowRank / 2 : kRowRank); ++u) {
+        const int k = h * (kRowRank / 2) + u;
+        if (RT == kRowRank || k < ld) acc_fma(acc, iv[k * ld], B[k * nj + ml]);
+      }
+      if (split)
+        acc = acc_merge(acc, dw_acc{__shfl_xor_sync(0xffffffffu, acc.s, 16), __shfl_xor_sync(0xffffffffu, acc.c, 16)});
+      x[q] = m < nj ? acc_value(acc) : dw_make(0.f);
+    } else {
+      x[q] = m < nj ? xr[m * ld] : dw_make(0.f);
+    }
+  }
+}
+
+// The row (as row_product leaves it) scaled to unit norm, its norm to *nrm.  Scaled by a
+// power of two first, as normonebase scales by the largest entry; a zero row gives
+// NaN, as there.
+template <int NC>
+__device__ __forceinline__ void row_normalise(dw* x, dw* nrm) {
+  constexpr int N = NC == 0 ? 1 : NC;
+  float big = 0.f;
+#pragma unroll
+  for (int q = 0; q < N; ++q) big = fmaxf(big, fabsf(x[q].hi));
+  const int bits = __reduce_max_sync(0xffffffffu, __float_as_int(big)), ex = bits >> 23;
+  const bool scaled = ex > 0 && ex < 254;
+  const float sc = scaled ? __int_as_float((254 - ex) << 23) : 1.f, back = scaled ? __int_as_float(ex << 23) : 1.f;
+  dw_acc sq = acc_zero();
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    x[q] = dw_make(x[q].hi * sc, x[q].lo * sc);
+    acc_fma(sq, x[q], x[q]);
+  }
+  const dw sum = NC == 0 ? lane_sum<16>(acc_value(sq)) : lane_sum<32>(acc_value(sq));
+  dw r = dw_sqrt(sum), rcp = dw_rcp(r);
+  if (!(bits > 0 && sum.hi > 0.f)) r = rcp = dw_make(__int_as_float(0x7fffffff));
+#pragma unroll
+  for (int q = 0; q < N; ++q) x[q] = dw_mul(x[q], rcp);
+  *nrm = dw_make(r.hi * back, r.lo * back);
+}
+
 }  // namespace dwsolve
 }  // namespace mlcp

@@ -19,15 +19,37 @@
 // refinement, falling back to a double-word LDL^T (dwsolve.cuh).
 //
 // GB300 layout: the loop over vectors is sequential, but within a mode step
-// the work over the earlier vectors k is independent.  One thread-block
-// cluster of up to 16 CTAs runs the whole orthogonalisation in one launch;
-// CTA `rank` owns the earlier vectors k = rank (mod cluster) and keeps their
-// factors, weights and overlaps resident in its shared memory (its global
-// scratch when they do not fit).  Each CTA computes its vectors' products,
-// coefficients and right-hand-side contributions; the partial right-hand
-// sides meet through distributed shared memory, and every CTA runs the same
-// small solve on the same data, so each holds the identical new factor and
-// nothing is broadcast back.  One cluster barrier per mode step.
+// the work over the earlier vectors k is independent.  For ranks up to 16 one
+// thread-block cluster of up to 16 CTAs runs the whole orthogonalisation in one
+// launch; CTA `rank` owns the earlier vectors k = rank (mod cluster) and keeps
+// their factors, weights and overlaps resident in its shared memory (blocks
+// that do not fit and larger ranks take the grid form, gs_grid.cu).  Each CTA
+// forms its vectors' part of the right-hand side and stores it into every peer
+// through distributed shared memory; every CTA then runs the same small solve
+// on the same data, so each holds the identical new factor and nothing is
+// broadcast back.
+//
+// What bounds it is the latency of a mode step's chain, so the step is arranged
+// to keep that short:
+//   - the new factor X of mode j is solved a row per warp, its norm taken there;
+//   - its Gram gives the next normal equations BB; warp 0 inverts BB in FP32 as
+//     soon as eight warps have written it, while the other fifteen refresh the
+//     overlaps (with the next mode's products, and the coefficients <Q_k, F> from
+//     those), form the right-hand side and exchange it;
+//   - the FP32 inverse is then corrected once (twice if need be) by
+//     Inv += (I - Inv BB) Inv with the residual in double-word (Schulz's
+//     iteration), which leaves one product per right-hand side to the solve
+//     instead of refinement rounds on it.  The left residual is used: the error of
+//     X is then of the size (residual)^2 |X| and (rounding) cond |X|, as for
+//     the refinement;
+//   - the weights enter every step linearly, so they are rescaled by a power of
+//     two only (exact) and divided by |F| once per vector.
+// A mode step of rank 16 and 10 basis functions (6 modes) takes 5.7 us in a block of 40 vectors
+// and 7.3 us in one of 100 (8.4 and 10.7 us with the weights normalised, the solve refined per
+// right-hand side and the parts fetched from the peers); its issue slots alone, at the ~19
+// of a double-word term with its two loads, are about 2 us.  Ranks above 16 have solves and inverses
+// too long for one CTA: a step of rank 24, two modes of 24, takes 23.4 us in the grid
+// form and took 42.5 here; rank 30 and 8 vectors, six modes of 8, 13.3 and 23.5.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -52,96 +74,83 @@ namespace {
 
 constexpr int kGsThreads = 512;
 constexpr int kGsWarps = kGsThreads / 32;
-static_assert(kGsWarps == 16, "block_sum reduces 16 warp partials");
-
-// Groups of arrays that move to global scratch (in this order) when shared
-// memory cannot hold them.
-enum : int { kGroupQ = 1, kGroupP = 2, kGroupF = 4, kGroupAll = 7 };
+constexpr int kGsInvert = dwsolve::kSolverThreads;        // warps 0..3: the inverse
+constexpr int kGsWorkers = kGsThreads - kGsInvert;         // warps 4..15: the right-hand side
+constexpr int kGsWorkerWarps = kGsWorkers / 32;
+constexpr int kGsRank = dwsolve::kRowRank;  // ranks of this form: a row of the solve per warp
+static_assert(kGsRank <= kGsWarps && 2 * kGsRank * kGsRank <= kGsThreads, "rows and entry halves of a step");
 
 struct GsDims {
-  int R, D, nD, npm, nkmax, gmask;
+  int R, D, nD, npm, nkmax, cl, level;
 };
 
 struct GsArrays {
-  dw *qf, *qw, *qc;        // [nkmax][R][nD] owned vectors' factors, the same times their weights; [nkmax][R] weights
-  dw *P, *psn, *ppsn, *part;  // [nkmax][D][R*R] overlaps (index r*R+i); [nkmax][R*R] products over d != j,
-                               // and over d not in {j, next mode}; [nkmax+1][2][R*npm] partial dot products
-  dw *fb, *g;              // [R][nD] vector being fitted; [D][R*R] its Grams
-  dw *fcs, *wf, *Gp, *pGp, *BB, *gpart, *gco, *bpart, *X, *b0, *res, *dinv, *u, *red, *misc;
-  float *gi, *rred, *prow;  // prow: [2][72] pivot rows of the inverse
-  dwsolve::ColScratch cs;
-  int *nb, *off, *flags;
-  FastDiv* fd;  // divisors of the step's index splits: R, R*R, RRp, then R*n_d per mode
+  dw *qf, *qc;    // [nkmax][R][ld] owned vectors' factors; [nkmax][R] their weights
+  // Overlaps (index r*R+i).  P [nkmax][D][R*R]: before step j the products over d' >= d of
+  // the old overlaps for d > j, the new overlaps of mode d for d < j; lead [nkmax][R*R]: c_k,r
+  // times the product of those over d < j; psn [nkmax][R*R]: c_k,r times the product over d != j.
+  dw *P, *lead, *psn;
+  dw *fb;         // [R][ld] vector being fitted
+  dw *g, *glead;  // [D][R*R], [R*R]: its Grams in the same way, without weights
+  dw *fcs, *fg;   // [R] its weights; [R*R] c_r times its Grams' products over d != j
+  dw *BB, *gpart; // [R*R] normal equations; [nkmax][ceil(R*R/32)] parts of <Q_k, F>
+  dw *bs;         // [cl][R n, even] parts of the right-hand side received
+  dw *Iv, *b0, *X;  // [R*R] inverse (column-major); [R][n] right-hand side; [i + m R] solution
+  dw *dinv, *u, *red;
+  float *gi, *Ef, *emax;  // [R*R] FP32 inverse and residual; [warps] largest residuals
+  int *nb, *off, *flags;  // flags: [0] inverse usable, [1] non-positive pivot in the fallback
+  FastDiv* fdn;  // [D] divisors n
 };
 
-// Entries of R*R rounded up to whole warps.
-__host__ __device__ inline int gs_rrp(int R) { return (R * R + 31) / 32 * 32; }
+// Row stride of the factors: odd, so that a warp reads different rows from different banks.
+__host__ __device__ inline int gs_ld(int nD) { return nD | 1; }
 
-// Assigns the arrays (null bases: sizes only).  Returns the shared-memory
-// bytes; *gwork receives the global scratch entries (dw) of one CTA.
-__host__ __device__ inline size_t gs_carve(const GsDims& m, GsArrays* a, unsigned char* sbase, dw* gbase,
-                                           size_t* gwork) {
+// 32-entry chunks of an R x R matrix (at most 8).
+__host__ __device__ inline int gs_chunks(int R) { return (R * R + 31) / 32; }
+
+// Assigns the arrays (null base: sizes only) and returns the bytes.
+// `level` 1 leaves P to global memory.
+__host__ __device__ inline size_t gs_carve(const GsDims& m, GsArrays* a, unsigned char* sbase) {
   const int R = m.R, nkm = m.nkmax;
   const size_t RR = (size_t)R * R, Rn = (size_t)R * m.npm;
-  size_t so = 0, go = 0;
+  size_t so = 0;
   auto take_s = [&](size_t bytes) -> unsigned char* {
     const size_t r = so;
     so += (bytes + 15) / 16 * 16;
     return sbase ? sbase + r : nullptr;
   };
-  auto take = [&](int group, size_t n) -> dw* {
-    if (m.gmask & group) {
-      const size_t r = go;
-      go += (n + 1) / 2 * 2;
-      return gbase ? gbase + r : nullptr;
-    }
-    return (dw*)take_s(sizeof(dw) * n);
-  };
-  a->qf = take(kGroupQ, (size_t)nkm * R * m.nD);
-  a->qw = take(kGroupQ, (size_t)nkm * R * m.nD);
-  a->qc = take(kGroupQ, (size_t)nkm * R);
-  a->P = take(kGroupP, (size_t)nkm * m.D * RR);
-  a->psn = take(kGroupP, (size_t)nkm * RR);
-  a->ppsn = take(kGroupP, (size_t)nkm * RR);
-  a->part = take(kGroupP, (size_t)(nkm + 1) * 2 * Rn);
-  a->fb = take(kGroupF, (size_t)R * m.nD);
-  a->g = take(kGroupF, (size_t)m.D * RR);
-  a->fcs = (dw*)take_s(sizeof(dw) * R);
-  a->wf = (dw*)take_s(sizeof(dw) * Rn);
-  a->Gp = (dw*)take_s(sizeof(dw) * RR);
-  a->pGp = (dw*)take_s(sizeof(dw) * RR);
-  a->BB = (dw*)take_s(sizeof(dw) * RR);
-  a->gpart = (dw*)take_s(sizeof(dw) * nkm * (gs_rrp(R) / 32));
-  a->gco = (dw*)take_s(sizeof(dw) * nkm);
-  a->bpart = (dw*)take_s(sizeof(dw) * 2 * Rn);
-  a->X = (dw*)take_s(sizeof(dw) * Rn);
-  a->b0 = (dw*)take_s(sizeof(dw) * Rn);
-  a->res = (dw*)take_s(sizeof(dw) * Rn);
-  a->dinv = (dw*)take_s(sizeof(dw) * R);
-  a->u = (dw*)take_s(sizeof(dw) * R);
-  a->red = (dw*)take_s(sizeof(dw) * kGsWarps);
-  a->misc = (dw*)take_s(sizeof(dw) * 4);
-  a->gi = (float*)take_s(sizeof(float) * 2 * RR);
-  a->rred = (float*)take_s(sizeof(float) * 4);
-  a->prow = (float*)take_s(sizeof(float) * 2 * 72);
-  a->cs.conv = (float*)take_s(sizeof(float) * 64);
-  a->cs.rmax = (float*)take_s(sizeof(float) * 16 * 32);
-  a->cs.rsum = (dw*)take_s(sizeof(dw) * 16 * 32);
+  auto take = [&](size_t n) -> dw* { return (dw*)take_s(sizeof(dw) * n); };
+  a->qf = take((size_t)nkm * R * gs_ld(m.nD));
+  a->qc = take((size_t)nkm * R);
+  if (m.level < 1) a->P = take((size_t)nkm * m.D * RR);
+  a->lead = take((size_t)nkm * RR);
+  a->psn = take((size_t)nkm * RR);
+  a->fb = take((size_t)R * gs_ld(m.nD));
+  a->g = take((size_t)m.D * RR);
+  a->glead = take(RR);
+  a->fcs = take(R);
+  a->fg = take(RR);
+  a->BB = take(RR);
+  a->gpart = take((size_t)nkm * gs_chunks(R));
+  a->bs = take((size_t)m.cl * ((Rn + 1) / 2 * 2));
+  a->Iv = take(RR);
+  a->b0 = take(Rn);
+  a->X = take(Rn);
+  a->dinv = take(R);
+  a->u = take(R);
+  a->red = take(kGsWarps);
+  a->gi = (float*)take_s(sizeof(float) * RR);
+  a->Ef = (float*)take_s(sizeof(float) * RR);
+  a->emax = (float*)take_s(sizeof(float) * kGsWarps);
   a->nb = (int*)take_s(sizeof(int) * (m.D + 1));
   a->off = (int*)take_s(sizeof(int) * (m.D + 1));
-  a->flags = (int*)take_s(sizeof(int) * 4);
-  a->fd = (FastDiv*)take_s(sizeof(FastDiv) * (m.D + 3));
-  if (gwork) *gwork = go;
+  a->flags = (int*)take_s(sizeof(int) * 2);
+  a->fdn = (FastDiv*)take_s(sizeof(FastDiv) * m.D);
   return so;
 }
 
 __device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-
-// Barrier of the threads w0..511 (named barrier 2).
-__device__ __forceinline__ void worker_sync(int w0) {
-  asm volatile("bar.sync 2, %0;" ::"r"(kGsThreads - w0) : "memory");
-}
 
 // Sum over the block; every thread gets the same value (dw_add is
 // commutative, so the butterflies agree across lanes and warps).
@@ -156,515 +165,462 @@ __device__ dw block_sum(dw v, dw* red) {
   return s;
 }
 
-// block_sum without its leading barrier, for callers after which no thread
-// can still be reading red from an earlier sum (many barriers since).
-__device__ dw block_sum_ready(dw v, dw* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int o = 16; o > 0; o >>= 1) v = dw_add(v, dwsolve::dw_shfl_xor(v, o));
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  dw s = red[lane & (kGsWarps - 1)];
-  for (int o = kGsWarps / 2; o > 0; o >>= 1) s = dw_add(s, dwsolve::dw_shfl_xor(s, o));
-  return s;
-}
-
+// RT: the rank when it is known at compile time (16), else 0: index splits and
+// strides of a step are then immediates (a step is bound by instruction issue).
+template <int RT>
 struct Gs {
   GsArrays a;
-  int R, RR, RRp, D, nD, npm, CL, rank, tid;
-  int G, cid, gr, NC;  // clusters, this CTA's cluster, its index over all CTAs, all CTAs
+  int R_, D, nD, ld, CL, rank, tid, lane, warp;
   int rv;  // rank of the vector being fitted (ragged blocks; R otherwise)
+  dw pen;
+  FastDiv fdr;
+  __device__ __forceinline__ int R() const { return RT ? RT : R_; }
+  __device__ __forceinline__ int RR() const { return R() * R(); }
+  __device__ __forceinline__ int chunks() const { return gs_chunks(R()); }
+  // e = r R + i
+  __device__ __forceinline__ void split(int e, int* r, int* i) const {
+    if (RT) {
+      *r = (unsigned)e / (RT ? RT : 1);
+      *i = (unsigned)e % (RT ? RT : 1);
+    } else {
+      fdr.divmod((unsigned)e, r, i);
+    }
+  }
 };
 
 // Ragged ranks: rows and columns >= rv of the normal equations are the
 // identity, so the padded terms stay decoupled from the fit.
-__device__ __forceinline__ dw mask_bb(const Gs& c, int i, int i2, dw v) {
-  return (i >= c.rv || i2 >= c.rv) ? dw_make(i == i2 ? 1.f : 0.f) : v;
+template <int RT>
+__device__ __forceinline__ dw normal_entry(const Gs<RT>& c, int i, int i2, dw v) {
+  if (i >= c.rv || i2 >= c.rv) return dw_make(i == i2 ? 1.f : 0.f);
+  return i == i2 ? dw_add(v, c.pen) : v;
 }
 
 // The vector iv as the working copy: factors, weights, penalty.
-__device__ void load_vector(const Gs& c, const GsParams& p, int iv) {
-  const double* fb = p.base + (size_t)iv * c.R * c.nD;
-  for (int e = c.tid; e < c.R * c.nD; e += kGsThreads) c.a.fb[e] = dw_from_double(fb[e]);
-  for (int i = c.tid; i < c.R; i += kGsThreads) c.a.fcs[i] = dw_from_double(p.coef[(size_t)iv * c.R + i]);
-  if (c.tid == 0) {
-    double pen = p.coef[(size_t)iv * c.R];
-    for (int i = 1; i < c.R; ++i) pen = fmax(pen, p.coef[(size_t)iv * c.R + i]);
-    c.a.misc[0] = dw_from_double(pen * 1.0e-10);  // FP64-build rule of the reference for this stage
+template <int RT>
+__device__ void load_vector(Gs<RT>& c, const GsParams& p, int iv) {
+  const int R = c.R();
+  const double* fb = p.base + (size_t)iv * R * c.nD;
+#pragma unroll 1
+  for (int e = c.tid; e < R * c.nD; e += kGsThreads) c.a.fb[e / c.nD * c.ld + e % c.nD] = dw_from_double(fb[e]);
+  if (c.tid < R) c.a.fcs[c.tid] = dw_from_double(p.coef[(size_t)iv * R + c.tid]);
+  __syncthreads();
+  dw pen = c.a.fcs[0];
+#pragma unroll 1
+  for (int i = 1; i < R; ++i)
+    if (dw_gt(c.a.fcs[i], pen)) pen = c.a.fcs[i];
+  c.pen = dw_mul(pen, dw_from_double(1.0e-10));  // FP64-build rule of the reference for this stage
+}
+
+// sum_m x[m sx] y[m sy], m < (N ? N : n)
+template <int N = 0>
+__device__ __forceinline__ dw dot(const dw* x, int sx, const dw* y, int sy, int n) {
+  dw_acc acc = acc_zero();
+  if (N) {
+#pragma unroll
+    for (int m = 0; m < N; ++m) acc_fma(acc, x[m * sx], y[m * sy]);
+  } else {
+#pragma unroll 4
+    for (int m = 0; m < n; ++m) acc_fma(acc, x[m * sx], y[m * sy]);
+  }
+  return acc_value(acc);
+}
+
+// The share of 32 lanes in <Q_k, F>, to gpart.
+template <int RT>
+__device__ __forceinline__ void put_coefficient(const Gs<RT>& c, int kl, int ch, dw contrib) {
+  const dw s = dwsolve::lane_sum<32>(contrib);
+  if (c.lane == 0) c.a.gpart[kl * c.chunks() + ch] = s;
+}
+
+// The products over d' >= d of the overlaps (Grams) v[d stride], into v[d stride] for
+// d >= 1; returns the product over d >= 1 (times `tail`, the value of mode D - 1).
+__device__ __forceinline__ dw suffix_products(dw* v, size_t stride, int D, dw tail) {
+  v[(D - 1) * stride] = tail;
+#pragma unroll 1
+  for (int d = D - 2; d > 0; --d) {
+    tail = dw_mul(tail, v[d * stride]);
+    v[d * stride] = tail;
+  }
+  return tail;
+}
+
+// A vector begins: its Grams and the owned vectors' overlaps with it, every
+// mode, and what the first step (mode 0) needs of them.
+template <int RT>
+__device__ void vector_start(const Gs<RT>& c, int nk, bool fit) {
+  const int R = c.R(), RR = c.RR(), D = c.D, ld = c.ld, nch = c.chunks();
+#pragma unroll 1
+  for (int q = c.warp; q < (nk + 1) * nch; q += kGsWarps) {
+    const int s = q / nch, ch = q - s * nch, ee = 32 * ch + c.lane;
+    const bool self = s == 0;  // the Grams first
+    const int kl = s - 1;
+    dw contrib = dw_make(0.f);
+    if (ee < RR) {
+      int r, i;
+      c.split(ee, &r, &i);
+      const dw *x = (self ? c.a.fb : c.a.qf + (size_t)kl * R * ld) + (size_t)r * ld, *y = c.a.fb + (size_t)i * ld;
+      dw* v = (self ? c.a.g : c.a.P + (size_t)kl * D * RR) + ee;
+      dw tail = dw_make(1.f);
+#pragma unroll 1
+      for (int d = 0; d < D; ++d) {
+        const int o = c.a.off[d];
+        tail = dot(x + o, 1, y + o, 1, c.a.nb[d]);
+        v[(size_t)d * RR] = tail;
+      }
+      tail = suffix_products(v, RR, D, tail);
+      const dw all = dw_mul(tail, v[0]);
+      if (self) {
+        c.a.glead[ee] = fit ? dw_make(1.f) : all;
+        c.a.BB[ee] = normal_entry(c, i, r, tail);
+        c.a.fg[ee] = dw_mul(c.a.fcs[r], tail);
+      } else {
+        const dw w = c.a.qc[kl * R + r];
+        c.a.lead[(size_t)kl * RR + ee] = w;
+        c.a.psn[(size_t)kl * RR + ee] = dw_mul(tail, w);
+        contrib = dw_mul(dw_mul(all, w), c.a.fcs[i]);
+      }
+    }
+    if (!self) put_coefficient(c, kl, ch, contrib);
   }
   __syncthreads();
 }
 
-// Grams of the working vector, every mode (symmetric, both triangles stored).
-__device__ void all_grams(const Gs& c) {
-  const int R = c.R, RR = c.RR;
-  for (int e = c.tid; e < c.D * RR; e += kGsThreads) {
-    const int d = e / RR, ee = e - d * RR, i = ee % R, i2 = ee / R;
-    if (i > i2) continue;
-    const dw* x = c.a.fb + (size_t)i * c.nD + c.a.off[d];
-    const dw* y = c.a.fb + (size_t)i2 * c.nD + c.a.off[d];
-    dw_acc acc = acc_zero();
-    for (int q = 0; q < c.a.nb[d]; ++q) acc_fma(acc, x[q], y[q]);
-    const dw s = acc_value(acc);
-    c.a.g[(size_t)d * RR + i + i2 * R] = s;
-    c.a.g[(size_t)d * RR + i2 + i * R] = s;
-  }
-  __syncthreads();
-}
-
-// Overlaps of the owned earlier vectors with the working vector, every mode.
-__device__ void all_overlaps(const Gs& c, int nk) {
-  const int R = c.R, RR = c.RR, DRR = c.D * RR;
-  for (int e = c.tid; e < nk * DRR; e += kGsThreads) {
-    const int kl = e / DRR, rem = e - kl * DRR, d = rem / RR, ee = rem - d * RR, r = ee / R, i = ee - r * R;
-    const dw* x = c.a.qf + ((size_t)kl * R + r) * c.nD + c.a.off[d];
-    const dw* y = c.a.fb + (size_t)i * c.nD + c.a.off[d];
-    dw_acc acc = acc_zero();
-    for (int q = 0; q < c.a.nb[d]; ++q) acc_fma(acc, x[q], y[q]);
-    c.a.P[(size_t)kl * DRR + rem] = acc_value(acc);
-  }
-  __syncthreads();
-}
-
-// Weights divided by sqrt(<F,F>).
-__device__ void normalize_weights(const Gs& c) {
-  const int R = c.R;
+// The finished vector: weights divided by sqrt(<F,F>), FP64 output (a share of each
+// CTA), and the owner's resident copy when later vectors use it.
+template <int RT>
+__device__ void finish_vector(const Gs<RT>& c, const GsParams& p, int iv, bool factors) {
+  const int R = c.R(), nD = c.nD;
   dw part = dw_make(0.f);
-  for (int e = c.tid; e < c.RR; e += kGsThreads) {
-    dw prod = dw_mul(c.a.fcs[e % R], c.a.fcs[e / R]);
-    for (int d = 0; d < c.D; ++d) prod = dw_mul(prod, c.a.g[(size_t)d * c.RR + e]);
-    part = dw_add(part, prod);
+  if (c.tid < c.RR()) {
+    int r, i;
+    c.split(c.tid, &r, &i);
+    part = dw_mul(dw_mul(c.a.fcs[r], c.a.fcs[i]), c.a.glead[c.tid]);
   }
   const dw q = dw_sqrt(dw_abs(block_sum(part, c.a.red)));
-  __syncthreads();  // every thread has read fcs
-  for (int i = c.tid; i < R; i += kGsThreads) c.a.fcs[i] = dw_div(c.a.fcs[i], q);
+  const bool own = iv < p.nbloc - 1 && iv % c.CL == c.rank;
+  const int kl = iv / c.CL;
+  if (c.tid < R) {
+    const dw x = dw_div(c.a.fcs[c.tid], q);
+    if (own) c.a.qc[(size_t)kl * R + c.tid] = x;
+    if (c.rank == 0) p.coef[(size_t)iv * R + c.tid] = dw_to_double(x);
+  }
+  if (own)
+#pragma unroll 1
+    for (int e = c.tid; e < R * c.ld; e += kGsThreads) c.a.qf[(size_t)kl * R * c.ld + e] = c.a.fb[e];
+  if (factors)
+#pragma unroll 1
+    for (int e = c.rank * kGsThreads + c.tid; e < R * nD; e += c.CL * kGsThreads)
+      p.base[(size_t)iv * R * nD + e] = dw_to_double(c.a.fb[e / nD * c.ld + e % nD]);
   __syncthreads();
 }
 
-// The finished vector: FP64 output (CTA 0 of the grid), and the owner's
-// resident copy when later vectors use it.
-__device__ void finish_vector(const Gs& c, const GsParams& p, int iv, bool factors) {
-  const int R = c.R, nD = c.nD;
-  if (c.gr == 0) {
-    double* fb = p.base + (size_t)iv * R * nD;
-    if (factors)
-      for (int e = c.tid; e < R * nD; e += kGsThreads) fb[e] = dw_to_double(c.a.fb[e]);
-    for (int i = c.tid; i < R; i += kGsThreads) p.coef[(size_t)iv * R + i] = dw_to_double(c.a.fcs[i]);
-  }
-  if (iv < p.nbloc - 1 && iv % c.NC == c.gr) {
-    const int kl = iv / c.NC;
-    dw* qf = c.a.qf + (size_t)kl * R * nD;
-    dw* qw = c.a.qw + (size_t)kl * R * nD;
-    for (int e = c.tid; e < R * nD; e += kGsThreads) {
-      const dw x = c.a.fb[e];
-      qf[e] = x;
-      qw[e] = dw_mul(c.a.fcs[e / nD], x);
-    }
-    for (int i = c.tid; i < R; i += kGsThreads) c.a.qc[(size_t)kl * R + i] = c.a.fcs[i];
-  }
-  __syncthreads();
-}
-
-// Step phase 1.  Unless the previous step's update already formed them
-// (`pre`), the products over d != j of the owned overlaps (psn) and of the
-// working Grams (Gp, and BB = Gp + pen I).  Always: the weighted factor
-// wf(r,m) = c_r F_r^j(m), and per warp of psn entries the partial sums of
-// c_k,r c_i P_k(r,i) over all modes (the coefficients <Q_k, F>).
-// Threads t0..511 (t0 a multiple of 32); ends with a barrier over them.
-__device__ void step_products(const Gs& c, int j, int nk, bool pre, int t0, dw qinv) {
-  const int R = c.R, RR = c.RR, RRp = c.RRp, D = c.D, nj = c.a.nb[j], offj = c.a.off[j];
-  const int npsn = nk * RRp, ngp = npsn + (pre ? 0 : RR), total = ngp + R * nj;
-  const dw pen = c.a.misc[0];
-  for (int e = c.tid - t0; e < total; e += kGsThreads - t0) {
-    if (e < npsn) {  // whole warps: npsn is a multiple of 32
-      int kl, ee;
-      c.a.fd[2].divmod((unsigned)e, &kl, &ee);
-      dw contrib = dw_make(0.f);
-      if (ee < RR) {
-        int r, i;
-        c.a.fd[0].divmod((unsigned)ee, &r, &i);
-        const dw* Pk = c.a.P + (size_t)kl * D * RR + ee;
-        const dw pj = Pk[(size_t)j * RR], w = dw_mul(c.a.qc[(size_t)kl * R + r], dw_mul(c.a.fcs[i], qinv));
-        dw prod;
-        if (pre) {
-          prod = c.a.psn[(size_t)kl * RR + ee];
-        } else {
-          prod = dw_make(1.f);
-          for (int d = 0; d < D; ++d)
-            if (d != j) prod = dw_mul(prod, Pk[(size_t)d * RR]);
+// This CTA's part of the right-hand side of mode j (warps 4..15): sources s < nk,
+//   -<Q_k, F> sum_r Q_k,r^j(m) psn_k(r,i),
+// and, in the CTA that will own the fitted vector, sum_r F_r^j(m) fg(r,i), stored into
+// every CTA of the cluster (entry i n + m).  Four lanes have two entries, two of them an
+// entry's sums over r in halves; each stores the pair into a quarter of the CTAs.
+template <int RT>
+__device__ void step_rhs(const Gs<RT>& c, int j, int nk, bool self) {
+  const int R = c.R(), RR = c.RR(), nj = c.a.nb[j], offj = c.a.off[j], Rn = R * nj, nch = c.chunks();
+  const int nsrc = nk + (self ? 1 : 0), np = (Rn + 1) / 2, h = c.lane & 1;
+  const int half = RT ? RT / 2 : (R + 1) / 2, r0 = h * half, nr = RT ? RT / 2 : min(R, r0 + half) - r0;
+  const FastDiv fdn = c.a.fdn[j];
+#pragma unroll 1
+  for (int e0 = 0;; e0 += kGsWorkers / 2) {
+    const int ew = e0 + 16 * (c.warp - kGsInvert / 32), e = ew + (c.lane >> 1);
+    const bool none = ew >= Rn || nsrc == 0;
+    dw v = dw_make(0.f);
+    if (!none) {
+      int i, m;
+      fdn.divmod((unsigned)(e < Rn ? e : 0), &i, &m);
+      const dw* A = c.a.qf + (size_t)r0 * c.ld + offj + m;
+      const dw* M = c.a.psn + r0 * R + i;
+      dw_acc tot = acc_zero();
+      dw co = dw_make(0.f);
+#pragma unroll 1
+      for (int s = 0; s < nsrc; ++s) {
+        if ((s & 3) == 0) {  // the coefficients of four sources, eight lanes each
+          const int sk = s + (c.lane >> 3), q = c.lane & 7;
+          co = sk < nk && q < nch ? c.a.gpart[sk * nch + q] : dw_make(0.f);
+          co = dwsolve::lane_sum<8>(co);
+          co = sk < nk ? dw_neg(co) : dw_make(1.f);
         }
-        contrib = dw_mul(dw_mul(prod, pj), w);
-        if (!pre) c.a.psn[(size_t)kl * RR + ee] = prod;
+        if (s == nk) {
+          A = c.a.fb + (size_t)r0 * c.ld + offj + m;
+          M = c.a.fg + r0 * R + i;
+        }
+        acc_fma(tot, dwsolve::dw_shfl(co, (s & 3) * 8), dot<RT / 2>(A, c.ld, M, R, nr));
+        A += (size_t)R * c.ld;
+        M += RR;
       }
-      for (int o = 16; o > 0; o >>= 1) contrib = dw_add(contrib, dwsolve::dw_shfl_xor(contrib, o));
-      if ((c.tid & 31) == 0) c.a.gpart[kl * (RRp / 32) + ee / 32] = contrib;
-    } else if (e < ngp) {
-      const int ee = e - npsn;
-      dw prod = dw_make(1.f);
-      for (int d = 0; d < D; ++d)
-        if (d != j) prod = dw_mul(prod, c.a.g[(size_t)d * RR + ee]);
-      c.a.Gp[ee] = prod;
-      int i2, i;
-      c.a.fd[0].divmod((unsigned)ee, &i2, &i);
-      c.a.BB[ee] = mask_bb(c, i, i2, (i == i2) ? dw_add(prod, pen) : prod);
-    } else {
-      const int ee = e - ngp;
-      int m, r;
-      c.a.fd[0].divmod((unsigned)ee, &m, &r);
-      c.a.wf[ee] = dw_mul(dw_mul(c.a.fcs[r], qinv), c.a.fb[(size_t)r * c.nD + offj + m]);
+      v = acc_value(
+          dwsolve::acc_merge(tot, dw_acc{__shfl_xor_sync(0xffffffffu, tot.s, 1), __shfl_xor_sync(0xffffffffu, tot.c, 1)}));
     }
-  }
-  if (t0 == 0) __syncthreads();
-  else worker_sync(t0);
-}
-
-// Step phase 2 (threads w0..511, while the lower warps invert BB): the dot
-// products over r, split in two halves,
-//   source 0:        sum_r wf(r,m) Gp(r,i)                      (self term)
-//   source 1 + kl:   sum_r c_k,r Q_k,r^j(m) psn_k(r,i)          (owned k)
-// at part[(2 s + h) R nj + i + m R]; and gco_k = -<Q_k, F> from the partials.
-__device__ void step_dots(const Gs& c, int j, int nk, int w0) {
-  const int R = c.R, RR = c.RR, nj = c.a.nb[j], offj = c.a.off[j], Rn = R * nj, half = (R + 1) / 2;
-  const int total = (nk + 1) * 2 * Rn, w = c.tid - w0, nw = kGsThreads - w0;
-  const FastDiv fdrn = c.a.fd[3 + j];
-  for (int e = w; e < total; e += nw) {
-    int sh, em, m, i;
-    fdrn.divmod((unsigned)e, &sh, &em);
-    c.a.fd[0].divmod((unsigned)em, &m, &i);
-    const int s = sh >> 1;
-    const int r0 = (sh & 1) ? half : 0, r1 = (sh & 1) ? R : half;
-    dw_acc acc = acc_zero();
-    if (s == 0) {
-      for (int r = r0; r < r1; ++r) acc_fma(acc, c.a.wf[r + m * R], c.a.Gp[r * R + i]);
-    } else {
-      const dw* A = c.a.qw + (size_t)(s - 1) * R * c.nD + offj + m;
-      const dw* M = c.a.psn + (size_t)(s - 1) * RR + i;
-      for (int r = r0; r < r1; ++r) acc_fma(acc, A[(size_t)r * c.nD], M[r * R]);
-    }
-    c.a.part[e] = acc_value(acc);
-  }
-  if (w < nk) {
-    const int nch = c.RRp / 32;
-    dw s = dw_make(0.f);
-    for (int q = 0; q < nch; ++q) s = dw_add(s, c.a.gpart[w * nch + q]);
-    c.a.gco[w] = dw_neg(s);
-  }
-  worker_sync(w0);
-}
-
-// Step phase 3 (threads w0..511): this CTA's part of the right-hand side,
-//   sum_k gco_k sum_r c_k,r Q_k,r^j(m) psn_k(r,i).
-__device__ void step_rhs_part(const Gs& c, int j, int nk, dw* bp, int w0) {
-  const int Rn = c.R * c.a.nb[j];
-  for (int e = c.tid - w0; e < Rn; e += kGsThreads - w0) {
-    dw_acc acc = acc_zero();
-    for (int kl = 0; kl < nk; ++kl) {
-      const dw g = c.a.gco[kl];
-      acc_fma(acc, g, c.a.part[(size_t)(2 * kl + 2) * Rn + e]);
-      acc_fma(acc, g, c.a.part[(size_t)(2 * kl + 3) * Rn + e]);
-    }
-    bp[e] = acc_value(acc);
-  }
-}
-
-// Step phase 4 (after the cluster barrier): the self term plus the partial
-// right-hand sides of the cluster, summed as a fixed tree over ranks so that
-// every CTA forms the identical system.  With several clusters (xout set)
-// the cluster's sum alone goes to xout (by rank 0) and the grid-wide step
-// below completes b0.
-// (ranks >= nown own no earlier vector yet; their parts are exact zeros)
-__device__ void step_gather(const Gs& c, int j, dw* bp, int nown, dw* xout = nullptr) {
-  const int Rn = c.R * c.a.nb[j];
-  for (int e = c.tid; e < Rn; e += kGsThreads) {
-    const uint32_t local = (uint32_t)__cvta_generic_to_shared(bp + e);
-    dw v[16];
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-      v[r] = dw_make(0.f);
-      if (r < nown) {
+    if (e0 == 0) cl_wait();  // every CTA has read the parts of the step before
+    if (none) return;
+    const dw o = dwsolve::dw_shfl_xor(v, 2);
+    const bool second = (c.lane & 2) != 0;
+    const dw v0 = second ? o : v, v1 = second ? v : o;
+    if (e < 2 * np) {
+      const uint32_t local = (uint32_t)__cvta_generic_to_shared(c.a.bs + 2 * ((size_t)c.rank * np + (e >> 1)));
+#pragma unroll 1
+      for (int r = c.lane & 3; r < c.CL; r += 4) {
         uint32_t remote;
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(r));
-        asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v[r].hi), "=f"(v[r].lo) : "r"(remote) : "memory");
+        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(remote), "f"(v0.hi), "f"(v0.lo), "f"(v1.hi),
+                     "f"(v1.lo)
+                     : "memory");
       }
     }
-    dw_acc acc = acc_zero();
-    if (xout) {
-#pragma unroll
-      for (int r = 0; r < 16; ++r) acc_add(acc, v[r]);
-      if (c.rank == 0) xout[e] = acc_value(acc);
-      continue;
-    }
-    acc_add(acc, c.a.part[e]);
-    acc_add(acc, c.a.part[(size_t)Rn + e]);
-#pragma unroll
-    for (int r = 0; r < 16; ++r) acc_add(acc, v[r]);
-    c.a.b0[e] = (e % c.R >= c.rv) ? dw_make(e / c.R == 0 ? 1.f : 0.f) : acc_value(acc);  // ragged padding
   }
-  __syncthreads();
 }
 
-// Iterations of the bounded wait for the other clusters' partial sums (each
-// a global load and a short sleep: about a tenth of a second in all, far
-// above the imbalance of one mode step).
-constexpr int kGridWaitLimit = 1 << 17;
-
-// Grid-wide step (several clusters): once every cluster leader has posted
-// its cluster sum for this step (xctr[0] >= G (step + 1)), every CTA forms
-// b0 = self term + the cluster sums in cluster order -- the identical system
-// everywhere.  The wait is bounded: the first CTA whose wait runs out sets
-// status bit 2 and the abort word xctr[1], after which no CTA waits again;
-// the kernel then runs to its end on whatever has arrived, and the result
-// is flagged invalid.
-__device__ void step_grid_sum(const Gs& c, const GsParams& p, int j, int step, const dw* xs) {
-  const int Rn = c.R * c.a.nb[j];
-  if (c.tid == 0) {
-    if (c.rank == 0) {
-      __threadfence();
-      atomicAdd(p.xctr, 1u);
-    }
-    const unsigned target = (unsigned)c.G * (unsigned)(step + 1);
-    volatile unsigned* ctr = p.xctr;
-    for (int it = 0; ctr[0] < target && ctr[1] == 0u; ++it) {
-      if (it >= kGridWaitLimit) {
-        atomicExch(p.xctr + 1, 1u);
-        atomicOr(p.status, 2);
-        break;
-      }
-      __nanosleep(64);
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  const size_t stride = (size_t)c.R * c.npm;
-  for (int e = c.tid; e < Rn; e += kGsThreads) {
+// After the exchange (every thread): the parts of the first nown CTAs in order, two lanes
+// per entry, scaled by the power of two that brings the largest weight into
+// [1, 2) (the weights enter linearly and are normalised at the vector's end).
+template <int RT>
+__device__ void step_gather(const Gs<RT>& c, int j, int nown) {
+  const int Rn = c.R() * c.a.nb[j], ld = (Rn + 1) / 2 * 2, h = c.tid & 1;
+  const float f = c.lane < c.R() ? fabsf(c.a.fcs[c.lane].hi) : 0.f;
+  const int ex = __reduce_max_sync(0xffffffffu, __float_as_int(f)) >> 23;
+  const float scale = ex > 0 && ex < 254 ? __int_as_float((254 - ex) << 23) : 1.f;
+#pragma unroll 1
+  for (int e0 = 0; e0 < Rn; e0 += kGsThreads / 2) {
+    const int e = e0 + (c.tid >> 1);
+    if (e0 + 16 * c.warp >= Rn) break;
     dw_acc acc = acc_zero();
-    acc_add(acc, c.a.part[e]);
-    acc_add(acc, c.a.part[(size_t)Rn + e]);
-    for (int g = 0; g < c.G; ++g) {
-      const dw* x = xs + (size_t)g * stride + e;
-      acc_add(acc, dw_make(__ldcg(&x->hi), __ldcg(&x->lo)));
-    }
-    c.a.b0[e] = (e % c.R >= c.rv) ? dw_make(e / c.R == 0 ? 1.f : 0.f) : acc_value(acc);  // ragged padding
+    const dw* v = c.a.bs + h * ld + (e < Rn ? e : 0);
+#pragma unroll 4
+    for (int r = h; r < nown; r += 2, v += 2 * ld) acc_add(acc, *v);
+    acc = dwsolve::acc_merge(acc, dw_acc{__shfl_xor_sync(0xffffffffu, acc.s, 1), __shfl_xor_sync(0xffffffffu, acc.c, 1)});
+    const dw b = acc_value(acc);
+    if (e < Rn && h == 0) c.a.b0[e] = dw_make(b.hi * scale, b.lo * scale);
   }
-  __syncthreads();
 }
 
-// Step phase 5 (every thread): X = BB^-1 b0 from the FP32 inverse formed
-// during phases 2-4 (the solver warps' LDL^T when that fails), rows
-// normalised, norms as the new weights.  Ends without a barrier.
-__device__ void step_solve(const Gs& c, int j, const float* inv, bool gj_ok) {
-  const int R = c.R, nj = c.a.nb[j];
-  if (!(gj_ok && dwsolve::refine_any<kGsThreads>(c.a.BB, R, c.a.b0, c.a.X, nj, inv, c.a.res, c.a.rred))) {
+// The inverse of the normal equations (warps 0..3; FP32 by warp 0): flags[0].
+template <int RT>
+__device__ void step_inverse(const Gs<RT>& c) {
+  if (c.warp == 0) {
+    const bool good = dwsolve::gj_inverse_warp(c.a.BB, c.R(), c.a.gi);
+    if (c.lane == 0) c.a.flags[0] = good;
+    __syncwarp();
+  }
+  dwsolve::solver_sync();
+  const bool ok = c.a.flags[0] != 0 && dwsolve::correct_inverse<RT>(c.a.BB, c.R(), c.a.gi, c.a.Iv, c.a.Ef, c.a.emax);
+  dwsolve::solver_sync();
+  if (c.tid == 0) c.a.flags[0] = ok;
+}
+
+// Row `warp` of the solution X = Iv b0 (of X itself after the fallback).
+template <int RT, int NC>
+__device__ void solve_row(const Gs<RT>& c, int j, bool solved) {
+  const int R = c.R(), nj = c.a.nb[j], i = c.warp;
+  dw x[NC ? NC : 1], nrm;
+  dwsolve::row_product<RT, NC>(c.a.Iv + i, R, c.a.b0, nj, solved, c.a.X + i, x);
+  dwsolve::row_normalise<NC>(x, &nrm);
+  const bool pad = i >= c.rv;  // ragged: the first unit vector, without weight
+#pragma unroll
+  for (int q = 0; q < (NC ? NC : 1); ++q) {
+    const int m = (NC ? c.lane : c.lane & 15) + 32 * q;
+    const dw y = pad ? dw_make(m == 0 ? 1.f : 0.f) : x[q];
+    if (m < nj && (NC || c.lane < 16)) {
+      c.a.X[i + m * R] = y;
+      c.a.fb[(size_t)i * c.ld + c.a.off[j] + m] = y;
+    }
+  }
+  if (c.lane == 0) c.a.fcs[i] = pad ? dw_make(0.f) : nrm;
+}
+
+// LDL^T in double-word (threads 0 .. 127); out of line: a step's own code has to stay in the
+// instruction cache.
+__device__ __noinline__ void fallback_solve(dw* A, int n, dw* dinv, dw* u, dw* X, int nrhs, int* bad_flag) {
+  const int bad = dwsolve::dw_ldlt(A, n, dinv, u);
+  dwsolve::dw_ldlt_solve(A, n, dinv, X, nrhs);
+  if (threadIdx.x == 0 && bad) *bad_flag = 1;
+}
+
+// The solve of mode j (every thread).
+template <int RT>
+__device__ void step_solve(const Gs<RT>& c, int j) {
+  const int R = c.R(), nj = c.a.nb[j];
+  const bool solved = c.a.flags[0] != 0;
+  if (!solved) {  // the FP32 inverse is no use: LDL^T in double-word
+    __syncthreads();
     if (c.tid < dwsolve::kSolverThreads) {
-      for (int e = c.tid; e < R * nj; e += dwsolve::kSolverThreads) c.a.X[e] = c.a.b0[e];
-      const int bad = dwsolve::dw_ldlt(c.a.BB, R, c.a.dinv, c.a.u);
-      dwsolve::dw_ldlt_solve(c.a.BB, R, c.a.dinv, c.a.X, nj);
-      if (c.tid == 0 && bad) c.a.flags[1] = 1;
+#pragma unroll 1
+      for (int e = c.tid; e < R * nj; e += dwsolve::kSolverThreads) c.a.X[e] = c.a.b0[e % R * nj + e / R];
+      fallback_solve(c.a.BB, R, c.a.dinv, c.a.u, c.a.X, nj, c.a.flags + 1);
     }
     __syncthreads();
   }
-  dwsolve::dw_normalise_rows<kGsThreads>(c.a.X, R, nj, c.a.fcs);
-}
-
-// When another step of this vector follows (mode jn): the products over d
-// not in {j, jn} of the owned overlaps (ppsn) and of the working Grams (pGp);
-// the update multiplies in mode j.  Threads t0, t0 + nt, ...
-__device__ void step_preproducts(const Gs& c, int j, int jn, int nk, int t0, int nt) {
-  const int RR = c.RR, D = c.D;
-  for (int e = t0; e < (nk + 1) * RR; e += nt) {
-    int kl, ee;
-    c.a.fd[1].divmod((unsigned)e, &kl, &ee);
-    const bool own = kl < nk;
-    const dw* src = own ? c.a.P + (size_t)kl * D * RR + ee : c.a.g + ee;
-    dw prod = dw_make(1.f);
-    for (int d = 0; d < D; ++d)
-      if (d != j && d != jn) prod = dw_mul(prod, src[(size_t)d * RR]);
-    if (own) c.a.ppsn[(size_t)kl * RR + ee] = prod;
-    else c.a.pGp[ee] = prod;
+  if (c.warp < R) {
+    if (nj <= 16) solve_row<RT, 0>(c, j, solved);
+    else if (nj <= 32) solve_row<RT, 1>(c, j, solved);
+    else solve_row<RT, 2>(c, j, solved);
   }
+  __syncthreads();
 }
 
-// Step phase 6: the new factor of mode j into the working vector, its Gram,
-// and the owned overlaps of mode j; with `pre`, the next step's products
-// psn, Gp and BB (mode jn) completed by multiplying in mode j.  Then the
-// weights are divided by sqrt(<F,F>), whose terms c_i c_i' prod_d G_d(i,i')
-// come with the new Gram.
-__device__ dw step_update(const Gs& c, int j, int jn, int nk, bool pre) {
-  const int R = c.R, RR = c.RR, nj = c.a.nb[j], offj = c.a.off[j], Rn = R * nj;
-  const int total = Rn + RR + nk * RR;
-  const dw pen = c.a.misc[0];
-  dw qpart = dw_make(0.f);
-  for (int e = c.tid; e < total; e += kGsThreads) {
-    if (e < Rn) {
-      int m, i;
-      c.a.fd[0].divmod((unsigned)e, &m, &i);
-      c.a.fb[(size_t)i * c.nD + offj + m] = c.a.X[e];
-    } else if (e < Rn + RR) {
-      const int ee = e - Rn;
-      int i2, i;
-      c.a.fd[0].divmod((unsigned)ee, &i2, &i);
-      if (i > i2) continue;
-      const int et = i2 + i * R;
-      // prod_{d != j} G_d: Gp, or with `pre` pGp = prod_{d not in {j, jn}} G_d times G_jn
-      const dw gp = pre ? c.a.pGp[ee] : c.a.Gp[ee], gq = pre ? dw_mul(gp, c.a.g[(size_t)jn * RR + ee]) : gp;
-      const dw w = dw_mul(c.a.fcs[i], c.a.fcs[i2]);
-      dw_acc acc = acc_zero();
-      for (int m = 0; m < nj; ++m) acc_fma(acc, c.a.X[i + m * R], c.a.X[i2 + m * R]);
-      const dw s = acc_value(acc);
-      c.a.g[(size_t)j * RR + ee] = s;
-      c.a.g[(size_t)j * RR + et] = s;
-      dw t = dw_mul(dw_mul(gq, s), w);
-      if (i != i2) t = dw{2.f * t.hi, 2.f * t.lo};
-      qpart = dw_add(qpart, t);
-      if (pre) {
-        const dw gn = dw_mul(gp, s);
-        c.a.Gp[ee] = gn;
-        c.a.Gp[et] = gn;
-        c.a.BB[ee] = mask_bb(c, i, i2, (i == i2) ? dw_add(gn, pen) : gn);
-        c.a.BB[et] = c.a.BB[ee];
+// The Gram of mode j from the new factor (every thread, two per entry) and, with
+// `more`, the next step's (mode jn) normal equations and self matrix.
+template <int RT>
+__device__ void update_gram(const Gs<RT>& c, int j, int jn, bool more) {
+  const int R = c.R(), RR = c.RR(), ee = c.tid >> 1, h = c.tid & 1, nj = c.a.nb[j], half = (nj + 1) / 2;
+  if (16 * c.warp >= RR) return;
+  const bool live = ee < RR;
+  int i2, i;
+  c.split(live ? ee : 0, &i2, &i);
+  const int m0 = h * half, nm = h ? nj - half : half;
+  dw_acc acc = acc_zero();
+  const dw *x = c.a.X + i + m0 * R, *y = c.a.X + i2 + m0 * R;
+#pragma unroll 4
+  for (int m = 0; m < nm; ++m) acc_fma(acc, x[m * R], y[m * R]);
+  const dw s = acc_value(
+      dwsolve::acc_merge(acc, dw_acc{__shfl_xor_sync(0xffffffffu, acc.s, 1), __shfl_xor_sync(0xffffffffu, acc.c, 1)}));
+  if (!live || h) return;
+  dw* v = c.a.g + ee;
+  dw lead = dw_mul(c.a.glead[ee], s), gn;
+  if (!more) {
+    c.a.glead[ee] = lead;
+    return;
+  }
+  if (jn > 0) {
+    v[(size_t)j * RR] = s;
+    gn = jn + 1 < c.D ? dw_mul(lead, v[(size_t)(jn + 1) * RR]) : lead;
+  } else {
+    gn = suffix_products(v, RR, c.D, s);
+    lead = dw_make(1.f);
+  }
+  c.a.glead[ee] = lead;
+  c.a.BB[ee] = normal_entry(c, i, i2, gn);
+  c.a.fg[ee] = dw_mul(c.a.fcs[i2], gn);
+}
+
+// The owned overlaps of mode j, the next step's products over d != jn and the
+// coefficients' parts (warps 4..15).
+template <int RT>
+__device__ void update_overlaps(const Gs<RT>& c, int j, int jn, int nk) {
+  const int R = c.R(), RR = c.RR(), nj = c.a.nb[j], offj = c.a.off[j], nch = c.chunks();
+#pragma unroll 1
+  for (int q = c.warp - kGsInvert / 32; q < nk * nch; q += kGsWorkerWarps) {
+    const int kl = q / nch, ch = q - kl * nch, ee = 32 * ch + c.lane;
+    dw contrib = dw_make(0.f);
+    if (ee < RR) {
+      int r, i;
+      c.split(ee, &r, &i);
+      dw* v = c.a.P + (size_t)kl * c.D * RR + ee;
+      const size_t le = (size_t)kl * RR + ee;
+      // (loads that may be from global memory before the products)
+      const dw ahead1 = v[(size_t)jn * RR], ahead2 = jn + 1 < c.D ? v[(size_t)(jn + 1) * RR] : dw_make(1.f),
+               lead0 = c.a.lead[le];
+      const dw s = dot(c.a.qf + ((size_t)kl * R + r) * c.ld + offj, 1, c.a.X + i, R, nj);
+      dw prod, next;  // products over d != jn and over all d
+      if (jn > 0) {
+        const dw lead = dw_mul(lead0, s);
+        v[(size_t)j * RR] = s;
+        c.a.lead[le] = lead;
+        prod = jn + 1 < c.D ? dw_mul(lead, ahead2) : lead;
+        next = dw_mul(lead, ahead1);
+      } else {
+        const dw w = c.a.qc[kl * R + r];
+        c.a.lead[le] = w;
+        prod = dw_mul(suffix_products(v, RR, c.D, s), w);
+        next = dw_mul(prod, ahead1);
       }
-    } else {
-      int kl, e2, r, i;
-      c.a.fd[1].divmod((unsigned)(e - Rn - RR), &kl, &e2);
-      c.a.fd[0].divmod((unsigned)e2, &r, &i);
-      const dw* x = c.a.qf + ((size_t)kl * R + r) * c.nD + offj;
-      const dw pre_k = pre ? c.a.ppsn[(size_t)kl * RR + e2] : dw_make(1.f);
-      dw_acc acc = acc_zero();
-      for (int m = 0; m < nj; ++m) acc_fma(acc, x[m], c.a.X[i + m * R]);
-      const dw s = acc_value(acc);
-      c.a.P[((size_t)kl * c.D + j) * RR + e2] = s;
-      if (pre) c.a.psn[(size_t)kl * RR + e2] = dw_mul(pre_k, s);
+      c.a.psn[le] = prod;
+      contrib = dw_mul(next, c.a.fcs[i]);
     }
+    put_coefficient(c, kl, ch, contrib);
   }
-  // 1 / sqrt(<F,F>) for every thread: the next step's products apply it to
-  // the weights as they read them (the solve then writes new weights), so
-  // the weights need no rewrite and no barrier of their own here; the sum's
-  // barrier also orders every write above before the next phase
-  return dw_rcp(dw_sqrt(dw_abs(block_sum_ready(qpart, c.a.red))));
 }
 
 }  // namespace
 
-// kResident: every array in shared memory (the compiler then addresses them
-// as such); otherwise the groups of p.gmask live in global scratch.
-template <bool kResident>
+template <int RT>
 __global__ void __launch_bounds__(kGsThreads, 1) gs_kernel(GsParams p) {
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Gs c;
+  Gs<RT> c;
   c.CL = (int)cluster.num_blocks();
   c.rank = (int)cluster.block_rank();
-  c.G = p.ngrp;
-  c.cid = blockIdx.x / c.CL;
-  c.gr = c.cid * c.CL + c.rank;
-  c.NC = c.G * c.CL;
-  c.R = p.R;
-  c.RR = p.R * p.R;
-  c.RRp = gs_rrp(p.R);
+  c.R_ = p.R;
+  c.fdr = FastDiv((unsigned)p.R);
   c.D = p.D;
   c.nD = p.nD;
-  c.npm = p.npmax;
+  c.ld = gs_ld(p.nD);
   c.tid = threadIdx.x;
+  c.lane = c.tid & 31;
+  c.warp = c.tid >> 5;
   c.rv = p.R;
-  const GsDims dims{p.R, p.D, p.nD, p.npmax, p.nkmax, kResident ? 0 : p.gmask};
-  gs_carve(dims, &c.a, smem_raw, reinterpret_cast<dw*>(p.work) + (size_t)c.gr * p.work_stride, nullptr);
+  gs_carve(GsDims{p.R, p.D, p.nD, p.npmax, p.nkmax, c.CL, p.level}, &c.a, smem_raw);
+  if (p.level) c.a.P = reinterpret_cast<dw*>(p.work) + (size_t)c.rank * p.nkmax * p.D * p.R * p.R;
+#pragma unroll 1
   for (int d = c.tid; d <= c.D; d += kGsThreads) {
     c.a.nb[d] = d < c.D ? p.nbas[d] : 0;
     c.a.off[d] = p.off[d];
+    if (d < c.D) {
+      c.a.fdn[d] = FastDiv((unsigned)p.nbas[d]);
+    }
   }
-  for (int q = c.tid; q < c.D + 3; q += kGsThreads)
-    c.a.fd[q] = FastDiv((unsigned)(q == 0 ? c.R : q == 1 ? c.RR : q == 2 ? c.RRp : c.R * p.nbas[q - 3]));
   if (c.tid == 0) {
+    c.a.flags[0] = 1;
     c.a.flags[1] = 0;
-    c.a.flags[2] = 1;
   }
+  // the cluster barrier is used twice per step: parts stored, parts read; this
+  // first arrival also says that the CTA runs
+  cl_arrive();
   __syncthreads();
 
   load_vector(c, p, 0);
-  all_grams(c);
-  normalize_weights(c);
+  vector_start(c, 0, false);
   finish_vector(c, p, 0, false);
 
-  int step = 0;
+#pragma unroll 1
   for (int iv = 1; iv < p.nbloc && p.nals > 0; ++iv) {
-    c.rv = p.rank_v ? p.rank_v[iv] : c.R;
+    c.rv = p.rank_v ? p.rank_v[iv] : p.R;
     load_vector(c, p, iv);
-    all_grams(c);
-    const int nk = (iv - c.gr + c.NC - 1) / c.NC;  // owned k = gr, gr + NC, ... < iv
-    all_overlaps(c, nk);
-    bool pre = false;
-    dw qinv = dw_make(1.f);  // 1 / |F| not yet applied to the weights (see step_update)
+    const int nk = (iv - c.rank + c.CL - 1) / c.CL;  // owned k = rank, rank + CL, ... < iv
+    vector_start(c, nk, true);
+#pragma unroll 1
     for (int it = 0; it < p.nals; ++it) {
-      for (int j = 0; j < c.D; ++j, ++step) {
-        dw* bp = c.a.bpart + (size_t)(step & 1) * c.R * c.npm;
+#pragma unroll 1
+      for (int j = 0; j < c.D; ++j) {
         const bool more = it + 1 < p.nals || j + 1 < c.D;  // another step of this vector follows
-        const int jn = j + 1 < c.D ? j + 1 : 0, nj = c.a.nb[j];
-        // FP32 inverse of BB (the first invert_warps(R) warps) concurrently
-        // with the right-hand side (threads w0..); when the previous update
-        // already formed BB, also concurrently with the products
-        const int w0 = 32 * dwsolve::invert_warps(c.R);
-        if (!pre) step_products(c, j, nk, pre, 0, qinv);
-        if (c.tid < w0) {
-          dwsolve::invert_any(c.a.BB, c.R, c.a.gi, c.a.prow, c.a.flags + 2);
+        const int jn = j + 1 < c.D ? j + 1 : 0;
+        if (c.tid < kGsInvert) {
+          cl_wait();
+          cl_arrive();
+          step_inverse(c);
         } else {
-          if (pre) step_products(c, j, nk, pre, w0, qinv);
-          step_dots(c, j, nk, w0);
-          step_rhs_part(c, j, nk, bp, w0);
+          step_rhs(c, j, nk, iv % c.CL == c.rank);
+          cl_arrive();
         }
-        // a peer's bpart of step s is rewritten at step s + 2, after every
-        // CTA has passed the barrier of step s + 1 (and so its gather of s)
-        cl_arrive();
         cl_wait();
-        {
-          // ranks of this cluster that own an earlier vector (the others' parts are zero)
-          const int nown = min(c.CL, max(0, iv - c.cid * c.CL));
-          if (c.G == 1) {
-            step_gather(c, j, bp, nown);
-          } else {
-            dw* xs = p.xpart + (size_t)(step & 1) * c.G * c.R * c.npm;
-            step_gather(c, j, bp, nown, xs + (size_t)c.cid * c.R * c.npm);
-            step_grid_sum(c, p, j, step, xs);
-          }
+        step_gather(c, j, min(c.CL, iv + 1));
+        __syncthreads();
+        cl_arrive();
+        step_solve(c, j);
+        update_gram(c, j, jn, more);
+        if (!more) break;
+        // the inverse starts with the complete BB, the right-hand side when the
+        // overlaps are complete too
+        if (c.tid < kGsInvert) {
+          asm volatile("bar.arrive 4, 512;" ::: "memory");
+          asm volatile("bar.sync 3, 512;" ::: "memory");
+        } else {
+          asm volatile("bar.arrive 3, 512;" ::: "memory");
+          update_overlaps(c, j, jn, nk);
+          asm volatile("bar.sync 4, 512;" ::: "memory");
         }
-        bool gj_ok = c.a.flags[2] != 0;
-        // the solve: refinement in registers (warps 0..nsw-1, one or two
-        // right-hand-side columns each) with the next step's partial products
-        // on the other warps, or the whole block's refinement / LDL^T
-        bool solved = false, pre_done = !more;
-        if (gj_ok && c.R <= 32 && nj <= 16) {
-          // rank <= 16: one column per warp, sums split over the half-warps
-          const bool split = c.R <= 16;
-          const int nsw = (split ? nj : dwsolve::solve_cols_warps(c.R, nj)) * 32;
-          if (c.tid < nsw) {
-            const bool ok = split ? dwsolve::solve_cols_split(c.a.BB, c.R, c.a.b0, c.a.X, nj, c.a.gi, c.a.fcs, c.a.cs)
-                                  : dwsolve::solve_cols_any(c.a.BB, c.R, c.a.b0, c.a.X, nj, c.a.gi, c.a.fcs, c.a.cs);
-            if (c.tid == 0) c.a.flags[3] = ok;
-          } else if (more) {
-            step_preproducts(c, j, jn, nk, c.tid - nsw, kGsThreads - nsw);
-          }
-          __syncthreads();
-          solved = c.a.flags[3] != 0;
-          pre_done = pre_done || nsw < kGsThreads;
-          gj_ok = false;  // not converged: straight to the LDL^T
-        }
-        if (!solved) step_solve(c, j, c.a.gi, gj_ok);
-        if (!pre_done) step_preproducts(c, j, jn, nk, c.tid, kGsThreads);
-        if (!solved || !pre_done) __syncthreads();
-        if (c.tid == 0) c.a.flags[2] = 1;
-        if (c.rv < c.R) {  // ragged: the padded terms keep zero weight
-          for (int i = c.rv + c.tid; i < c.R; i += kGsThreads) c.a.fcs[i] = dw_make(0.f);
-          __syncthreads();
-        }
-        qinv = step_update(c, j, jn, nk, more);
-        pre = more;
       }
     }
-    for (int i = c.tid; i < c.R; i += kGsThreads) c.a.fcs[i] = dw_mul(c.a.fcs[i], qinv);
     __syncthreads();
     finish_vector(c, p, iv, true);
   }
-  if (c.gr == 0 && c.tid == 0 && c.a.flags[1]) atomicOr(p.status, 1);
-  // no CTA leaves while a peer may still read its shared memory
-  cl_arrive();
+  if (c.rank == 0 && c.tid == 0 && c.a.flags[1]) atomicOr(p.status, 1);
+  // no CTA leaves while a peer may still store into its shared memory
   cl_wait();
 }
 
@@ -679,76 +635,46 @@ int gs_cluster_size(int nbloc, int pref) {
 
 namespace {
 
-// Most clusters a grid may hold (the GB300's 152 SMs at one 16-CTA cluster
-// per 16 SMs); the scratch is sized for it.
-constexpr int kMaxGroups = 9;
-
 // Cluster sizes the search tries (each clamped to the block).
 constexpr int kClusterCandidates[] = {16, 12, 8};
 
-int gs_nkmax(int nbloc, int ngrp, int cl) {
-  const int nc = gs_cluster_size(nbloc, cl) * ngrp;
-  return std::max(1, (nbloc - 1 + nc - 1) / nc);
-}
+int gs_nkmax(int nbloc, int nc) { return std::max(1, (nbloc - 1 + nc - 1) / nc); }
 
-// Global scratch entries (dw) of one CTA with every movable group there.
-size_t gs_cta_work(int nbloc, int R, int nD, int D, int npm, int ngrp, int cl) {
+// Bytes of the one-cluster form with clusters of cl CTAs.
+size_t gs_bytes(const GsParams& p, int cl, int level) {
   GsArrays a;
-  size_t gw = 0;
-  gs_carve(GsDims{R, D, nD, npm, gs_nkmax(nbloc, ngrp, cl), kGroupAll}, &a, nullptr, nullptr, &gw);
-  return gw;
+  return gs_carve(GsDims{p.R, p.D, p.nD, p.npmax, gs_nkmax(p.nbloc, cl), cl, level}, &a, nullptr);
 }
 
-// Shared-memory layout: keep as much resident as fits (the owned vectors
-// move out first, then their overlaps, then the working vector).
-bool gs_fit(const GsParams& p, int ngrp, int smem_max, int* gmask, size_t* smem) {
-  static const int masks[4] = {0, kGroupQ, kGroupQ | kGroupP, kGroupAll};
-  for (int q = 0; q < 4; ++q) {
-    GsArrays a;
-    const size_t b = gs_carve(GsDims{p.R, p.D, p.nD, p.npmax, gs_nkmax(p.nbloc, ngrp, p.cl), masks[q]}, &a,
-                              nullptr, nullptr, nullptr);
-    if (b <= (size_t)smem_max) {
-      *gmask = masks[q];
-      *smem = b;
-      return true;
-    }
-  }
-  return false;
+// How one cluster of cl CTAs can run the block: the smallest level that fits, or -1 (the grid
+// form).  With P in global memory a step of 150 vectors, rank 16, takes 9.0 us and 10.8 in the
+// grid form; with the leading products there too, 250 vectors take 12.4 and 11.0, so that stays out.
+int gs_level(const GsParams& p, int cl, int smem_max) {
+  if (p.R > kGsRank || p.D < 2) return -1;
+  for (int level = 0; level < 2; ++level)
+    if (gs_bytes(p, cl, level) <= (size_t)smem_max) return level;
+  return -1;
+}
+
+// Shared memory that a shape may not exceed: its normal equations and inverse, a
+// mode's factor five times and a coefficient per chunk of the overlaps of nkm vectors.
+size_t gs_core_bytes(int R, int D, int npm, int nkm) {
+  const size_t RR = (size_t)R * R, Rn = (size_t)R * npm;
+  size_t o = 0;
+  for (size_t bytes : {8 * (size_t)R, 8 * Rn, 8 * RR, 8 * RR, 8 * RR, 8 * nkm * ((RR + 31) / 32), 8 * (size_t)nkm, 16 * Rn,
+                       8 * Rn, 8 * Rn, 8 * Rn, 8 * (size_t)R, 8 * (size_t)R, (size_t)128, (size_t)32, 8 * RR, (size_t)16,
+                       (size_t)256, (size_t)2048, (size_t)4096, 4 * (size_t)(D + 1), 4 * (size_t)(D + 1),
+                       (size_t)16, sizeof(FastDiv) * (D + 3)})
+    o += (bytes + 15) / 16 * 16;
+  return o;
 }
 
 }  // namespace
 
 size_t gs_work_doubles(int nbloc, int R, int nD, int D, int npm) {
-  // the per-CTA scratch of the largest grid (one cluster owns the most per
-  // CTA, so size the scratch for every CTA of kMaxGroups clusters at the
-  // one-cluster share), for every cluster size the search may pick, then
-  // the cluster partials and the arrival counter
-  size_t most = 0;
-  for (int c : kClusterCandidates) {
-    const int cl = gs_cluster_size(nbloc, c);
-    most = std::max(most, (size_t)cl * kMaxGroups * gs_cta_work(nbloc, R, nD, D, npm, 1, c));
-  }
-  return most + (size_t)2 * kMaxGroups * R * npm + 2;
+  // the overlaps of 16 CTAs' vectors (fewer CTAs: fewer vectors in all), or the grid form's
+  return std::max(gs_grid_dw(nbloc, R, nD, D, npm), ((size_t)nbloc + 16) * D * R * R);
 }
-
-namespace {
-
-// Clusters for a block: one when everything fits in shared memory (small
-// blocks are bound by the latency of each mode step, and a grid-wide step
-// would only add to it); otherwise as many as the SMs hold at one CTA each,
-// up to one owned vector per CTA, so that the owned arrays' work spreads
-// over more SMs.
-int gs_groups(const GsParams& p, int num_sms, int smem_max) {
-  int gmask = 0;
-  size_t smem = 0;
-  if (gs_fit(p, 1, smem_max, &gmask, &smem) && gmask == 0) return 1;
-  const int cl = gs_cluster_size(p.nbloc, p.cl);
-  int g = std::min(kMaxGroups, num_sms / cl);
-  g = std::min(g, (p.nbloc - 1 + cl - 1) / cl);
-  return std::max(1, g);
-}
-
-}  // namespace
 
 int gs_launch(const GsParams& prm, cudaStream_t st) {
   GsParams p = prm;
@@ -757,56 +683,30 @@ int gs_launch(const GsParams& prm, cudaStream_t st) {
   MLCP_CUDA_TRY(cudaGetDevice(&dev));
   MLCP_CUDA_TRY(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   MLCP_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const char* env = getenv("MLCP_GB300_GS_GROUPS");  // a fixed cluster count (tests)
-  int ngrp = env ? std::max(1, std::min(kMaxGroups, atoi(env))) : gs_groups(p, nsm, smem_max);
-  if (ngrp * cl > nsm) ngrp = std::max(1, nsm / cl);
-  void (*kern)(GsParams) = nullptr;
-  size_t smem = 0;
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[2];
-  for (int pass = 0;; ++pass) {
-    p.ngrp = ngrp;
-    p.nkmax = gs_nkmax(p.nbloc, ngrp, p.cl);
-    p.work_stride = (long long)gs_cta_work(p.nbloc, p.R, p.nD, p.D, p.npmax, ngrp, p.cl);
-    int gmask = 0;
-    if (!gs_fit(p, ngrp, smem_max, &gmask, &smem)) {
-      set_error("intertwinecpp_: Gram-Schmidt needs more shared memory than %d bytes (rank %d)", smem_max, p.R);
-      return kTooLarge;
-    }
-    p.gmask = gmask;
-    kern = p.gmask == 0 ? gs_kernel<true> : gs_kernel<false>;
-    MLCP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    if (cl > 8) MLCP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    cfg = {};
-    cfg.gridDim = dim3(cl * ngrp);
-    cfg.blockDim = dim3(kGsThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = cl;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    // several clusters wait on one another each step: all of them must be
-    // resident together, which a cooperative launch guarantees (or refuses)
-    attr[1].id = cudaLaunchAttributeCooperative;
-    attr[1].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (ngrp == 1) break;
-    // no more clusters than the GPU holds at once at this size and shared
-    // memory (the GPCs bound how many clusters of 8-16 CTAs fit); with fewer
-    // clusters each CTA owns more earlier vectors, so the layout is redone
-    int maxc = 0;
-    MLCP_CUDA_TRY(cudaOccupancyMaxActiveClusters(&maxc, (const void*)kern, &cfg));
-    if (maxc >= ngrp || pass >= 3) break;
-    ngrp = std::max(1, maxc);
+  // shapes beyond what one CTA can hold of a mode step are refused
+  if (gs_core_bytes(p.R, p.D, p.npmax, gs_nkmax(p.nbloc, std::min(nsm, 9 * cl))) > (size_t)smem_max) {
+    set_error("intertwinecpp_: Gram-Schmidt needs more shared memory than %d bytes (rank %d)", smem_max, p.R);
+    return kTooLarge;
   }
-  // the cluster partials and the arrival counter follow the per-CTA scratch
-  dw* after = reinterpret_cast<dw*>(p.work) + (size_t)cl * ngrp * p.work_stride;
-  p.xpart = after;
-  p.xctr = reinterpret_cast<unsigned*>(after + (size_t)2 * kMaxGroups * p.R * p.npmax);
-  if (ngrp > 1) MLCP_CUDA_TRY(cudaMemsetAsync(p.xctr, 0, 2 * sizeof(unsigned), st));  // arrivals, abort word
-  cfg.numAttrs = ngrp > 1 ? 2 : 1;
+  p.level = gs_level(p, cl, smem_max);
+  if (p.level < 0) return gs_grid_launch(p, st);
+  const size_t smem = gs_bytes(p, cl, p.level);
+  p.nkmax = gs_nkmax(p.nbloc, cl);
+  void (*kern)(GsParams) = p.R == kGsRank ? gs_kernel<kGsRank> : gs_kernel<0>;
+  MLCP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (cl > 8) MLCP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cl);
+  cfg.blockDim = dim3(kGsThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cl;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   MLCP_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p));
   return kOk;
 }
@@ -816,7 +716,8 @@ int gs_launch(const GsParams& prm, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 // A larger cluster spreads the earlier vectors over more CTAs but pays a
 // longer gather and cluster barrier at every mode step; which wins depends on
-// the block (measured on the 40-vector rank-16 block: 16 CTAs 27.7 ms per
+// the block, and the grid form takes the blocks whose arrays 16 CTAs cannot hold
+// (measured on the 40-vector rank-16 block: 16 CTAs 27.7 ms per
 // cycle, 12 CTAs 28.7, 8 CTAs 31.2).  The first cycle of a block shape runs
 // one Gram-Schmidt sweep (nals = 1) twice with each candidate size on a
 // scratch copy of the block, times it with CUDA events on the cycle's stream
@@ -858,10 +759,13 @@ int gs_tuned_cluster(const GsParams& p, int device, double* scratch_base, double
       return kOk;
     }
   }
-  std::vector<int> cand;
+  int smem_max = 0;
+  MLCP_CUDA_TRY(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+  std::vector<int> cand;  // sizes whose CTAs hold the block
   for (int c : kClusterCandidates) {
     const int cl = gs_cluster_size(p.nbloc, c);
-    if (std::find(cand.begin(), cand.end(), cl) == cand.end()) cand.push_back(cl);
+    if (gs_level(p, cl, smem_max) >= 0 && std::find(cand.begin(), cand.end(), cl) == cand.end())
+      cand.push_back(cl);
   }
   GsTuneEntry entry;
   if (cand.size() > 1) {

@@ -83,17 +83,12 @@ struct GsParams {
   const int* offp;
   double* base;   // block, in place
   double* coef;
-  double* work;   // per-CTA scratch for the arrays that do not fit in shared memory (gs_work_doubles)
+  double* work;   // gs_work_doubles: scratch of the grid form, overlaps of the one-cluster form
   int* status;
   const int* rank_v;  // [nbloc] ranks <= R (terms beyond carry zero weight), or null: all R
   int cl;             // CTAs per cluster asked for (0: the 16-CTA rule; see gs_tuned_cluster)
-  // set by gs_launch
-  int nkmax;             // earlier vectors owned by one CTA, at most
-  int gmask;             // array groups placed in global scratch
-  long long work_stride; // scratch entries of one CTA
-  int ngrp;              // clusters sharing the block (1: one cluster, no grid-wide step)
-  dw* xpart;             // [2][ngrp][R * npmax] cluster partial right-hand sides (ngrp > 1)
-  unsigned* xctr;        // [0] arrivals of the cluster leaders, [1] abort word; zeroed before the launch (ngrp > 1)
+  int nkmax;          // earlier vectors owned by one CTA, at most (set by gs_launch)
+  int level;          // what the one-cluster form leaves to `work` (set by gs_launch)
 };
 int gs_launch(const GsParams& p, cudaStream_t st);
 // The measured cluster size for p's block shape (cached per process, device
@@ -104,6 +99,9 @@ int gs_tuned_cluster(const GsParams& p, int device, double* scratch_base, double
                      int* cl);
 // Appends one line per tuned block shape to out.
 void gs_tune_report(std::string& out);
+// The grid form (gs_grid.cu) and its scratch (dw).
+int gs_grid_launch(const GsParams& p, cudaStream_t st);
+size_t gs_grid_dw(int nbloc, int R, int nD, int D, int npm);
 // Doubles of GsParams::work needed for a block of nbloc vectors (npm: the
 // largest 4-padded basis size).
 size_t gs_work_doubles(int nbloc, int R, int nD, int D, int npm);

@@ -285,7 +285,7 @@ size_t plan_cycle(const Layout& Ly, const OpTable& t, int R, int B, CycleBuffers
   cb->eigv = (double*)take(sizeof(double) * B);
   cb->gwork = (double*)take(sizeof(double) * gep_work_doubles(B));
   cb->wts = (double*)take(sizeof(double) * (size_t)B * B * R);
-  cb->uwork = (dw*)take(sizeof(dw) * upd_work_dw(B, R, Ly.D));
+  cb->uwork = (dw*)take(sizeof(dw) * upd_work_dw(B, R, Ly.D, Ly.npmax));
   cb->qdw = (dw*)take(sizeof(dw) * upd_qdw_dw(B, R, Ly.nD));
   cb->shift = (double*)take(sizeof(double) * B);
   cb->meta = (int*)take(sizeof(int) * (3 * (Ly.D + 1) + B));
@@ -321,7 +321,7 @@ int run_updates(Context* ctx, const Layout& Ly, const CycleBuffers& cb, const in
                 int B, int nals, cudaStream_t st, const int* d_rank = nullptr) {
   UpdParams u{};
   u.rank_v = d_rank;
-  u.D = Ly.D; u.R = R; u.B = B; u.nD = Ly.nD; u.npmax = Ly.npmax; u.nals = nals; u.tile = 0;
+  u.D = Ly.D; u.R = R; u.B = B; u.nD = Ly.nD; u.npmax = Ly.npmax; u.nals = nals; u.h_off = Ly.off.data();
   u.nbas = d_nbas; u.off = d_off; u.q = cb.q; u.qc = cb.qc; u.U = cb.U; u.qn = cb.qn; u.qnc = cb.qnc;
   u.qdw = cb.qdw; u.work = cb.uwork; u.pen_factor = kPen; u.status = cb.status;
   return upd_launch(u, (int)ctx->smem_optin, st);

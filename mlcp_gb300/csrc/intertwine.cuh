@@ -111,24 +111,22 @@ size_t gs_work_doubles(int nbloc, int R, int nD, int D, int npm);
 // Q_i, of sum_k U(k,i) Q_k, weights then divided by its norm; double-word.
 struct UpdParams {
   int D, R, B, nD, npmax, nals;
-  int tile;               // block terms per shared-memory tile (set by upd_launch)
-  int cl;                 // CTAs per output vector (a cluster; set by upd_launch)
-  int resident;           // 1: the block overlaps of a CTA's terms in shared memory (set by upd_launch)
   const int* nbas;        // [D] (device)
   const int* off;         // [D+1] reference-layout offsets (device)
+  const int* h_off;       // the same in host memory, for the launches
   const double* q;        // old block (reference layout)
   const double* qc;
   const double* U;        // [B][B] column-major: U(k, i) = U[k + i B]
   double* qn;             // new block
   double* qnc;
   dw* qdw;                // upd_qdw_dw(B, R, nD): the old block's factors, double-word, mode-major
-  dw* work;               // upd_work_dw(B, R, D): per-vector overlaps, Grams, target weights
+  dw* work;               // upd_work_dw(B, R, D, npmax): overlaps, Grams, target weights, parts of sums
   double pen_factor;      // penalty = pen_factor * max(weights of Q_i)
   int* status;            // [B] bit 0: non-positive pivot
   const int* rank_v;      // [B] ranks <= R (terms beyond carry zero weight), or null: all R
 };
-int upd_launch(UpdParams p, int smem_optin, cudaStream_t st);
-size_t upd_work_dw(int B, int R, int D);
+int upd_launch(const UpdParams& p, int smem_optin, cudaStream_t st);
+size_t upd_work_dw(int B, int R, int D, int npm);
 size_t upd_qdw_dw(int B, int R, int nD);
 
 // Block Rayleigh-Ritz inner products: QHQ(i,j) = <Q_j, HQ_i>, S(i,j) = <Q_j, Q_i>, j <= i.

@@ -4,8 +4,8 @@
 // intertwinecpp_ (src/Solver.f90:499-504).
 //
 // The reference applies every Hamiltonian term to every rank-1 term of v and
-// accumulates <v, w> (O(R T (sum n^2 + R nD)) per vector).  Here one CTA per
-// vector computes, for every distinct operator u of every mode d (slot 0 is
+// accumulates <v, w> (O(R T (sum n^2 + R nD)) per vector).  Here the CTAs of a
+// vector, a cluster that shares its columns j, compute for every distinct operator u of every mode d (slot 0 is
 // the identity), the Gram
 //   M_d,u(i, j) = <v_i^d, h_u v_j^d>
 // once, after which
@@ -13,16 +13,21 @@
 //   <v|v>   = sum_ij c_i c_j prod_d M_d,0(i, j).
 // Everything is FP64, as in the reference: the work per vector is small and
 // the result is an eigenvalue estimate compared at the 1e-7 relative level.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "common.cuh"
 #include "intertwine.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace mlcp {
 
 namespace {
 
 constexpr int kRqThreads = 256;
+constexpr int kRqCluster = 8;  // CTAs per vector, at most (the portable cluster size)
 
 // Sum over the block in a fixed order; thread 0 gets the result.
 __device__ double block_sum64(double v, double* red) {
@@ -44,60 +49,76 @@ __device__ __forceinline__ int slot_mode(const OpTable& t, int g) {
   return d;
 }
 
+// Vector v0 + blockIdx.x / CL, columns j = rank (mod CL) of a cluster of CL CTAs.  Bound
+// by the FP64 pipe (a warp instruction holds an SM's for ~18 cycles), so the columns are
+// dealt to enough CTAs to use every SM: 40 vectors of rank 16 on 6 x 10 take 35 us
+// (61 with a CTA per vector), two 29 (78).
 __global__ void __launch_bounds__(kRqThreads) rq_kernel(RqParams p) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int CL = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const OpTable& t = p.ops;
-  const int v = p.v0 + blockIdx.x;
-  const int R = t.R, D = t.D, nD = p.nD, npm = t.npmax, RR = R * R, U = t.utot;
+  const int slot = blockIdx.x / CL, v = p.v0 + slot;
+  const int R = t.R, D = t.D, nD = p.nD, npm = t.npmax, U = t.utot;
+  const int nc = (R - rank + CL - 1) / CL, RC = R * nc;  // own columns
   const double* vb = p.base + (size_t)v * R * nD;
   const double* vc = p.coef + (size_t)v * R;
-  double* M = p.work + (size_t)blockIdx.x * p.work_stride;  // [U][R][R]
-  double* Y = M + (size_t)U * RR;                                 // [U][npm][R]
-  __shared__ double red[kRqThreads / 32];
+  double* M = p.work + (size_t)slot * p.work_stride;  // [U][R][R]
+  // the columns of the ranks below come first in Y: [U][npm][nc]
+  double* Y = M + (size_t)U * R * R + (size_t)U * npm * (rank * (R / CL) + min(rank, R % CL));
+  __shared__ double red[kRqThreads / 32], parts[2][kRqThreads];
 
   // Y_u(a, j) = sum_b h_u(a, b) v_j^d(b) for the non-identity operators
-  for (int e = threadIdx.x; e < U * npm * R; e += kRqThreads) {
-    const int g = e / (npm * R), rem = e - g * npm * R, a = rem / R, j = rem - a * R;
+  for (int e = threadIdx.x; e < U * npm * nc; e += kRqThreads) {
+    const int g = e / (npm * nc), rem = e - g * npm * nc, a = rem / nc, jc = rem - a * nc;
     const int d = slot_mode(t, g), n = t.nbas[d];
     if (a >= n || t.ident[g]) continue;
     const double* h = t.hmat64 + (size_t)g * npm * npm + (size_t)a * npm;
-    const double* x = vb + (size_t)j * nD + t.off[d];
+    const double* x = vb + (size_t)(rank + jc * CL) * nD + t.off[d];
     double acc = 0.0;
     for (int b = 0; b < n; ++b) acc = fma(h[b], x[b], acc);
-    Y[(size_t)g * npm * R + a * R + j] = acc;
+    Y[e] = acc;
   }
   __syncthreads();
   // M_u(i, j) = sum_a v_i^d(a) Y_u(a, j); the identity gives the mode Gram
-  for (int e = threadIdx.x; e < U * RR; e += kRqThreads) {
-    const int g = e / RR, ij = e - g * RR, i = ij / R, j = ij - i * R;
+  for (int e = threadIdx.x; e < U * RC; e += kRqThreads) {
+    const int g = e / RC, ij = e - g * RC, i = ij / nc, jc = ij - i * nc;
     const int d = slot_mode(t, g), n = t.nbas[d];
     const double* xi = vb + (size_t)i * nD + t.off[d];
     double acc = 0.0;
     if (t.ident[g]) {
-      const double* xj = vb + (size_t)j * nD + t.off[d];
+      const double* xj = vb + (size_t)(rank + jc * CL) * nD + t.off[d];
       for (int a = 0; a < n; ++a) acc = fma(xi[a], xj[a], acc);
     } else {
-      const double* y = Y + (size_t)g * npm * R + j;
-      for (int a = 0; a < n; ++a) acc = fma(xi[a], y[a * R], acc);
+      const double* y = Y + (size_t)g * npm * nc + jc;
+      for (int a = 0; a < n; ++a) acc = fma(xi[a], y[a * nc], acc);
     }
-    M[(size_t)g * RR + ij] = acc;
+    M[(size_t)g * R * R + i * R + rank + jc * CL] = acc;
   }
-  __syncthreads();
-  // the term sums and the norm
-  const int T = t.T;
-  double num = 0.0, den = 0.0;
-  for (int e = threadIdx.x; e < (T + 1) * RR; e += kRqThreads) {
-    const int tt = e / RR, ij = e - tt * RR, i = ij / R, j = ij - i * R;
-    double prod = vc[i] * vc[j];
-    if (tt < T) {
-      for (int d = 0; d < D; ++d) prod *= M[(size_t)(t.uoff[d] + t.uid[(size_t)tt * D + d]) * RR + ij];
-      num = fma(t.alpha[tt], prod, num);
-    } else {
-      for (int d = 0; d < D; ++d) prod *= M[(size_t)t.uoff[d] * RR + ij];
-      den += prod;
+  cluster.sync();
+  // the term sums and the norm: entries e = q mod kRqThreads are one sum, the sums dealt to
+  // the CTAs and put together by the first in a fixed order (the same for any CL)
+  const int T = t.T, RR = R * R, per = (kRqThreads + CL - 1) / CL, q = rank * per + threadIdx.x;
+  if ((int)threadIdx.x < per && q < kRqThreads) {
+    double num = 0.0, den = 0.0;
+    for (int e = q; e < (T + 1) * RR; e += kRqThreads) {
+      const int tt = e / RR, ij = e - tt * RR, i = ij / R, j = ij - i * R;
+      double prod = vc[i] * vc[j];
+      if (tt < T) {
+        for (int d = 0; d < D; ++d) prod *= M[(size_t)(t.uoff[d] + t.uid[(size_t)tt * D + d]) * RR + ij];
+        num = fma(t.alpha[tt], prod, num);
+      } else {
+        for (int d = 0; d < D; ++d) prod *= M[(size_t)t.uoff[d] * RR + ij];
+        den += prod;
+      }
     }
+    double* to = cluster.map_shared_rank(&parts[0][0], 0);
+    to[q] = num;
+    to[kRqThreads + q] = den;
   }
-  num = block_sum64(num, red);
-  den = block_sum64(den, red);
+  cluster.sync();
+  if (rank > 0) return;
+  const double num = block_sum64(parts[0][threadIdx.x], red);
+  const double den = block_sum64(parts[1][threadIdx.x], red);
   if (threadIdx.x == 0) p.out[v] = num / den;
 }
 
@@ -232,8 +253,23 @@ int rq_launch(const RqParams& p, cudaStream_t st) {
   if (nv <= 0) return kOk;
   RqParams q = p;
   q.work_stride = (long long)rq_work_doubles(p.ops);
-  rq_kernel<<<nv, kRqThreads, 0, st>>>(q);
-  MLCP_CUDA_TRY(cudaGetLastError());
+  // CTAs per vector: as many as keep about one CTA on every SM, each with a column or more
+  int dev = 0, nsm = 0;
+  MLCP_CUDA_TRY(cudaGetDevice(&dev));
+  MLCP_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const int cl = std::max(1, std::min(std::min(kRqCluster, p.ops.R), (nsm + nv - 1) / nv));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)nv * cl);
+  cfg.blockDim = dim3(kRqThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cl;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  MLCP_CUDA_TRY(cudaLaunchKernelEx(&cfg, rq_kernel, q));
   return kOk;
 }
 

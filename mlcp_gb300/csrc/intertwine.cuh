@@ -65,6 +65,7 @@ struct OpAlsParams {
   double* g64;            // [nvec][D][R][R] FP64 Grams of F
   int* status;            // [nvec]
   dw* gscr;               // opals_grid_dw(ops, nvec): scratch of the grid form
+  int keep;               // one-CTA form: h_u Fo_j of every mode fits (set by opals_launch)
   const int* rank_v;      // [nvec] ranks <= R (terms beyond carry zero weight), or null: all R
 };
 

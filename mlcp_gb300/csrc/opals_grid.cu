@@ -40,7 +40,6 @@ namespace mlcp {
 namespace {
 
 constexpr int kOpThreads = 128;
-constexpr int kSolveThreads = 256;  // opstep.cuh's sums are over this many threads
 constexpr int kChunkK = 32;         // rows of one right-hand-side stage
 
 __device__ __forceinline__ uint32_t og_saddr(const void* p) {
@@ -79,7 +78,7 @@ __host__ __device__ inline size_t og_carve(const OpTable& t, int nvec, dw* base,
 }
 
 // F (= Fo) in double-word, weights, penalty, Grams of F.  One CTA per vector.
-__global__ void __launch_bounds__(kSolveThreads) og_setup_kernel(OpAlsParams p) {
+__global__ void __launch_bounds__(kStepThreads) og_setup_kernel(OpAlsParams p) {
   const OpTable& t = p.ops;
   const int v = blockIdx.x, R = t.R, D = t.D, nD = p.nD, RR = R * R;
   OgScratch s;
@@ -128,7 +127,7 @@ __global__ void __launch_bounds__(kOpThreads) og_products_kernel(OpAlsParams p, 
   og_carve(t, p.nvec, p.gscr, &s);
   if (u == nu) {
     const dw* G = reinterpret_cast<const dw*>(p.g64) + (size_t)v * D * RR;
-    s.bb[(size_t)v * RR + e] = normal_equation(G, D, j, e, R, p.rank_v ? p.rank_v[v] : R, s.pen[v]);
+    s.bb[(size_t)v * RR + e] = normal_equation(G, D, j, e % R, e / R, R, p.rank_v ? p.rank_v[v] : R, s.pen[v]);
     return;
   }
   const dw* __restrict__ M = p.mscr + (size_t)v * t.utot * RR + e;
@@ -230,7 +229,7 @@ __global__ void __launch_bounds__(kOpThreads) og_rhs_kernel(OpAlsParams p, int j
 }
 
 // The solve of mode j and what follows from the new factor; one CTA per vector.
-__global__ void __launch_bounds__(kSolveThreads, 1) og_solve_kernel(OpAlsParams p, int j) {
+__global__ void __launch_bounds__(kStepThreads, 1) og_solve_kernel(OpAlsParams p, int j) {
   const OpTable& t = p.ops;
   const int v = blockIdx.x, R = t.R, RR = R * R, npm = t.npmax, nD = p.nD, nj = t.nbas[j], opj = t.offp[j];
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -238,10 +237,10 @@ __global__ void __launch_bounds__(kSolveThreads, 1) og_solve_kernel(OpAlsParams 
   step_carve(m, smem_raw, R, npm);
   OgScratch s;
   og_carve(t, p.nvec, p.gscr, &s);
-  for (int e = threadIdx.x; e < RR; e += kSolveThreads) m.BB[e] = s.bb[(size_t)v * RR + e];
-  for (int e = threadIdx.x; e < R * nj; e += kSolveThreads) m.b0[e] = s.b0[(size_t)v * R * npm + e];
+  for (int e = threadIdx.x; e < RR; e += kStepThreads) m.BB[e] = s.bb[(size_t)v * RR + e];
+  for (int e = threadIdx.x; e < R * nj; e += kStepThreads) m.b0[e] = s.b0[(size_t)v * R * npm + e];
   if (threadIdx.x == 0) {
-    m.flags[0] = m.flags[1] = 0;
+    m.flags[1] = 0;
     m.flags[2] = 1;
   }
   __syncthreads();
@@ -257,7 +256,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) og_solve_kernel(OpAlsParams 
   step_factor(m, R, nj, fb + t.off[j], nD, s.f + (size_t)v * R * t.nDp + opj, t.nDp, G + (size_t)j * RR);
   __syncthreads();
   if (p.mode == 0 && j == t.D - 1) step_renormalise(m, R, t.D, G, fc);
-  for (int i = threadIdx.x; i < R; i += kSolveThreads) cf[i] = m.cf[i];
+  for (int i = threadIdx.x; i < R; i += kStepThreads) cf[i] = m.cf[i];
   if (threadIdx.x == 0 && m.flags[1]) atomicOr(&p.status[v], 1);
 }
 
@@ -426,7 +425,7 @@ int opals_grid_launch(const OpAlsParams& p, cudaStream_t st) {
   StepSmem m;
   const size_t ssm = step_carve(m, nullptr, R, t.npmax);
   MLCP_CUDA_TRY(cudaFuncSetAttribute(og_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));
-  og_setup_kernel<<<p.nvec, kSolveThreads, 0, st>>>(p);
+  og_setup_kernel<<<p.nvec, kStepThreads, 0, st>>>(p);
   MLCP_CUDA_TRY(cudaGetLastError());
   for (int d = 0; d < D; ++d)
     if (int rc = operators_any(p, d, t.h_uoff[d + 1] - t.h_uoff[d], t.h_nbas[d], nsm, true, st)) return rc;
@@ -439,7 +438,7 @@ int opals_grid_launch(const OpAlsParams& p, cudaStream_t st) {
       if (R <= 16) og_rhs_kernel<2><<<dim3((nj + 15) / 16, 1, p.nvec), kOpThreads, 0, st>>>(p, j);
       else og_rhs_kernel<4><<<dim3((nj + 15) / 16, (R + 31) / 32, p.nvec), kOpThreads, 0, st>>>(p, j);
       MLCP_CUDA_TRY(cudaGetLastError());
-      og_solve_kernel<<<p.nvec, kSolveThreads, ssm, st>>>(p, j);
+      og_solve_kernel<<<p.nvec, kStepThreads, ssm, st>>>(p, j);
       MLCP_CUDA_TRY(cudaGetLastError());
       if (sw + 1 < p.nsweeps || j + 1 < D)  // the last factor's products are not needed
         if (int rc = operators_any(p, j, nu, nj, nsm, p.mode == 0, st)) return rc;

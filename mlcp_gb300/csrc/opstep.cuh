@@ -1,5 +1,5 @@
 // One mode step of the ALS-fitted Hamiltonian applications from its normal
-// equations and right-hand side on, for a CTA of 256 threads that holds one
+// equations and right-hand side on, for a CTA of 512 threads that holds one
 // vector: shared by the one-CTA form (opals.cu) and the grid form
 // (opals_grid.cu), so that both run the same operations in the same order.
 #pragma once
@@ -11,24 +11,25 @@ namespace mlcp {
 
 namespace {
 
-constexpr int kStepThreads = 256;
-constexpr int kStepWarps = kStepThreads / 32;
+constexpr int kStepThreads = 512;
+constexpr int kSumThreads = 256;  // threads (the first ones) whose partial sums make a sum's order
+constexpr int kSumWarps = kSumThreads / 32;
 
 struct StepSmem {
   dw* X;      // [R][npmax] solution (column-major, ld R)
   dw* b0;     // [R][npmax] right-hand side
   dw* res;    // [R][npmax] refinement residual
   dw* BB;     // [R][R] normal equations
-  float* gi;  // [2][R][R] FP32 inverse of BB
+  float* gi;  // [R][R] FP32 inverse of BB (its place is twice that)
   dw* cf;     // [R] weights of F
-  dw* red;    // [kStepWarps] reduction scratch
+  dw* red;    // [kSumWarps] reduction scratch
   dw* dinv;   // [R] LDL^T reciprocal pivots
   dw* u;      // [R] LDL^T scratch column
   dw* misc;   // [2] penalty, norm
   float* rred;  // [4] refinement scratch
   float* prow;  // [2][72] pivot rows of the inverse
   dwsolve::ColScratch cs;
-  int* flags;  // [4] [0] buffer of the inverse, [1] non-positive pivot seen, [2] inverse usable, [3] solved
+  int* flags;  // [4] [1] non-positive pivot seen, [2] inverse usable, [3] solved
 };
 
 // Carves the shared memory (null base: sizes only); returns the bytes.
@@ -46,7 +47,7 @@ __host__ __device__ inline size_t step_carve(StepSmem& s, unsigned char* base, i
   s.BB = (dw*)take(sizeof(dw) * RR);
   s.gi = (float*)take(sizeof(float) * 2 * RR);
   s.cf = (dw*)take(sizeof(dw) * R);
-  s.red = (dw*)take(sizeof(dw) * kStepWarps);
+  s.red = (dw*)take(sizeof(dw) * kSumWarps);
   s.dinv = (dw*)take(sizeof(dw) * R);
   s.u = (dw*)take(sizeof(dw) * R);
   s.misc = (dw*)take(sizeof(dw) * 2);
@@ -59,49 +60,26 @@ __host__ __device__ inline size_t step_carve(StepSmem& s, unsigned char* base, i
   return o;
 }
 
-// Entry e of prod_{d != j} G_d + pen I (G: the Grams of F, [D][R][R]); rows
-// and columns beyond the vector's rank rv are the identity.
-__device__ __forceinline__ dw normal_equation(const dw* G, int D, int j, int e, int R, int rv, dw pen) {
-  const int RR = R * R;
+// Entry (i, i2) of prod_{d != j} G_d + pen I (G: the Grams of F, [D][R][R]);
+// rows and columns beyond the vector's rank rv are the identity.
+__device__ __forceinline__ dw normal_equation(const dw* G, int D, int j, int i, int i2, int R, int rv, dw pen) {
+  const int RR = R * R, e = i + i2 * R;
   dw bb = dw_make(1.f);
   for (int d = 0; d < D; ++d)
     if (d != j) bb = dw_mul(bb, G[(size_t)d * RR + e]);
-  if (e % R == e / R) bb = dw_add(bb, pen);
-  if (e % R >= rv || e / R >= rv) bb = dw_make(e % R == e / R ? 1.f : 0.f);
+  if (i == i2) bb = dw_add(bb, pen);
+  if (i >= rv || i2 >= rv) bb = dw_make(i == i2 ? 1.f : 0.f);
   return bb;
-}
-
-// Threads that step_invert keeps busy: warp 0 in registers for R <= 32, else
-// warps 0-3.
-__host__ __device__ inline int step_invert_threads(int R) { return R <= 32 ? 32 : dwsolve::kSolverThreads; }
-
-// The FP32 inverse of BB, the refinement's preconditioner.
-__device__ inline void step_invert(const StepSmem& s, int R) {
-  if (threadIdx.x >= step_invert_threads(R)) return;
-  if (R <= 32) {
-    const bool g = dwsolve::gj_inverse_warp(s.BB, R, s.gi);
-    if (threadIdx.x == 0) {
-      s.flags[2] = g;
-      s.flags[0] = 0;
-    }
-  } else {
-    bool ok;
-    const float* iv = dwsolve::gj_inverse(s.BB, R, s.gi, &ok);
-    if (threadIdx.x == 0) {
-      s.flags[2] = ok;
-      s.flags[0] = iv == s.gi ? 0 : 1;
-    }
-  }
 }
 
 // X = BB^-1 b0 with unit rows, their norms to cf; ends with a block barrier.
 // (Norms by 128 threads: their partial sums depend on how many share a row.)
 __device__ inline void step_solve(const StepSmem& s, int R, int nj) {
   bool gj_ok = s.flags[2] != 0;
-  const float* inv = s.gi + (size_t)s.flags[0] * R * R;
+  const float* inv = s.gi;
   bool solved = false;
   const int nsw = dwsolve::solve_cols_warps(R, nj);
-  if (gj_ok && R <= 32 && nj <= 16 && nsw <= kStepWarps) {
+  if (gj_ok && R <= 32 && nj <= 16 && nsw <= kSumWarps) {
     if (threadIdx.x < nsw * 32) {
       const bool ok = dwsolve::solve_cols_any(s.BB, R, s.b0, s.X, nj, inv, s.cf, s.cs);
       if (threadIdx.x == 0) s.flags[3] = ok;
@@ -173,23 +151,23 @@ __device__ inline void step_factor(const StepSmem& s, int R, int nj, double* fb,
   }
 }
 
-// Sum over the block; thread 0 gets the result (fixed order).
+// Sum over the first kSumThreads threads; thread 0 gets the result (fixed order).
 __device__ inline dw step_block_sum(dw v, dw* red) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int o = 16; o > 0; o >>= 1) v = dw_add(v, dwsolve::dw_shfl_xor(v, o));
   __syncthreads();
-  if (lane == 0) red[warp] = v;
+  if (lane == 0 && warp < kSumWarps) red[warp] = v;
   __syncthreads();
   dw s = dw_make(0.f);
   if (threadIdx.x == 0)
-    for (int w = 0; w < kStepWarps; ++w) s = dw_add(s, red[w]);
+    for (int w = 0; w < kSumWarps; ++w) s = dw_add(s, red[w]);
   return s;
 }
 
 // Weight renormalisation after a POW sweep (src/intertw_mvp.cu:491-494).
 __device__ inline void step_renormalise(const StepSmem& s, int R, int D, const dw* G, double* fc) {
   dw part = dw_make(0.f);
-  for (int e = threadIdx.x; e < R * R; e += kStepThreads) {
+  for (int e = threadIdx.x; e < R * R && threadIdx.x < kSumThreads; e += kSumThreads) {
     dw prod = dw_mul(s.cf[e % R], s.cf[e / R]);
     for (int d = 0; d < D; ++d) prod = dw_mul(prod, G[(size_t)d * R * R + e]);
     part = dw_add(part, prod);

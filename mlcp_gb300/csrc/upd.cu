@@ -239,9 +239,9 @@ __global__ void __launch_bounds__(kStepThreads, 1) upd_solve_kernel(UpdParams p,
   const int i = blockIdx.x, R = p.R, RR = R * R, D = p.D, n = p.nbas[k], rv = p.rank_v ? p.rank_v[i] : R;
   const size_t vec = (size_t)R * p.npmax;
   dw* G = s.fg + (size_t)i * D * RR;
-  for (int e = threadIdx.x; e < RR; e += kStepThreads) m.BB[e] = normal_equation(G, D, k, e, R, rv, s.pen[i]);
+  for (int e = threadIdx.x; e < RR; e += kStepThreads) m.BB[e] = normal_equation(G, D, k, e % R, e / R, R, rv, s.pen[i]);
   if (threadIdx.x == 0) {
-    m.flags[0] = m.flags[1] = 0;
+    m.flags[1] = 0;
     m.flags[2] = 1;
   }
   const dw* part = s.part + i * vec;

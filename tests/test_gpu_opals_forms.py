@@ -30,6 +30,7 @@ CASES = [  # nbas, rank, vectors, terms, ishift, ragged
     ([6, 5, 7], 15, 40, 400, 1, False),
     ([4, 4, 4], 3, 2, 4, 1, False),   # one CTA per vector
     ([10, 9, 8], 12, 5, 8, -1, True),  # one CTA per vector
+    ([6, 5, 6, 6, 6, 7, 6, 6], 20, 2, 12, 1, True),  # one CTA, h_u Fo_j of one mode at a time
 ]
 
 

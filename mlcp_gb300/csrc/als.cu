@@ -33,6 +33,14 @@
 //    inverse (the refinement's preconditioner) is computed in registers by a
 //    warp that phase B leaves idle, when there is one.
 // One launch covers all sweeps; the host is not involved between steps.
+//
+// What bounds it.  64 vectors of 30 modes (12 functions, rank 20, 3200 terms): a step takes
+// 29 us, phase B 12.5 and the solve beside phase A 15, both at about 60 % of the issue
+// slots of 16 warps; hence no tests per entry on full tiles, the first tiles of phase B
+// loaded during the solve, and a solve whose entries stay in registers (a step took
+// 31.4 us without).  One vector of 6 modes, rank 16, is the solve's chain of latencies: 12.8 us a
+// step (16.2 with the inverse formed in the solve and the parts fetched one
+// entry at a time).
 
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
@@ -458,6 +466,88 @@ __device__ void load_factor(const Cta& c, const AlsParams& p, int d, float* dst,
   }
 }
 
+// One item of a product pass: the tile's 128 terms and four F terms.  kFull: every
+// one of them exists (no test per entry; the passes are bound by issue slots).
+template <bool kFull>
+__device__ __forceinline__ void product_item(const Cta& c, const AlsParams& p, const float* tile, int gs, int np, int d,
+                                             bool divide, int ex, int T, int iq) {
+  float po[4][4];
+  tile_dots(tile, gs, c.fa + iq * 4 * c.gsmax, c.gsmax, np, c.lane, po);
+  const int j0 = T * kAlsTileRows + c.lane;
+  float* P[4];
+#pragma unroll
+  for (int cc = 0; cc < 4; ++cc) P[cc] = c.P + (iq * 4 + cc) * c.ldP + j0;
+  auto live = [&](int a, int cc) { return kFull || (j0 + 32 * a < c.nrows && iq * 4 + cc < c.rF); };
+  // every load before any store: a shared-memory store would order each
+  // later load behind it (the compiler cannot prove they do not alias)
+  float pv[4][4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int cc = 0; cc < 4; ++cc) pv[a][cc] = live(a, cc) ? P[cc][32 * a] : 0.f;
+  // quotients without any call in the unrolled loop (a call would keep
+  // the sixteen independent chains from overlapping); the rare unsafe
+  // ones are marked and rebuilt afterwards
+  unsigned rebuild = 0u;
+  if (!divide) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int cc = 0; cc < 4; ++cc) pv[a][cc] *= po[a][cc];
+  } else {
+    int safe = 1;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int cc = 0; cc < 4; ++cc) {
+        const float x = pv[a][cc], qv = div_nr(x, po[a][cc]);
+        // also catches a zero divisor
+        if (kFull) {
+          safe &= (int)(fabsf(x) >= FLT_MIN) & (int)(fabsf(qv) <= FLT_MAX);
+          po[a][cc] = qv;
+        } else {
+          const bool ok = fabsf(x) >= FLT_MIN && fabsf(qv) <= FLT_MAX;
+          if (!ok && live(a, cc)) rebuild |= 1u << (a * 4 + cc);
+          pv[a][cc] = qv;
+        }
+      }
+    if (kFull) {
+      if (!safe) {
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int cc = 0; cc < 4; ++cc)
+            if (!(fabsf(pv[a][cc]) >= FLT_MIN && fabsf(po[a][cc]) <= FLT_MAX)) rebuild |= 1u << (a * 4 + cc);
+      }
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int cc = 0; cc < 4; ++cc) pv[a][cc] = po[a][cc];
+    }
+  }
+  // rebuilds, one entry at a time by the whole warp
+  for (unsigned pending = __ballot_sync(0xffffffffu, rebuild != 0u); pending;
+       pending = __ballot_sync(0xffffffffu, rebuild != 0u)) {
+    const int L = __ffs(pending) - 1;
+    const int bit = __ffs(__shfl_sync(0xffffffffu, rebuild, L)) - 1;
+    const int a = bit >> 2, cc = bit & 3;
+    const float qv = rebuild_product(c, p, T * kAlsTileRows + L + 32 * a, iq * 4 + cc, ex, d);
+    if (c.lane == L) {
+      rebuild &= rebuild - 1;
+#pragma unroll
+      for (int a2 = 0; a2 < 4; ++a2)
+#pragma unroll
+        for (int c2 = 0; c2 < 4; ++c2)
+          if (a2 * 4 + c2 == bit) pv[a2][c2] = qv;
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int cc = 0; cc < 4; ++cc)
+      if (live(a, cc)) P[cc][32 * a] = pv[a][cc];
+}
+
 // Product pass over the tiles of mode d, items (tile, i-quad) dealt
 // round-robin to warps [w0, w0 + nw):
 //   divide = false: P(j,i) *= <G_j^d, F_i^d>            (prologue)
@@ -474,65 +564,9 @@ __device__ void product_pass(const Cta& c, const AlsParams& p, unsigned seq, int
     const unsigned g = seq + (unsigned)T;
     if (wait_tile(c, g)) {
       const float* tile = c.ring + (size_t)(g % (unsigned)c.stages) * c.stage_floats;
-      float po[4][4];
-      tile_dots(tile, gs, c.fa + iq * 4 * c.gsmax, c.gsmax, np, c.lane, po);
-      // every load before any store: a shared-memory store would order each
-      // later load behind it (the compiler cannot prove they do not alias)
-      float pv[4][4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const int j = T * kAlsTileRows + c.lane + 32 * a;
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-          const int i = iq * 4 + cc;
-          pv[a][cc] = (j < c.nrows && i < c.rF) ? c.P[(size_t)i * c.ldP + j] : 0.f;
-        }
-      }
-      // quotients without any call in the unrolled loop (a call would keep
-      // the sixteen independent chains from overlapping); the rare unsafe
-      // ones are marked and rebuilt afterwards
-      unsigned rebuild = 0u;
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-          if (!divide) {
-            pv[a][cc] *= po[a][cc];
-          } else {
-            const float x = pv[a][cc];
-            const float qv = div_nr(x, po[a][cc]);
-            const bool ok = fabsf(x) >= FLT_MIN && fabsf(qv) <= FLT_MAX;  // also catches a zero divisor
-            const int j = T * kAlsTileRows + c.lane + 32 * a, i = iq * 4 + cc;
-            if (!ok && j < c.nrows && i < c.rF) rebuild |= 1u << (a * 4 + cc);
-            pv[a][cc] = qv;
-          }
-        }
-      // rebuilds, one entry at a time by the whole warp
-      for (unsigned pending = __ballot_sync(0xffffffffu, rebuild != 0u); pending;
-           pending = __ballot_sync(0xffffffffu, rebuild != 0u)) {
-        const int L = __ffs(pending) - 1;
-        const int bit = __ffs(__shfl_sync(0xffffffffu, rebuild, L)) - 1;
-        const int a = bit >> 2, cc = bit & 3;
-        const float qv = rebuild_product(c, p, T * kAlsTileRows + L + 32 * a, iq * 4 + cc, ex, d);
-        if (c.lane == L) {
-          rebuild &= rebuild - 1;
-#pragma unroll
-          for (int a2 = 0; a2 < 4; ++a2)
-#pragma unroll
-            for (int c2 = 0; c2 < 4; ++c2)
-              if (a2 * 4 + c2 == bit) pv[a2][c2] = qv;
-        }
-      }
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const int j = T * kAlsTileRows + c.lane + 32 * a;
-        if (j >= c.nrows) continue;
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-          const int i = iq * 4 + cc;
-          if (i < c.rF) c.P[(size_t)i * c.ldP + j] = pv[a][cc];
-        }
-      }
+      const bool full = (T + 1) * kAlsTileRows <= c.nrows && iq * 4 + 4 <= c.rF;
+      if (full) product_item<true>(c, p, tile, gs, np, d, divide, ex, T, iq);
+      else product_item<false>(c, p, tile, gs, np, d, divide, ex, T, iq);
     }
     release_tile(c, g, T, c.nIq, src);
   }
@@ -540,33 +574,34 @@ __device__ void product_pass(const Cta& c, const AlsParams& p, unsigned seq, int
 
 // Phase B, first right-hand-side columns [0, MW) (round 0): P(j,i) *= <G_j^kp,
 // Fnew_i^kp>, then acc(i,m) += cG_j P(j,i) G_j^k(m) for the warp's i-quad.
-template <int MW>
+template <int MW, bool kFull>
 __device__ __forceinline__ void item_b0(const Cta& c, const float* tp, int gsp, int npp, const float* tk, int gsk,
                                         int T, int iq, float (&acc)[4][MW]) {
   float pn[4][4];
   tile_dots(tp, gsp, c.fb + iq * 4 * c.gsmax, c.gsmax, npp, c.lane, pn);
-  // every load before any store (see product_pass), then the products, then
+  // every load before any store (see product_item), then the products, then
   // the stores; w ends as the weighted products cG_j P(j,i)
   float w[4][4], cwj[4];
+  const int j0 = T * kAlsTileRows + c.lane;
+  float* P[4];
+#pragma unroll
+  for (int cc = 0; cc < 4; ++cc) P[cc] = c.P + (iq * 4 + cc) * c.ldP + j0;
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
-    const int j = T * kAlsTileRows + c.lane + 32 * a;
-    const bool live = j < c.nrows;
-    cwj[a] = live ? c.cw[j] : 0.f;
+    const bool live = kFull || j0 + 32 * a < c.nrows;
+    cwj[a] = live ? c.cw[j0 + 32 * a] : 0.f;
 #pragma unroll
-    for (int cc = 0; cc < 4; ++cc) w[a][cc] = live ? c.P[(size_t)(iq * 4 + cc) * c.ldP + j] : 0.f;
+    for (int cc = 0; cc < 4; ++cc) w[a][cc] = live ? P[cc][32 * a] : 0.f;
   }
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
     for (int cc = 0; cc < 4; ++cc) w[a][cc] *= pn[a][cc];
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int j = T * kAlsTileRows + c.lane + 32 * a;
-    if (j < c.nrows)
+  for (int a = 0; a < 4; ++a)
+    if (kFull || j0 + 32 * a < c.nrows)
 #pragma unroll
-      for (int cc = 0; cc < 4; ++cc) c.P[(size_t)(iq * 4 + cc) * c.ldP + j] = w[a][cc];
-  }
+      for (int cc = 0; cc < 4; ++cc) P[cc][32 * a] = w[a][cc];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
@@ -619,11 +654,11 @@ __device__ __forceinline__ void item_bm(const Cta& c, const float* tk, int gsk, 
   }
 }
 
-// Whether the last warp has no i-quad in phase B (16 not a multiple of the
-// i-quad count) and rF <= 32: it then inverts the step's normal equations in
-// registers during the first round.
+// Whether the last warp has no item in phase B (16 not a multiple of the
+// i-quad count, or fewer tiles than warps per i-quad) and rF <= 32: it then
+// inverts the step's normal equations in registers during the first round.
 __device__ __forceinline__ bool phase_b_inverts(const Cta& c) {
-  return !c.tc && c.rF <= 32 && (kAlsWarps / c.nIq) * c.nIq < kAlsWarps;
+  return !c.tc && c.rF <= 32 && ((kAlsWarps / c.nIq) * c.nIq < kAlsWarps || (kAlsWarps - 1) / c.nIq >= c.ntiles);
 }
 
 // Sums the 4 MW accumulators of each lane over the warp into out[cc MW + m]
@@ -667,8 +702,10 @@ __device__ __forceinline__ void warp_sum_values(const float (&acc)[4][MW], int l
 // One round of phase B over all tiles (all 16 warps; warp -> i-quad iq =
 // warp mod nIq, tiles T = warp / nIq (mod warps per i-quad)), ending with the
 // CTA's partial right-hand side columns [16 round, 16 round + MW) in bout.
+// `started`: its first tiles are on their way already.
 template <int MW>
-__device__ void phase_b_round(const Cta& c, const AlsParams& p, unsigned seq, int round, int k, int kp, float* bout) {
+__device__ void phase_b_round(const Cta& c, const AlsParams& p, unsigned seq, int round, int k, int kp, float* bout,
+                              bool started) {
   const int nk = p.nbas[k], gsk = als_gstride(nk);
   const int npp = round_up(p.nbas[kp], 4), gsp = als_gstride(p.nbas[kp]);
   const float* slab_k = c.gm + (long long)p.offg[k] * c.rG;
@@ -677,13 +714,13 @@ __device__ void phase_b_round(const Cta& c, const AlsParams& p, unsigned seq, in
   const int wpi = kAlsWarps / c.nIq;
   const bool active = c.warp < wpi * c.nIq;
   const int iq = c.warp % c.nIq, sub = c.warp / c.nIq;
-  if (c.tid == 0) start_phase(c, seq, src);
+  if (c.tid == 0 && !started) start_phase(c, seq, src);
   float acc[4][MW];
 #pragma unroll
   for (int cc = 0; cc < 4; ++cc)
 #pragma unroll
     for (int m = 0; m < MW; ++m) acc[cc][m] = 0.f;
-  if (!active && round == 0 && c.warp == kAlsWarps - 1 && phase_b_inverts(c)) {
+  if (round == 0 && c.warp == kAlsWarps - 1 && phase_b_inverts(c)) {
     // the idle warp inverts this step's normal equations (formed at the end
     // of the previous solve) for the solver warps
     const bool g = dwsolve::gj_inverse_warp(c.BB, c.rF, c.gi);
@@ -694,10 +731,14 @@ __device__ void phase_b_round(const Cta& c, const AlsParams& p, unsigned seq, in
       const unsigned g = seq + (unsigned)T;
       if (wait_tile(c, g)) {
         const float* tile = c.ring + (size_t)(g % (unsigned)c.stages) * c.stage_floats;
-        if (round == 0)
-          item_b0<MW>(c, tile, gsp, npp, tile + kAlsTileRows * gsp, gsk, T, iq, acc);
-        else
+        if (round == 0) {
+          if ((T + 1) * kAlsTileRows <= c.nrows)
+            item_b0<MW, true>(c, tile, gsp, npp, tile + kAlsTileRows * gsp, gsk, T, iq, acc);
+          else
+            item_b0<MW, false>(c, tile, gsp, npp, tile + kAlsTileRows * gsp, gsk, T, iq, acc);
+        } else {
           item_bm<MW>(c, tile, gsk, 16 * round, T, iq, acc);
+        }
       }
       release_tile(c, g, T, c.nIq, src);
     }
@@ -715,16 +756,16 @@ __device__ void phase_b_round(const Cta& c, const AlsParams& p, unsigned seq, in
 }
 
 // All rounds of phase B for mode k (previous mode kp); returns tiles used.
-__device__ unsigned phase_b(const Cta& c, const AlsParams& p, unsigned seq, int k, int kp, float* bout) {
+__device__ unsigned phase_b(const Cta& c, const AlsParams& p, unsigned seq, int k, int kp, float* bout, bool started) {
   const int npk = round_up(p.nbas[k], 4);
   unsigned used = 0;
   for (int round = 0; 16 * round < npk; ++round) {
     const int mw = min(16, npk - 16 * round);
     switch (mw) {
-      case 4: phase_b_round<4>(c, p, seq + used, round, k, kp, bout); break;
-      case 8: phase_b_round<8>(c, p, seq + used, round, k, kp, bout); break;
-      case 12: phase_b_round<12>(c, p, seq + used, round, k, kp, bout); break;
-      default: phase_b_round<16>(c, p, seq + used, round, k, kp, bout); break;
+      case 4: phase_b_round<4>(c, p, seq + used, round, k, kp, bout, started && round == 0); break;
+      case 8: phase_b_round<8>(c, p, seq + used, round, k, kp, bout, started && round == 0); break;
+      case 12: phase_b_round<12>(c, p, seq + used, round, k, kp, bout, started && round == 0); break;
+      default: phase_b_round<16>(c, p, seq + used, round, k, kp, bout, started && round == 0); break;
     }
     used += (unsigned)c.ntiles;
   }
@@ -1258,20 +1299,31 @@ __device__ void dw_suffix(const Cta& c, int t, int nt) {
 }
 
 // Gram matrix of the unit-normalised new factor of mode k (rows of X), stored
-// for the suffix products of the next sweep and folded into the prefix L.
+// for the suffix products of the next sweep, folded into the prefix L and, unless
+// the sweep ends, with the suffix sk of the next mode into the next normal
+// equations.  One thread per pair i <= i2; both triangles hold the same bits.
 __device__ void dw_new_gram(const Cta& c, int k, int nk, int t, int nt) {
   const int rF = c.rF, rr = rF * rF;
-  for (int e = t; e < rr; e += nt) {
-    const int i = e % rF, i2 = e / rF;
-    if (i > i2) continue;
+  const dw pen = c.misc[0];
+  for (int e = t; e < rF * (rF + 1) / 2; e += nt) {
+    int i2 = (int)((sqrtf(8.f * e + 1.f) - 1.f) * 0.5f);
+    i2 += (i2 + 1) * (i2 + 2) / 2 <= e ? 1 : 0;
+    i2 -= i2 * (i2 + 1) / 2 > e ? 1 : 0;
+    const int i = e - i2 * (i2 + 1) / 2, lo = i + i2 * rF, up = i2 + i * rF;
     dw_acc acc = acc_zero();
+#pragma unroll 4
     for (int q = 0; q < nk; ++q) acc_fma(acc, c.X[i + q * rF], c.X[i2 + q * rF]);
     const dw s = acc_value(acc);
-    c.gram[(size_t)k * rr + i + i2 * rF] = s;
-    c.gram[(size_t)k * rr + i2 + i * rF] = s;
+    c.gram[(size_t)k * rr + lo] = s;
+    c.gram[(size_t)k * rr + up] = s;
     if (k < c.D - 1) {
-      c.L[i + i2 * rF] = dw_mul(c.L[i + i2 * rF], s);
-      if (i != i2) c.L[i2 + i * rF] = dw_mul(c.L[i2 + i * rF], s);
+      const dw l = dw_mul(c.L[lo], s);
+      c.L[lo] = l;
+      c.L[up] = l;
+      dw b = dw_mul(l, c.sk[lo]);
+      if (i == i2) b = dw_add(b, pen);
+      c.BB[lo] = b;
+      c.BB[up] = b;
     }
   }
 }
@@ -1294,21 +1346,62 @@ __device__ void post_solve(const Cta& c, const AlsParams& p, int k, int kn, int 
     for (int i = t; i < rF; i += nt) p.coef[p.term_off[c.v] + i] = dw_to_double(c.nrm[i]);
   }
   dw_new_gram(c, k, nk, t, nt);
-  cp_async_wait_all();
+  if (k < c.D - 1) return;
+  // the sweep ends: suffix products from the new Grams, then the normal equations
   if (warp_only) __syncwarp(); else solver_sync();
-  if (k == c.D - 1) {
-    dw_suffix(c, t, nt);
-    if (warp_only) __syncwarp(); else solver_sync();
-    for (int e = t; e < rr; e += nt) c.sk[e] = c.suf[(size_t)kn * rr + e];
-  }
-  // the next step's normal equations (sk: the suffix of mode kn, copied at
-  // the start of the solve unless the sweep just ended)
+  dw_suffix(c, t, nt);
+  if (warp_only) __syncwarp(); else solver_sync();
   const dw pen = c.misc[0];
   for (int e = t; e < rr; e += nt) {
-    const dw sk = c.sk[e];
+    const dw sk = c.suf[(size_t)kn * rr + e];
+    c.sk[e] = sk;
     dw b = dw_mul(c.L[e], sk);
     if (e % rF == e / rF) b = dw_add(b, pen);
     c.BB[e] = b;
+  }
+}
+
+// refine_solve for the step; up to four entries a thread in registers (the same bits).
+__device__ __forceinline__ bool refine_step(const Cta& c, int nk, const float* inv) {
+  const int rF = c.rF, n = rF * nk;
+  float* rh = reinterpret_cast<float*>(c.res);
+  if (n <= kSolverThreads) return dwsolve::refine_solve_q<kSolverThreads, 1>(c.BB, rF, c.b0, c.X, nk, inv, rh, c.red);
+  if (n <= 2 * kSolverThreads)
+    return dwsolve::refine_solve_q<kSolverThreads, 2>(c.BB, rF, c.b0, c.X, nk, inv, rh, c.red);
+  if (n <= 4 * kSolverThreads)
+    return dwsolve::refine_solve_q<kSolverThreads, 4>(c.BB, rF, c.b0, c.X, nk, inv, rh, c.red);
+  return refine_solve(c.BB, rF, c.b0, c.X, nk, inv, c.res, c.red);
+}
+
+// b0 from the cluster's partial right-hand sides (n of them): NR >= CL parts
+// of NE entries a thread loaded together, then added in rank order.
+template <int NR, int NE>
+__device__ __forceinline__ void gather_parts(const Cta& c, const float* part, int n) {
+  const int rF = c.rF;
+  for (int e0 = c.tid; e0 < n; e0 += NE * kSolverThreads) {
+    float v[NE][NR];
+#pragma unroll
+    for (int u = 0; u < NE; ++u) {
+      const int e = e0 + u * kSolverThreads, q = e / rF, i = e - q * rF;
+      const uint32_t local = smem_addr(part + i * c.npmax + q);
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        v[u][r] = 0.f;
+        if (r < c.CL && e < n) {
+          uint32_t remote;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(r));
+          asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[u][r]) : "r"(remote) : "memory");
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < NE; ++u) {
+      dw s = dw_make(0.f);
+#pragma unroll
+      for (int r = 0; r < NR; ++r)
+        if (r < c.CL) s = dw_add_f(s, v[u][r]);
+      if (e0 + u * kSolverThreads < n) c.b0[e0 + u * kSolverThreads] = s;
+    }
   }
 }
 
@@ -1324,25 +1417,8 @@ __device__ void solve_step(const Cta& c, const AlsParams& p, cg::cluster_group& 
   const size_t boff = (size_t)(t & 1) * c.rFp * c.npmax;
   // (mapa + ld.shared::cluster: explicit distributed-shared-memory loads,
   // all issued before the sums)
-  for (int e = c.tid; e < rF * nk; e += kSolverThreads) {
-    const int i = e % rF, n = e / rF;
-    const uint32_t local = smem_addr(c.bpart + boff + i * c.npmax + n);
-    float v[16];
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-      v[r] = 0.f;
-      if (r < c.CL) {
-        uint32_t remote;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(r));
-        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[r]) : "r"(remote) : "memory");
-      }
-    }
-    dw s = dw_make(0.f);
-#pragma unroll
-    for (int r = 0; r < 16; ++r)
-      if (r < c.CL) s = dw_add_f(s, v[r]);
-    c.b0[i + n * rF] = s;
-  }
+  if (c.CL <= 4) gather_parts<4, 2>(c, c.bpart + boff, rF * nk);
+  else gather_parts<16, 2>(c, c.bpart + boff, rF * nk);
   // the normal equations BB (prefix of this sweep x suffix of the previous
   // one + penalty) were formed when the previous step ended
   solver_sync();
@@ -1363,12 +1439,13 @@ __device__ void solve_step(const Cta& c, const AlsParams& p, cg::cluster_group& 
     inv = gj_inverse(c.BB, rF, c.gi, &gj_ok);
   }
   int bad = 0;
-  if (!(gj_ok && refine_solve(c.BB, rF, c.b0, c.X, nk, inv, c.res, c.red))) {
+  if (!(gj_ok && refine_step(c, nk, inv))) {
     for (int e = c.tid; e < rF * nk; e += kSolverThreads) c.X[e] = c.b0[e];
     bad = dw_ldlt(c.BB, rF, c.dinv, c.u);
     dw_ldlt_solve(c.BB, rF, c.dinv, c.X, nk);
   }
   dwsolve::dw_normalise_rows(c.X, rF, nk, c.nrm);
+  cp_async_wait_all();  // sk
   solver_sync();
   // new factor: FP32 copy for phase B and for this CTA's rebuilds; the
   // caller's FP64 arrays from cluster rank 0
@@ -1569,7 +1646,7 @@ __global__ void __launch_bounds__(kAlsThreads, 1) als_cluster_kernel(AlsParams p
       seq += tc_phase_b(c, p, seq, tcseq, k, kp, c.bpart + (size_t)(t & 1) * c.rFp * c.npmax);
       tcseq += (unsigned)c.ntiles;
     } else {
-      seq += phase_b(c, p, seq, k, kp, c.bpart + (size_t)(t & 1) * c.rFp * c.npmax);
+      seq += phase_b(c, p, seq, k, kp, c.bpart + (size_t)(t & 1) * c.rFp * c.npmax, t > 0);
     }
     cluster_arrive();
     if (c.warp < kAlsSolverWarps) {
@@ -1577,15 +1654,24 @@ __global__ void __launch_bounds__(kAlsThreads, 1) als_cluster_kernel(AlsParams p
       solve_step(c, p, cluster, t, k, kn);
     } else {
       if (t + 1 < nsteps) {
+        if (c.tid == kAlsThreads - 32)
+          start_phase(c, seq, TileSrc{c.gm + (long long)p.offg[kn] * c.rG, als_gstride(p.nbas[kn]), nullptr, 0});
         load_factor(c, p, kn, c.fa, kSolverThreads, kAlsThreads - kSolverThreads);
         worker_sync();
-        if (c.tid == kSolverThreads)
-          start_phase(c, seq, TileSrc{c.gm + (long long)p.offg[kn] * c.rG, als_gstride(p.nbas[kn]), nullptr, 0});
         if (kTc) {
           if ((rF + 2) / 3 <= 8) tc_product_pass<8, true>(c, p, seq, tcseq, kn, k, kSolverWarpsAls, kTcDivideWarps);
           else tc_product_pass<16, true>(c, p, seq, tcseq, kn, k, kSolverWarpsAls, kTcDivideWarps);
         } else if (c.warp >= kAlsWarps - kDivideWarps) {
           product_pass(c, p, seq, kn, true, k, kAlsWarps - kDivideWarps, kDivideWarps);
+        }
+        if (!kTc) {
+          // the ring is idle: the first tiles of the next phase B load while
+          // the solve still runs (they took its first 3.5 k cycles)
+          worker_sync();
+          if (c.tid == kSolverThreads)
+            start_phase(c, seq + (unsigned)c.ntiles,
+                        TileSrc{c.gm + (long long)p.offg[k] * c.rG, als_gstride(p.nbas[k]),
+                                c.gm + (long long)p.offg[kn] * c.rG, als_gstride(p.nbas[kn])});
         }
       }
       cluster_wait();

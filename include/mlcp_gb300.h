@@ -243,6 +243,21 @@ MLCP_API int mlcp_mlp_colsum(const void *G, int rows, int n, int ld, float *db, 
  * not NULL, the transposed BF16 copy [cols][rows]. */
 MLCP_API int mlcp_mlp_adam(float *w, const float *g, float *m1, float *m2, int rows, int cols, float lr, float b1,
                            float b2, float eps, int step, void *wb, void *wt, void *stream);
+/* The same for up to six parameter matrices in one launch: matrix k has its
+ * pointers (w, g, m1, m2, wb, wt; the last two may be NULL) at t[6 k] and its rows and
+ * columns at dims[2 k]. */
+MLCP_API int mlcp_mlp_adam_layers(int count, void *const *t, const int *dims, float lr, float b1, float b2, float eps,
+                                  int step, void *stream);
+/* One forward (backward = 0) or backward pass of the three-layer network
+ * X -> H1 -> H2 -> Y (ReLU, ReLU, linear; mean squared error against T), all of
+ * its launches from one call.  dims: padded rows, valid rows, padded input, hidden
+ * and output widths, output width, row stride of X (the input width for
+ * backward).  t: status, X, H1, H1 transposed, H2, H2
+ * transposed, Y, then w and b of the layers 1 to 3 (BF16 weights); for
+ * backward also T, loss, X transposed (written), dY, dY transposed, dZ2, dZ2
+ * transposed, dZ1, dZ1 transposed, then the transposed weights and the gradients of
+ * w and b of the layers 1 to 3.  Layouts as in mlcp_mlp_gemm. */
+MLCP_API int mlcp_mlp_step(int backward, void *const *t, const int *dims, void *stream);
 /* Feature rows of a batch of reduction targets (reference layout, every
  * mode of basis size n): row v*ndof + d holds, for the ntop (<= 64)
  * largest-|weight| target terms of vector v (terms d_g_off[v] ..

@@ -114,6 +114,10 @@ def load(build_if_missing: bool = True) -> ctypes.CDLL:
         L.mlcp_mlp_colsum.argtypes = [_V, _i, _i, _i, _V, _V]
         L.mlcp_mlp_adam.restype = _i
         L.mlcp_mlp_adam.argtypes = [_V, _V, _V, _V, _i, _i, _F, _F, _F, _F, _i, _V, _V, _V]
+        L.mlcp_mlp_adam_layers.restype = _i
+        L.mlcp_mlp_adam_layers.argtypes = [_i, _V, _V, _F, _F, _F, _F, _i, _V]
+        L.mlcp_mlp_step.restype = _i
+        L.mlcp_mlp_step.argtypes = [_i, _V, _V, _V]
         L.mlcp_ws_features.restype = _i
         L.mlcp_ws_features.argtypes = [_i, _i, _i, _i, _V, _V, _i, _V, _V, _V, _i, _V]
         L.mlcp_ws_targets.restype = _i

@@ -29,6 +29,8 @@
 // the ring, and no lane writes single elements across rows.  With 256-wide
 // tiles (six CTAs), two stages and element-wise stores the five shapes of a
 // training step took 51-77 us each.
+#include <algorithm>
+
 #include <cuda_bf16.h>
 
 #include <cstdint>
@@ -396,59 +398,78 @@ __global__ void __launch_bounds__(kTileThreads) mlp_loss_kernel(const float* Y, 
   if (threadIdx.x == 0) atomicAdd(loss, part / ((float)m * (float)n));
 }
 
-// db[c] = sum over rows of G[r][c] (BF16 [rows][ld]): a CTA per 32 columns,
-// each warp every 32nd row, the warps' sums added in order (one thread per
-// column walked its rows alone: 45 us -> 5.1 us for 768 x 256).
-__global__ void __launch_bounds__(1024) mlp_colsum_kernel(const __nv_bfloat16* G, int rows, int n, int ld, float* db) {
+// db[c] = sum over rows of G[r][c] (BF16 [rows][ld]) for up to three matrices
+// (blockIdx.y): a CTA per 32 columns, each warp every 32nd row, the warps' sums added
+// in order (one thread per column walked its rows alone: 45 us -> 5.1 us for 768 x 256).
+__global__ void __launch_bounds__(1024) mlp_colsum_kernel(MlpColsums p) {
   __shared__ float red[32][33];
+  const __nv_bfloat16* G = p.G[blockIdx.y];
+  const int n = p.n[blockIdx.y], ld = p.ld[blockIdx.y];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
   float s = 0.f;
   if (c < n)
 #pragma unroll 8
-    for (int r = warp; r < rows; r += 32) s += __bfloat162float(G[(size_t)r * ld + c]);
+    for (int r = warp; r < p.rows; r += 32) s += __bfloat162float(G[(size_t)r * ld + c]);
   red[warp][lane] = s;
   __syncthreads();
   if (warp == 0 && c < n) {
     float t = 0.f;
     for (int w = 0; w < 32; ++w) t += red[w][lane];
-    db[c] = t;
+    p.db[blockIdx.y][c] = t;
   }
 }
 
-// Adam step on FP32 master parameters [rows][cols]; writes the BF16 copy
-// and, when wt is given, the transposed BF16 copy [cols][rows] (32 x 32
-// tiles, as in the loss kernel).
-__global__ void __launch_bounds__(kTileThreads) mlp_adam_kernel(float* w, const float* g, float* m1, float* m2,
-                                                                int rows, int cols, float lr, float b1, float b2,
-                                                                float eps, float c1, float c2, __nv_bfloat16* wb,
-                                                                __nv_bfloat16* wt) {
+// Adam step on FP32 master parameters [rows][cols] of up to six matrices, the tiles of
+// one after those of the other; writes the BF16 copy and the transposed BF16 copy
+// [cols][rows] where they are given (32 x 32 tiles, as in the loss kernel).
+__global__ void __launch_bounds__(kTileThreads) mlp_adam_kernel(MlpAdam p) {
   __shared__ __nv_bfloat16 tile[kTileDim][kTileDim + 2];
+  int b = blockIdx.x, k = 0;
+  while (k + 1 < p.count && b >= p.tiles[k]) b -= p.tiles[k++];
+  const MlpParam& s = p.param[k];
+  const int rows = s.rows, cols = s.cols;
   const int tx = threadIdx.x % kTileDim, ty = threadIdx.x / kTileDim;
   const int across = (cols + kTileDim - 1) / kTileDim;
-  const int r0 = blockIdx.x / across * kTileDim, x0 = blockIdx.x % across * kTileDim;
+  const int r0 = b / across * kTileDim, x0 = b % across * kTileDim;
 #pragma unroll
   for (int u = 0; u < kTileDim; u += kTileThreads / kTileDim) {
     const int r = r0 + ty + u, c = x0 + tx;
     if (r >= rows || c >= cols) continue;
     const size_t e = (size_t)r * cols + c;
-    const float gv = g[e];
-    const float a = b1 * m1[e] + (1.f - b1) * gv;
-    const float b = b2 * m2[e] + (1.f - b2) * gv * gv;
-    m1[e] = a;
-    m2[e] = b;
-    const float x = w[e] - lr * (a / c1) / (sqrtf(b / c2) + eps);
-    w[e] = x;
+    const float gv = s.g[e];
+    const float a = p.b1 * s.m1[e] + (1.f - p.b1) * gv;
+    const float v = p.b2 * s.m2[e] + (1.f - p.b2) * gv * gv;
+    s.m1[e] = a;
+    s.m2[e] = v;
+    const float x = s.w[e] - p.lr * (a / p.c1) / (sqrtf(v / p.c2) + p.eps);
+    s.w[e] = x;
     const __nv_bfloat16 xb = __float2bfloat16_rn(x);
-    if (wb) wb[e] = xb;
+    if (s.wb) s.wb[e] = xb;
     tile[ty + u][tx] = xb;
   }
-  if (!wt) return;
+  if (!s.wt) return;
   __syncthreads();
 #pragma unroll
   for (int u = 0; u < kTileDim; u += kTileThreads / kTileDim) {
     const int c = x0 + ty + u, r = r0 + tx;
-    if (r < rows && c < cols) wt[(size_t)c * rows + r] = tile[tx][ty + u];
+    if (r < rows && c < cols) s.wt[(size_t)c * rows + r] = tile[tx][ty + u];
   }
+}
+
+// out[c][r] = in[r][c], BF16 (32 x 32 tiles).
+__global__ void __launch_bounds__(kTileThreads) mlp_transpose_kernel(const __nv_bfloat16* in, int rows, int cols,
+                                                                     __nv_bfloat16* out) {
+  __shared__ __nv_bfloat16 tile[kTileDim][kTileDim + 2];
+  const int tx = threadIdx.x % kTileDim, ty = threadIdx.x / kTileDim;
+  const int across = (cols + kTileDim - 1) / kTileDim;
+  const int r0 = blockIdx.x / across * kTileDim, c0 = blockIdx.x % across * kTileDim;
+#pragma unroll
+  for (int u = 0; u < kTileDim; u += kTileThreads / kTileDim)
+    if (r0 + ty + u < rows && c0 + tx < cols) tile[ty + u][tx] = in[(size_t)(r0 + ty + u) * cols + c0 + tx];
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < kTileDim; u += kTileThreads / kTileDim)
+    if (c0 + ty + u < cols && r0 + tx < rows) out[(size_t)(c0 + ty + u) * rows + r0 + tx] = tile[tx][ty + u];
 }
 
 int mlp_loss_launch(const float* Y, const float* T, int m, int n, int ld, int rows_p, __nv_bfloat16* dY,
@@ -458,19 +479,85 @@ int mlp_loss_launch(const float* Y, const float* T, int m, int n, int ld, int ro
   return kOk;
 }
 
-int mlp_colsum_launch(const __nv_bfloat16* G, int rows, int n, int ld, float* db, cudaStream_t st) {
-  mlp_colsum_kernel<<<(n + 31) / 32, 1024, 0, st>>>(G, rows, n, ld, db);
+int mlp_colsums_launch(const MlpColsums& p, int count, cudaStream_t st) {
+  int n = 0;
+  for (int k = 0; k < count; ++k) n = std::max(n, p.n[k]);
+  mlp_colsum_kernel<<<dim3((n + 31) / 32, count), 1024, 0, st>>>(p);
   MLCP_CUDA_TRY(cudaGetLastError());
   return kOk;
 }
 
-int mlp_adam_launch(float* w, const float* g, float* m1, float* m2, int rows, int cols, float lr, float b1, float b2,
-                    float eps, int step, __nv_bfloat16* wb, __nv_bfloat16* wt, cudaStream_t st) {
-  const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
-  mlp_adam_kernel<<<tile_count(rows, cols), kTileThreads, 0, st>>>(w, g, m1, m2, rows, cols, lr, b1, b2, eps, c1, c2,
-                                                                   wb, wt);
+int mlp_colsum_launch(const __nv_bfloat16* G, int rows, int n, int ld, float* db, cudaStream_t st) {
+  MlpColsums p{};
+  p.rows = rows;
+  p.G[0] = G; p.n[0] = n; p.ld[0] = ld; p.db[0] = db;
+  return mlp_colsums_launch(p, 1, st);
+}
+
+int mlp_adam_launch(MlpAdam p, int step, cudaStream_t st) {
+  p.c1 = 1.f - powf(p.b1, (float)step);
+  p.c2 = 1.f - powf(p.b2, (float)step);
+  int total = 0;
+  for (int k = 0; k < p.count; ++k) total += p.tiles[k] = (int)tile_count(p.param[k].rows, p.param[k].cols);
+  mlp_adam_kernel<<<total, kTileThreads, 0, st>>>(p);
   MLCP_CUDA_TRY(cudaGetLastError());
   return kOk;
+}
+
+namespace {
+MlpGemm gemm_of(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, int M, int N, int K, int valid_m,
+                int* status) {
+  MlpGemm g{};
+  g.A = A; g.B = B; g.M = M; g.N = N; g.K = K; g.lda = lda; g.ldb = ldb;
+  g.valid_m = valid_m; g.status = status;
+  return g;
+}
+}  // namespace
+
+int mlp_forward(const MlpStep& s, cudaStream_t st) {
+  const int M = s.rows_p, h = s.h_p;
+  MlpGemm g = gemm_of(s.X, s.ldx, s.w[0], s.in_p, M, h, s.in_p, s.rows, s.status);
+  g.bias = s.b[0]; g.act = 1; g.Cb = s.H1; g.ldcb = h; g.Ct = s.H1t; g.ldct = M;
+  if (int rc = mlp_gemm_launch(g, st)) return rc;
+  g = gemm_of(s.H1, h, s.w[1], h, M, h, h, s.rows, s.status);
+  g.bias = s.b[1]; g.act = 1; g.Cb = s.H2; g.ldcb = h; g.Ct = s.H2t; g.ldct = M;
+  if (int rc = mlp_gemm_launch(g, st)) return rc;
+  g = gemm_of(s.H2, h, s.w[2], h, M, s.out_p, h, s.rows, s.status);
+  g.bias = s.b[2]; g.C = s.Y; g.ldc = s.out_p;
+  return mlp_gemm_launch(g, st);
+}
+
+int mlp_backward(const MlpStep& s, cudaStream_t st) {
+  const int M = s.rows_p, h = s.h_p, o = s.out_p;
+  MLCP_CUDA_TRY(cudaMemsetAsync(s.loss, 0, sizeof(float), st));
+  if (int rc = mlp_loss_launch(s.Y, s.T, s.rows, s.out_dim, o, M, s.dY, s.dYt, s.loss, st)) return rc;
+  mlp_transpose_kernel<<<tile_count(M, s.in_p), kTileThreads, 0, st>>>(s.X, M, s.in_p, s.Xt);
+  MLCP_CUDA_TRY(cudaGetLastError());
+  // layer 3: dW3 = dY^T H2, dZ2 = (dY W3) * (H2 > 0)
+  MlpGemm g = gemm_of(s.dYt, M, s.H2t, M, o, h, M, o, s.status);
+  g.C = s.gw[2]; g.ldc = h;
+  if (int rc = mlp_gemm_launch(g, st)) return rc;
+  g = gemm_of(s.dY, o, s.wt[2], o, M, h, o, s.rows, s.status);
+  g.act = 2; g.mask = s.H2; g.ldm = h; g.Cb = s.dZ2; g.ldcb = h; g.Ct = s.dZ2t; g.ldct = M;
+  if (int rc = mlp_gemm_launch(g, st)) return rc;
+  // layer 2
+  g = gemm_of(s.dZ2t, M, s.H1t, M, h, h, M, h, s.status);
+  g.C = s.gw[1]; g.ldc = h;
+  if (int rc = mlp_gemm_launch(g, st)) return rc;
+  g = gemm_of(s.dZ2, h, s.wt[1], h, M, h, h, s.rows, s.status);
+  g.act = 2; g.mask = s.H1; g.ldm = h; g.Cb = s.dZ1; g.ldcb = h; g.Ct = s.dZ1t; g.ldct = M;
+  if (int rc = mlp_gemm_launch(g, st)) return rc;
+  // layer 1
+  g = gemm_of(s.dZ1t, M, s.Xt, M, h, s.in_p, M, h, s.status);
+  g.C = s.gw[0]; g.ldc = s.in_p;
+  if (int rc = mlp_gemm_launch(g, st)) return rc;
+  // the bias gradients: column sums of dY, dZ2, dZ1
+  MlpColsums c{};
+  c.rows = M;
+  c.G[0] = s.dY; c.n[0] = c.ld[0] = o; c.db[0] = s.gb[2];
+  c.G[1] = s.dZ2; c.n[1] = c.ld[1] = h; c.db[1] = s.gb[1];
+  c.G[2] = s.dZ1; c.n[2] = c.ld[2] = h; c.db[2] = s.gb[0];
+  return mlp_colsums_launch(c, 3, st);
 }
 
 }  // namespace mlcp

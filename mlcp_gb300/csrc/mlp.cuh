@@ -35,9 +35,42 @@ struct MlpGemm {
 int mlp_gemm_launch(const MlpGemm& g, cudaStream_t st);
 int mlp_loss_launch(const float* Y, const float* T, int m, int n, int ld, int rows_p, __nv_bfloat16* dY,
                     __nv_bfloat16* dYt, float* loss, cudaStream_t st);
+// Column sums of up to three matrices of the same rows.
+struct MlpColsums {
+  const __nv_bfloat16* G[3];
+  int n[3], ld[3];
+  float* db[3];
+  int rows;
+};
+int mlp_colsums_launch(const MlpColsums& p, int count, cudaStream_t st);
 int mlp_colsum_launch(const __nv_bfloat16* G, int rows, int n, int ld, float* db, cudaStream_t st);
-int mlp_adam_launch(float* w, const float* g, float* m1, float* m2, int rows, int cols, float lr, float b1, float b2,
-                    float eps, int step, __nv_bfloat16* wb, __nv_bfloat16* wt, cudaStream_t st);
+// One Adam step of up to six parameter matrices.
+struct MlpParam {
+  float* w;
+  const float* g;
+  float *m1, *m2;
+  __nv_bfloat16 *wb, *wt;  // BF16 copies, may be null
+  int rows, cols;
+};
+struct MlpAdam {
+  MlpParam param[6];
+  int count, tiles[6];     // tiles: set by the launch
+  float lr, b1, b2, eps, c1, c2;  // c1, c2: set by the launch
+};
+int mlp_adam_launch(MlpAdam p, int step, cudaStream_t st);
+
+// The three-layer network's buffers for one forward or backward pass (padded rows
+// rows_p, of them `rows` valid): layer k maps X, H1, H2 to H1, H2, Y.
+struct MlpStep {
+  int rows_p, rows, in_p, h_p, out_p, out_dim, ldx;  // ldx: row stride of X
+  const __nv_bfloat16 *X, *w[3], *wt[3];
+  const float *b[3], *T;
+  __nv_bfloat16 *H1, *H1t, *H2, *H2t, *Xt, *dY, *dYt, *dZ2, *dZ2t, *dZ1, *dZ1t;
+  float *Y, *loss, *gw[3], *gb[3];
+  int* status;
+};
+int mlp_forward(const MlpStep& s, cudaStream_t st);
+int mlp_backward(const MlpStep& s, cudaStream_t st);
 
 // Feature rows, training targets and proposals of the warm start (one row
 // per (vector, mode); every mode has the same basis size n).

@@ -327,8 +327,75 @@ extern "C" int mlcp_mlp_adam(float* w, const float* g, float* m1, float* m2, int
   int rc = kOk;
   cudaStream_t st = ws_stream(stream, &rc);
   if (rc) return finish_status(rc);
-  return finish_status(mlp_adam_launch(w, g, m1, m2, rows, cols, lr, b1, b2, eps, step,
-                                       static_cast<__nv_bfloat16*>(wb), static_cast<__nv_bfloat16*>(wt), st));
+  MlpAdam p{};
+  p.count = 1;
+  p.param[0] = MlpParam{w, g, m1, m2, static_cast<__nv_bfloat16*>(wb), static_cast<__nv_bfloat16*>(wt), rows, cols};
+  p.lr = lr; p.b1 = b1; p.b2 = b2; p.eps = eps;
+  return finish_status(mlp_adam_launch(p, step, st));
+}
+
+extern "C" int mlcp_mlp_adam_layers(int count, void* const* t, const int* dims, float lr, float b1, float b2, float eps,
+                                    int step, void* stream) {
+  int rc = kOk;
+  cudaStream_t st = ws_stream(stream, &rc);
+  if (rc) return finish_status(rc);
+  if (count < 1 || count > 6 || !t || !dims) {
+    set_error("mlcp_mlp_adam_layers: bad arguments");
+    return finish_status(kBadArgument);
+  }
+  MlpAdam p{};
+  p.count = count;
+  for (int k = 0; k < count; ++k) {
+    void* const* q = t + 6 * k;
+    p.param[k] = MlpParam{static_cast<float*>(q[0]), static_cast<const float*>(q[1]), static_cast<float*>(q[2]),
+                          static_cast<float*>(q[3]), static_cast<__nv_bfloat16*>(q[4]),
+                          static_cast<__nv_bfloat16*>(q[5]), dims[2 * k], dims[2 * k + 1]};
+  }
+  p.lr = lr; p.b1 = b1; p.b2 = b2; p.eps = eps;
+  return finish_status(mlp_adam_launch(p, step, st));
+}
+
+namespace {
+// mlcp_mlp_step's buffers, in the order of include/mlcp_gb300.h.
+MlpStep make_step(void* const* t, const int* dims, bool backward) {
+  using bf = __nv_bfloat16;
+  MlpStep s{};
+  s.rows_p = dims[0]; s.rows = dims[1]; s.in_p = dims[2]; s.h_p = dims[3]; s.out_p = dims[4]; s.out_dim = dims[5]; s.ldx = dims[6];
+  auto b16 = [&](int i) { return static_cast<bf*>(t[i]); };
+  auto f32 = [&](int i) { return static_cast<float*>(t[i]); };
+  s.status = static_cast<int*>(t[0]);
+  s.X = b16(1); s.H1 = b16(2); s.H1t = b16(3); s.H2 = b16(4); s.H2t = b16(5); s.Y = f32(6);
+  for (int k = 0; k < 3; ++k) {
+    s.w[k] = b16(7 + 2 * k);
+    s.b[k] = f32(8 + 2 * k);
+  }
+  if (!backward) return s;
+  s.T = f32(13); s.loss = f32(14); s.Xt = b16(15); s.dY = b16(16); s.dYt = b16(17);
+  s.dZ2 = b16(18); s.dZ2t = b16(19); s.dZ1 = b16(20); s.dZ1t = b16(21);
+  for (int k = 0; k < 3; ++k) {
+    s.wt[k] = b16(22 + 3 * k);
+    s.gw[k] = f32(23 + 3 * k);
+    s.gb[k] = f32(24 + 3 * k);
+  }
+  return s;
+}
+}  // namespace
+
+extern "C" int mlcp_mlp_step(int backward, void* const* t, const int* dims, void* stream) {
+  int rc = kOk;
+  cudaStream_t st = ws_stream(stream, &rc);
+  if (rc) return finish_status(rc);
+  if (!t || !dims) {
+    set_error("mlcp_mlp_step: bad arguments");
+    return finish_status(kBadArgument);
+  }
+  for (int i = 1; i < (backward ? 31 : 13); ++i)
+    if (!t[i]) {
+      set_error("mlcp_mlp_step: buffer %d is null", i);
+      return finish_status(kBadArgument);
+    }
+  const MlpStep s = make_step(t, dims, backward != 0);
+  return finish_status(backward ? mlp_backward(s, st) : mlp_forward(s, st));
 }
 
 namespace {

@@ -27,10 +27,6 @@ def _pad(x: int, m: int) -> int:
     return (x + m - 1) // m * m
 
 
-def _ptr(t) -> int:
-    return t.data_ptr()
-
-
 def torch_stream():
     """Handle of torch's current stream for the library calls, so that they
     order with the torch operations that fill and read the buffers (the
@@ -91,15 +87,16 @@ class Mlp:
         self.loss = t.zeros(1, dtype=t.float32, device=self.dev)
         self._rows = rows_p
 
-    def _gemm(self, A, B, M, N, K, bias=None, act=0, mask=None, C=None, Cb=None, Ct=None, valid_m=None):
-        L = _lib.load()
-        rc = L.mlcp_mlp_gemm(_ptr(A), _ptr(B), M, N, K, A.shape[1], B.shape[1], _ptr(bias) if bias is not None else None,
-                             act, _ptr(mask) if mask is not None else None, mask.shape[1] if mask is not None else 0,
-                             _ptr(C) if C is not None else None, C.shape[1] if C is not None else 0,
-                             _ptr(Cb) if Cb is not None else None, Cb.shape[1] if Cb is not None else 0,
-                             _ptr(Ct) if Ct is not None else None, Ct.shape[1] if Ct is not None else 0,
-                             M if valid_m is None else valid_m, _ptr(self.status), torch_stream())
-        _lib.check(rc)
+    def _step(self, backward: bool, Xp, rows: int, *more):
+        """One library call for all launches of a pass: the buffers' addresses of
+        this call, in the order of mlcp_mlp_step."""
+        bufs = [self.status, Xp, self.H1, self.H1t, self.H2, self.H2t, self.Y]
+        for Ly in self.layers:
+            bufs += (Ly["wb"], Ly["b"])
+        bufs += more
+        t = (ctypes.c_void_p * len(bufs))(*[b.data_ptr() for b in bufs])
+        dims = (ctypes.c_int * 7)(Xp.shape[0], rows, self.in_p, self.h_p, self.out_p, self.out_dim, Xp.shape[1])
+        _lib.check(_lib.load().mlcp_mlp_step(int(backward), t, dims, torch_stream()))
 
     def pad_inputs(self, X):
         """BF16 [rows_p][in_p] copy of X (rows x in_dim, any float dtype)."""
@@ -112,52 +109,31 @@ class Mlp:
 
     def forward(self, Xp, rows: int):
         """Xp: BF16 [rows_p][in_p] (pad_inputs).  Returns Y FP32 [rows_p][out_p]."""
-        rows_p = Xp.shape[0]
-        self._buffers(rows_p)
-        L1, L2, L3 = self.layers
-        self._gemm(Xp, L1["wb"], rows_p, self.h_p, self.in_p, bias=L1["b"], act=1, Cb=self.H1, Ct=self.H1t,
-                   valid_m=rows)
-        self._gemm(self.H1, L2["wb"], rows_p, self.h_p, self.h_p, bias=L2["b"], act=1, Cb=self.H2, Ct=self.H2t,
-                   valid_m=rows)
-        self._gemm(self.H2, L3["wb"], rows_p, self.out_p, self.h_p, bias=L3["b"], act=0, C=self.Y, valid_m=rows)
+        self._buffers(Xp.shape[0])
+        self._step(False, Xp, rows)
         return self.Y
 
     def backward(self, Xp, rows: int, T):
         """Gradients of the mean squared error of the last forward against T
         (FP32 [rows_p][out_p]; columns >= out_dim ignored) into each layer's
         gw/gb.  Returns the loss (device scalar)."""
-        L = _lib.load()
-        rows_p = Xp.shape[0]
-        L1, L2, L3 = self.layers
-        self.loss.zero_()
-        _lib.check(L.mlcp_mlp_loss(_ptr(self.Y), _ptr(T), rows, self.out_dim, self.out_p, rows_p, _ptr(self.dY),
-                                   _ptr(self.dYt), _ptr(self.loss), torch_stream()))
-        self.Xt.copy_(Xp.t())
-        # layer 3: dW3 = dY^T H2, db3 = colsum dY, dZ2 = (dY W3) * (H2 > 0)
-        self._gemm(self.dYt, self.H2t, self.out_p, self.h_p, rows_p, C=L3["gw"])
-        _lib.check(L.mlcp_mlp_colsum(_ptr(self.dY), rows_p, self.out_p, self.out_p, _ptr(L3["gb"]), torch_stream()))
-        self._gemm(self.dY, L3["wt"], rows_p, self.h_p, self.out_p, act=2, mask=self.H2, Cb=self.dZ2, Ct=self.dZ2t,
-                   valid_m=rows)
-        # layer 2
-        self._gemm(self.dZ2t, self.H1t, self.h_p, self.h_p, rows_p, C=L2["gw"])
-        _lib.check(L.mlcp_mlp_colsum(_ptr(self.dZ2), rows_p, self.h_p, self.h_p, _ptr(L2["gb"]), torch_stream()))
-        self._gemm(self.dZ2, L2["wt"], rows_p, self.h_p, self.h_p, act=2, mask=self.H1, Cb=self.dZ1, Ct=self.dZ1t,
-                   valid_m=rows)
-        # layer 1
-        self._gemm(self.dZ1t, self.Xt, self.h_p, self.in_p, rows_p, C=L1["gw"])
-        _lib.check(L.mlcp_mlp_colsum(_ptr(self.dZ1), rows_p, self.h_p, self.h_p, _ptr(L1["gb"]), torch_stream()))
+        if tuple(Xp.shape) != (self._rows, self.in_p):
+            raise RuntimeError(f"inputs of shape {tuple(Xp.shape)}, the last forward's were {(self._rows, self.in_p)}")
+        more = [T, self.loss, self.Xt, self.dY, self.dYt, self.dZ2, self.dZ2t, self.dZ1, self.dZ1t]
+        for Ly in self.layers:
+            more += (Ly["wt"], Ly["gw"], Ly["gb"])
+        self._step(True, Xp, rows, *more)
         return self.loss
 
     def adam(self, lr: float = 1e-3, b1: float = 0.9, b2: float = 0.999, eps: float = 1e-8):
-        L = _lib.load()
         self.step_no += 1
+        t, dims = [], []
         for Ly in self.layers:
-            _lib.check(L.mlcp_mlp_adam(_ptr(Ly["w"]), _ptr(Ly["gw"]), _ptr(Ly["mw"]), _ptr(Ly["vw"]), Ly["rows"],
-                                       Ly["cols"], ctypes.c_float(lr), ctypes.c_float(b1), ctypes.c_float(b2),
-                                       ctypes.c_float(eps), self.step_no, _ptr(Ly["wb"]), _ptr(Ly["wt"]), torch_stream()))
-            _lib.check(L.mlcp_mlp_adam(_ptr(Ly["b"]), _ptr(Ly["gb"]), _ptr(Ly["mb"]), _ptr(Ly["vb"]), 1, Ly["rows"],
-                                       ctypes.c_float(lr), ctypes.c_float(b1), ctypes.c_float(b2),
-                                       ctypes.c_float(eps), self.step_no, None, None, torch_stream()))
+            t += [Ly[k].data_ptr() for k in ("w", "gw", "mw", "vw", "wb", "wt")]
+            t += [Ly[k].data_ptr() for k in ("b", "gb", "mb", "vb")] + [None, None]
+            dims += (Ly["rows"], Ly["cols"], 1, Ly["rows"])
+        _lib.check(_lib.load().mlcp_mlp_adam_layers(6, (ctypes.c_void_p * 36)(*t), (ctypes.c_int * 12)(*dims), lr, b1, b2,
+                                                    eps, self.step_no, torch_stream()))
 
     def check_status(self):
         if int(self.status.item()) != 0:

@@ -655,16 +655,16 @@ int qhq_full(Context* ctx, const double* base, const double* coef, const int* nb
   double* qc = reinterpret_cast<double*>(b + o_qc);
   double* y = reinterpret_cast<double*>(b + o_y);
   double* A = reinterpret_cast<double*>(b + o_a);
-  double* S = reinterpret_cast<double*>(b + o_s);
+  double* S = s_out ? reinterpret_cast<double*>(b + o_s) : nullptr;  // overlaps only when asked for
   MLCP_CUDA_TRY(cudaMemcpyAsync(q, base, sizeof(double) * nvals, cudaMemcpyHostToDevice, st));
   MLCP_CUDA_TRY(cudaMemcpyAsync(qc, coef, sizeof(double) * B * R, cudaMemcpyHostToDevice, st));
   if ((rc = rq_apply_launch(tab, B, Ly.nD, q, y, st))) return rc;
   RqPairParams rp;
   rp.ops = tab; rp.nvec = B; rp.nD = Ly.nD; rp.base = q; rp.coef = qc; rp.y = y; rp.A = A; rp.S = S;
   if ((rc = rq_pair_launch(rp, (int)ctx->smem_optin, st))) return rc;
-  std::vector<double> ha((size_t)B * B), hs((size_t)B * B);
+  std::vector<double> ha((size_t)B * B), hs(S ? (size_t)B * B : 0);
   MLCP_CUDA_TRY(cudaMemcpyAsync(ha.data(), A, sizeof(double) * B * B, cudaMemcpyDeviceToHost, st));
-  MLCP_CUDA_TRY(cudaMemcpyAsync(hs.data(), S, sizeof(double) * B * B, cudaMemcpyDeviceToHost, st));
+  if (S) MLCP_CUDA_TRY(cudaMemcpyAsync(hs.data(), S, sizeof(double) * B * B, cudaMemcpyDeviceToHost, st));
   MLCP_CUDA_TRY(cudaStreamSynchronize(st));
   for (int j = 0; j < B; ++j)
     for (int i = j; i < B; ++i) {

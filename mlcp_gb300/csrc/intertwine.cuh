@@ -173,7 +173,7 @@ struct RqPairParams {
   const double* coef;
   const double* y;  // [nvec][utot][R][npmax]
   double* A;
-  double* S;
+  double* S;  // or null: no overlaps
 };
 int rq_apply_launch(const OpTable& t, int nvec, int nD, const double* base, double* y, cudaStream_t st);
 int rq_pair_launch(const RqPairParams& p, int smem_optin, cudaStream_t st);

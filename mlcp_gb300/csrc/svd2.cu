@@ -52,6 +52,7 @@ constexpr int kSvdThreads = 1024;
 constexpr int kSvdWarps = kSvdThreads / 32;
 constexpr int kPairLanes = 16;                  // lanes per column pair in the sweeps
 constexpr int kGroupsPerWarp = 32 / kPairLanes;
+constexpr int kFormThreads = 256, kFormTerms = 32, kFormStage = 64;
 constexpr int kMaxN = 256;       // min(nr, nc)
 constexpr int kMaxM = 4096;      // max(nr, nc)
 constexpr int kMaxSweeps = 40;
@@ -83,43 +84,61 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// M(i, j) of vector blockIdx.y, i < m (row factor), j < n (column factor),
-// stored at work[v][j * m + i].
-__global__ void __launch_bounds__(256) svd2_form_kernel(Svd2Params p) {
+// M(i, j) of vector blockIdx.y, i < m (row factor), j < n (column factor), stored at
+// work[v][j * m + i], one entry per thread.  FP64-bound, so the products of the weights with
+// the mode-1 factors are formed once per CTA, in shared memory, when its 256 entries have
+// few of them (64 matrices of 40 x 40 from 336 terms: 85 us, 145 with a product per
+// entry; H v of 144 vectors on 12 x 12: 127, 262).
+__global__ void __launch_bounds__(kFormThreads) svd2_form_kernel(Svd2Params p) {
+  __shared__ double cx[kFormTerms][kFormStage];
   const Shape s = shape_of(p.nr, p.nc);
   const int v = blockIdx.y;
-  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (long long)s.m * s.n) return;
+  const long long e0 = (long long)blockIdx.x * kFormThreads, last = (long long)s.m * s.n - 1;
+  const bool live = e0 + threadIdx.x <= last;
+  const long long e = live ? e0 + threadIdx.x : last;
   const int j = (int)(e / s.m), i = (int)(e - (long long)j * s.m);
   // row factor: mode 2 when transposed, else mode 1; column factor the other
   const int ia = s.tr ? j : i, ib = s.tr ? i : j;  // index into mode 1 / mode 2
+  // the mode-1 indices of this CTA: all rows, or (transposed) its columns
+  const long long e1 = e0 + kFormThreads - 1 < last ? e0 + kFormThreads - 1 : last;
+  const int a0 = s.tr ? (int)(e0 / s.m) : 0, na = s.tr ? (int)(e1 / s.m) - a0 + 1 : s.m;
+  const bool staged = na <= kFormStage;
+  // to + sum_k (c_k x_k[ia]) y_k[ib] over n terms, strides ldx and ldy (every thread)
+  auto add_terms = [&](const double* c, const double* x, int ldx, const double* y, int ldy, int n, double to) {
+    if (!staged) {
+      for (int k = 0; k < n; ++k) to = fma(c[k] * x[(size_t)k * ldx + ia], y[(size_t)k * ldy + ib], to);
+      return to;
+    }
+    for (int k0 = 0; k0 < n; k0 += kFormTerms) {
+      const int kn = min(kFormTerms, n - k0);
+      __syncthreads();
+      for (int q = threadIdx.x; q < kn * na; q += kFormThreads) {
+        const int k = q / na, a = q - k * na;
+        cx[k][a] = c[k0 + k] * x[(size_t)(k0 + k) * ldx + a0 + a];
+      }
+      __syncthreads();
+#pragma unroll 8
+      for (int k = 0; k < kn; ++k) to = fma(cx[k][ia - a0], y[(size_t)(k0 + k) * ldy + ib], to);
+    }
+    return to;
+  };
   double acc = 0.0;
   if (!p.hv) {
     const int nD = p.nr + p.nc;
     const double* b = p.in_base + (p.shared_base ? (size_t)0 : (size_t)v * p.K * nD);
-    const double* c = p.in_coef + (size_t)v * p.K;
-    for (int k = 0; k < p.K; ++k) acc = fma(c[k] * b[(size_t)k * nD + ia], b[(size_t)k * nD + p.nr + ib], acc);
+    acc = add_terms(p.in_coef + (size_t)v * p.K, b, nD, b + p.nr, nD, p.K, 0.0);
   } else {
     const OpTable& t = p.ops;
-    const int R = t.R, npm = t.npmax;
+    const int R = t.R, npm = t.npmax, u0 = t.uoff[0], u1 = t.uoff[1];
     const double* y = p.y + (size_t)v * t.utot * R * npm;
     const double* c = p.v_coef + (size_t)v * R;
-    const int u0 = t.uoff[0], u1 = t.uoff[1];
-    for (int tt = 0; tt < t.T; ++tt) {
-      const double* ya = y + (size_t)(u0 + t.uid[2 * tt]) * R * npm + ia;
-      const double* yb = y + (size_t)(u1 + t.uid[2 * tt + 1]) * R * npm + ib;
-      double st = 0.0;
-      for (int r = 0; r < R; ++r) st = fma(c[r] * ya[(size_t)r * npm], yb[(size_t)r * npm], st);
-      acc = fma(t.alpha[tt], st, acc);
+    for (int tt = 0; tt <= t.T; ++tt) {  // the last: the shift terms of PRODHV (ishift = 1): - shift_v * v
+      const int ga = u0 + (tt < t.T ? t.uid[2 * tt] : 0), gb = u1 + (tt < t.T ? t.uid[2 * tt + 1] : 0);
+      const double st = add_terms(c, y + (size_t)ga * R * npm, npm, y + (size_t)gb * R * npm, npm, R, 0.0);
+      acc = fma(tt < t.T ? t.alpha[tt] : -p.shift[v], st, acc);
     }
-    // the shift terms of PRODHV (ishift = 1): - shift_v * v
-    const double* ya = y + (size_t)u0 * R * npm + ia;
-    const double* yb = y + (size_t)u1 * R * npm + ib;
-    double st = 0.0;
-    for (int r = 0; r < R; ++r) st = fma(c[r] * ya[(size_t)r * npm], yb[(size_t)r * npm], st);
-    acc = fma(-p.shift[v], st, acc);
   }
-  p.work[(size_t)v * work_doubles(s) + e] = acc;
+  if (live) p.work[(size_t)v * work_doubles(s) + e] = acc;
 }
 
 // Jacobi rotation that makes columns x and y orthogonal, from their Gram
@@ -453,8 +472,8 @@ int svd2_launch(const Svd2Params& p, int smem_optin, cudaStream_t st) {
     return kTooLarge;
   }
   const long long elems = (long long)s.m * s.n;
-  dim3 fg((unsigned)((elems + 255) / 256), (unsigned)p.nvec);
-  svd2_form_kernel<<<fg, 256, 0, st>>>(p);
+  dim3 fg((unsigned)((elems + kFormThreads - 1) / kFormThreads), (unsigned)p.nvec);
+  svd2_form_kernel<<<fg, kFormThreads, 0, st>>>(p);
   MLCP_CUDA_TRY(cudaGetLastError());
   const size_t smem = sizeof(double) * work_doubles(s);
   // static shared arrays of the kernel, with room for their alignment

@@ -112,6 +112,8 @@ size_t gs_work_doubles(int nbloc, int R, int nD, int D, int npm);
 // Q_i, of sum_k U(k,i) Q_k, weights then divided by its norm; double-word.
 struct UpdParams {
   int D, R, B, nD, npmax, nals;
+  int tile;               // block terms per shared-memory tile (cluster form; set by upd_launch)
+  int cl;                 // CTAs per output vector (a cluster; set by upd_launch)
   const int* nbas;        // [D] (device)
   const int* off;         // [D+1] reference-layout offsets (device)
   const int* h_off;       // the same in host memory, for the launches
@@ -128,6 +130,9 @@ struct UpdParams {
 };
 int upd_launch(const UpdParams& p, int smem_optin, cudaStream_t st);
 size_t upd_work_dw(int B, int R, int D, int npm);
+// The grid form (upd_grid.cu) and its scratch (dw).
+int upd_grid_launch(const UpdParams& p, cudaStream_t st);
+size_t upd_grid_dw(int B, int R, int D, int npm);
 size_t upd_qdw_dw(int B, int R, int nD);
 
 // Block Rayleigh-Ritz inner products: QHQ(i,j) = <Q_j, HQ_i>, S(i,j) = <Q_j, Q_i>, j <= i.

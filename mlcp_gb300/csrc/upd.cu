@@ -1,4 +1,5 @@
-// Vector updates of the intertwined cycle in double-word arithmetic.
+// Vector updates of the intertwined cycle in double-word arithmetic (smaller blocks;
+// upd_grid.cu has the form for larger ones).
 //
 // Reference: VectorUpdates / UPDATES_ALS (src/intertw_lcv.cu:209-304) with
 // lcv_build_linear_system(gs = false) (:75-127).  Every vector i of the block
@@ -15,260 +16,349 @@
 // are the Grams and the solve; FP32 right-hand sides are not accurate enough
 // for that rule.
 //
-// GB300 layout: the vectors are fitted independently, so a mode step of all of
-// them is three launches over the whole GPU:
-//   upd_rhs_kernel      the right-hand sides: a CTA per vector, rows i' and range
-//                       of the B R block terms lr; the products over d != k of 32
-//                       terms at a time go through shared memory into the
-//                       contraction with their mode-k factors (12-16 sums a thread);
-//   upd_solve_kernel    a CTA per vector: the ranges summed in order, the solve, the
-//                       new factor and its Gram (opstep.cuh);
-//   upd_overlap_kernel  the overlaps <Q_lr^k, F_i'^k> of every block term with every
-//                       vector's new factor: one matrix product of the two factor lists.
-// The block's factors are converted once to a double-word, mode-major copy (the
-// mode-k slice of all B R terms is one contiguous run); since F starts from Q, the
-// first overlaps are that copy's with itself.
-//
-// What bounds it: the compensated multiply-add (13 FP32 instructions), 2 B^2 R^2 n of them per
-// mode step, and reading the overlaps of the other modes once
-// per step (72 MB each for 100 vectors of rank 30).  100 such vectors on a 6 x 48 node, one sweep, take
-// 4.2 ms (70 ms with a CTA per vector, operands through L2); two sweeps of 40 of rank 16 on
-// 3 x 30 take 0.33 ms (0.70 ms with a cluster of three CTAs per vector).  Blocks of 2 to 12 small vectors
-// are bound by the launches and the solves, 3 D of them per sweep, and are no slower than that form.
+// GB300 layout: a cluster of cl CTAs per output vector (the updates are
+// independent: the reference writes each new vector to the host and keeps
+// fitting the old block); cl is the largest of 1-4 that keeps the whole
+// block's clusters on the SMs at once.  The block's factors are converted
+// once to a double-word, mode-major copy shared by all CTAs (the mode-k
+// slice of all B R terms is one contiguous run, L2-resident).  CTA `rank`
+// of a cluster owns a contiguous range of the B R block terms lr and keeps
+// the per-mode overlaps Gram_d(i', lr) = <Q_lr^d, F_i'^d> of its terms with
+// the fitted vector's terms i' (only mode k changes per step) in shared memory;
+// every CTA keeps the same F Grams.  The right-hand side streams the CTA's block
+// terms through shared memory in tiles: the products w_lr prod_{d!=k}
+// Gram_d(i', lr) of a tile first, then the contraction with the tile's mode-k
+// factors, while the first warps invert BB (the refinement's preconditioner).  The
+// partial right-hand sides meet through distributed shared memory, summed in
+// rank order, so every CTA solves the identical system and holds the
+// identical new factor; one cluster barrier per mode step.  One launch covers
+// all sweeps, which is what small blocks want: their steps are a chain of barriers of
+// 10 to 30 us in all.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "common.cuh"
 #include "dword.cuh"
 #include "dwsolve.cuh"
 #include "intertwine.cuh"
-#include "opstep.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace mlcp {
 
 namespace {
 
-constexpr int kRhsThreads = 128;
-constexpr int kChunk = 32;     // block terms of one stage of the right-hand side
-constexpr int kTile = 64;      // rows and columns of an overlap tile
-constexpr int kOvThreads = 256;
-constexpr int kRhsCtas = 608;  // CTAs the right-hand side is split into: four for every SM
+constexpr int kThreads = 512;
+constexpr int kMaxCl = 4;
+constexpr int kWarps = kThreads / 32;
 
-// Scratch (dw).
-struct UpdScratch {
-  dw *gram;  // [D][B R][B R]: <Q_lr^d, F_i'^d> at row i R + i', column lr
-  dw *fg;    // [B][D][R R] Grams of F
-  dw *w;     // [B][B R] target weights U(l,i) c_lr
-  dw *fk;    // [B R][n_k] the mode's new factors
-  dw *part;  // [ranges][B][R npmax] parts of the right-hand sides (i + m R)
-  dw *pen;   // [B]
+struct UpdSmem {
+  dw* X;      // [R][npmax] solution (column-major, ld R)
+  dw* b0;     // [R][npmax] right-hand side
+  dw* res;    // [R][npmax] refinement residual
+  dw* BB;     // [R][R]
+  float* gi;  // [2][R][R] FP32 inverse of BB
+  dw* cf;     // [R] weights of F (row norms)
+  dw* dinv;   // [R]
+  dw* u;      // [R]
+  dw* misc;   // [2] penalty, norm
+  dw* red;    // [kWarps]
+  float* rred;
+  float* prow;  // [2][72] pivot rows of the inverse
+  dwsolve::ColScratch cs;
+  dw* P;      // [R][TL] products of one tile of block terms
+  dw* Qt;     // [TL][npmax] mode-k factors of the tile
+  dw* bacc;   // [max(nw, R*npmax)] partial right-hand sides
+  dw* bpart;  // [2][R*npmax] this CTA's partial right-hand side (read by the cluster)
+  dw* gram;   // [D][R][nlr] block overlaps of the CTA's terms
+  int* flags; // [4]
 };
-// Most ranges times vectors of a right-hand side.
-__host__ __device__ inline size_t upd_parts(int B) { return (size_t)kRhsCtas + B; }
-__host__ __device__ inline size_t upd_scratch(int B, int R, int D, int npm, dw* base, UpdScratch* s) {
+
+// Shared memory; nlr: block terms per CTA.
+__host__ __device__ inline size_t upd_carve(UpdSmem& s, unsigned char* base, int R, int npm, int TL, int D, int nlr) {
   size_t o = 0;
-  auto take = [&](size_t n) -> dw* {
-    dw* r = base ? base + o : nullptr;
-    o += (n + 1) / 2 * 2;
-    return r;
+  auto take = [&](size_t bytes) -> unsigned char* {
+    const size_t r = o;
+    o += (bytes + 15) / 16 * 16;
+    return base ? base + r : nullptr;
   };
-  const size_t BR = (size_t)B * R;
-  s->gram = take((size_t)D * BR * BR);
-  s->fg = take((size_t)B * D * R * R);
-  s->w = take(BR * B);
-  s->fk = take(BR * npm);
-  s->part = take(upd_parts(B) * R * npm);
-  s->pen = take(B);
+  const size_t Rn = (size_t)R * npm, RR = (size_t)R * R;
+  s.X = (dw*)take(sizeof(dw) * Rn);
+  s.b0 = (dw*)take(sizeof(dw) * Rn);
+  s.res = (dw*)take(sizeof(dw) * Rn);
+  s.BB = (dw*)take(sizeof(dw) * RR);
+  s.gi = (float*)take(sizeof(float) * 2 * RR);
+  s.cf = (dw*)take(sizeof(dw) * R);
+  s.dinv = (dw*)take(sizeof(dw) * R);
+  s.u = (dw*)take(sizeof(dw) * R);
+  s.misc = (dw*)take(sizeof(dw) * 2);
+  s.red = (dw*)take(sizeof(dw) * kWarps);
+  s.rred = (float*)take(sizeof(float) * 4);
+  s.prow = (float*)take(sizeof(float) * 2 * 72);
+  s.cs.conv = (float*)take(sizeof(float) * 64);
+  s.cs.rmax = (float*)take(sizeof(float) * 16 * 32);
+  s.cs.rsum = (dw*)take(sizeof(dw) * 16 * 32);
+  s.P = (dw*)take(sizeof(dw) * (size_t)R * TL);
+  s.Qt = (dw*)take(sizeof(dw) * (size_t)TL * npm);
+  s.bacc = (dw*)take(sizeof(dw) * (Rn > (size_t)kThreads ? Rn : (size_t)kThreads));
+  s.bpart = (dw*)take(sizeof(dw) * 2 * Rn);
+  s.gram = (dw*)take(sizeof(dw) * (size_t)D * R * nlr);
+  s.flags = (int*)take(sizeof(int) * 4);
   return o;
 }
 
-// Block factors to the double-word mode-major copy (mode d of block term lr
-// at qdw[off[d] * BR + lr * n_d + m]), target weights, penalties.
+__device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// Block terms per CTA when cl CTAs share a vector's B R terms.
+__host__ __device__ inline int upd_per(int BR, int cl) { return (BR + cl - 1) / cl; }
+
+// Global scratch (dw) of one CTA: F Grams, target weights.
+__host__ __device__ inline size_t upd_cta_dw(int BR, int R, int D, int cl) {
+  return (size_t)D * R * R + (size_t)upd_per(BR, cl);
+}
+
+// Block factors to the double-word mode-major copy: mode d of block term lr
+// at qdw[off[d] * BR + lr * n_d + m].
 __global__ void upd_prep_kernel(UpdParams p) {
   const int BR = p.B * p.R;
-  UpdScratch s;
-  upd_scratch(p.B, p.R, p.D, p.npmax, p.work, &s);
-  const long long n = (long long)BR * p.nD, nw = (long long)BR * p.B;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n + nw + p.B;
+  const long long n = (long long)BR * p.nD;
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
        e += (long long)gridDim.x * blockDim.x) {
-    if (e < n) {
-      const int lr = (int)(e / p.nD), c = (int)(e - (long long)lr * p.nD);
-      int d = 0;
-      while (p.off[d + 1] <= c) ++d;
-      const int m = c - p.off[d], nd = p.off[d + 1] - p.off[d];
-      p.qdw[(size_t)p.off[d] * BR + (size_t)lr * nd + m] = dw_from_double(p.q[e]);
-    } else if (e < n + nw) {
-      const int i = (int)((e - n) / BR), lr = (int)(e - n - (long long)i * BR);
-      s.w[e - n] = dw_from_double(p.U[lr / p.R + (size_t)i * p.B] * p.qc[lr]);
-    } else {
-      const int i = (int)(e - n - nw);
-      const double* c = p.qc + (size_t)i * p.R;
-      double pen = c[0];
-      for (int r = 1; r < p.R; ++r) pen = c[r] > pen ? c[r] : pen;
-      s.pen[i] = dw_from_double(pen * p.pen_factor);
-    }
+    const int lr = (int)(e / p.nD), c = (int)(e - (long long)lr * p.nD);
+    int d = 0;
+    while (p.off[d + 1] <= c) ++d;
+    const int m = c - p.off[d], nd = p.off[d + 1] - p.off[d];
+    p.qdw[(size_t)p.off[d] * BR + (size_t)lr * nd + m] = dw_from_double(p.q[e]);
   }
 }
 
-// Overlaps of mode d0 + blockIdx.z: a 64 x 64 tile of F's terms (rows; the block's own
-// with `first`, when the Grams of F are its diagonal blocks) and the block's.  Both
-// operands whole in shared memory, transposed; 16 sums a thread.
-__global__ void __launch_bounds__(kOvThreads) upd_overlap_kernel(UpdParams p, int d0, int first) {
-  constexpr int ld = kTile + 1;
+__device__ dw block_sum(dw v, dw* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int o = 16; o > 0; o >>= 1) v = dw_add(v, dwsolve::dw_shfl_xor(v, o));
+  __syncthreads();
+  if (lane == 0) red[warp] = v;
+  __syncthreads();
+  dw s = dw_make(0.f);
+  if (threadIdx.x == 0)
+    for (int w = 0; w < kWarps; ++w) s = dw_add(s, red[w]);
+  return s;
+}
+
+__global__ void __launch_bounds__(kThreads, 1) upd_kernel(UpdParams p) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int CL = p.cl, rank = CL > 1 ? (int)cluster.block_rank() : 0;
+  const int i = blockIdx.x / CL;
+  const int R = p.R, B = p.B, D = p.D, nD = p.nD, npm = p.npmax, RR = R * R, BR = B * R, TL = p.tile;
+  const int per = upd_per(BR, CL), lr0 = min(BR, rank * per), nlr = min(BR, lr0 + per) - lr0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  UpdScratch s;
-  upd_scratch(p.B, p.R, p.D, p.npmax, p.work, &s);
-  const int d = d0 + blockIdx.z, n = p.nbas[d], R = p.R, BR = p.B * R, c0 = blockIdx.x * kTile, r0 = blockIdx.y * kTile;
-  dw* fs = reinterpret_cast<dw*>(smem_raw);
-  dw* qs = fs + (size_t)n * ld;
-  const dw* q = p.qdw + (size_t)p.off[d] * BR;
-  const dw* f = first ? q : s.fk;
-  for (int e = threadIdx.x; e < kTile * n; e += kOvThreads) {
-    const int t = e / n, m = e - t * n;
-    fs[m * ld + t] = r0 + t < BR ? f[(size_t)r0 * n + e] : dw_make(0.f);
-    qs[m * ld + t] = c0 + t < BR ? q[(size_t)c0 * n + e] : dw_make(0.f);
-  }
-  __syncthreads();
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  dw_acc acc[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = acc_zero();
-  for (int m = 0; m < n; ++m) {
-    dw y[4];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) y[b] = qs[m * ld + tx + 16 * b];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const dw x = fs[m * ld + ty + 16 * a];
-#pragma unroll
-      for (int b = 0; b < 4; ++b) acc_fma(acc[a][b], x, y[b]);
-    }
-  }
-  dw* G = s.gram + (size_t)d * BR * BR;
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int r = r0 + ty + 16 * a, c = c0 + tx + 16 * b;
-      if (r >= BR || c >= BR) continue;
-      const dw v = acc_value(acc[a][b]);
-      G[(size_t)r * BR + c] = v;
-      if (first && r / R == c / R) s.fg[((size_t)(r / R) * p.D + d) * R * R + r % R + c % R * R] = v;
-    }
-}
-
-// Right-hand side of mode k: vector blockIdx.z, rows 8 A blockIdx.y .., block terms of range
-// blockIdx.x (`per` of them); all n_k <= 16 NC columns.
-template <int A, int NC>
-__global__ void __launch_bounds__(kRhsThreads) upd_rhs_kernel(UpdParams p, int k, int per) {
-  constexpr int TR = 8 * A, ldw = TR + 1, NP = kChunk * TR / kRhsThreads;  // NP products a thread
-  __shared__ dw ws[kChunk * ldw];
-  __shared__ dw zs[kChunk * 16 * NC];
-  UpdScratch s;
-  upd_scratch(p.B, p.R, p.D, p.npmax, p.work, &s);
-  const int R = p.R, D = p.D, BR = p.B * R, n = p.nbas[k], i = blockIdx.z, i0 = blockIdx.y * TR;
-  const int lr1 = min(BR, (int)(blockIdx.x + 1) * per);
-  const int lane = threadIdx.x % 32, wq = threadIdx.x / 32, tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const dw* q = p.qdw + (size_t)p.off[k] * BR;
-  const dw* w = s.w + (size_t)i * BR;
-  const dw* g = s.gram + ((size_t)i * R + i0 + wq) * BR + lane;
-  dw_acc acc[A][NC];
-#pragma unroll
-  for (int a = 0; a < A; ++a)
-#pragma unroll
-    for (int b = 0; b < NC; ++b) acc[a][b] = acc_zero();
-  for (int c0 = blockIdx.x * per; c0 < lr1; c0 += kChunk) {
-    const int cn = min(kChunk, lr1 - c0);
-    __syncthreads();
-    for (int e = threadIdx.x; e < cn * n; e += kRhsThreads)
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(zs + e)),
-                   "l"(q + (size_t)c0 * n + e)
-                   : "memory");
-    {
-      const bool term = lane < cn;
-      const dw w0 = term ? w[c0 + lane] : dw_make(0.f);
-      dw pr[NP];
-#pragma unroll
-      for (int u = 0; u < NP; ++u) pr[u] = term && i0 + wq + 4 * u < R ? w0 : dw_make(0.f);
-      for (int d = 0; d < D; ++d) {
-        if (d == k) continue;
-        const dw* gd = g + (size_t)d * BR * BR + c0;
-        dw v[NP];
-#pragma unroll
-        for (int u = 0; u < NP; ++u)
-          v[u] = term && i0 + wq + 4 * u < R ? gd[(size_t)(4 * u) * BR] : dw_make(0.f);
-#pragma unroll
-        for (int u = 0; u < NP; ++u) pr[u] = dw_mul(pr[u], v[u]);
-      }
-#pragma unroll
-      for (int u = 0; u < NP; ++u) ws[lane * ldw + wq + 4 * u] = pr[u];
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-    for (int c = 0; c < cn; ++c) {
-      dw z[NC];
-#pragma unroll
-      for (int b = 0; b < NC; ++b) z[b] = zs[c * n + tx + 16 * b];
-#pragma unroll
-      for (int a = 0; a < A; ++a) {
-        const dw x = ws[c * ldw + ty + 8 * a];
-#pragma unroll
-        for (int b = 0; b < NC; ++b) acc_fma(acc[a][b], x, z[b]);
-      }
-    }
-  }
-  dw* part = s.part + ((size_t)blockIdx.x * p.B + i) * R * p.npmax;
-#pragma unroll
-  for (int a = 0; a < A; ++a)
-#pragma unroll
-    for (int b = 0; b < NC; ++b) {
-      const int ip = i0 + ty + 8 * a, m = tx + 16 * b;
-      if (ip < R && m < n) part[ip + m * R] = acc_value(acc[a][b]);
-    }
-}
-
-// The solve of mode k for vector blockIdx.x; `last`: its weights are divided by its norm too
-// (src/intertw_lcv.cu:269-273).
-__global__ void __launch_bounds__(kStepThreads, 1) upd_solve_kernel(UpdParams p, int k, int nrange, int last) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  StepSmem m;
-  step_carve(m, smem_raw, p.R, p.npmax);
-  UpdScratch s;
-  upd_scratch(p.B, p.R, p.D, p.npmax, p.work, &s);
-  const int i = blockIdx.x, R = p.R, RR = R * R, D = p.D, n = p.nbas[k], rv = p.rank_v ? p.rank_v[i] : R;
-  const size_t vec = (size_t)R * p.npmax;
-  dw* G = s.fg + (size_t)i * D * RR;
-  for (int e = threadIdx.x; e < RR; e += kStepThreads) m.BB[e] = normal_equation(G, D, k, e % R, e / R, R, rv, s.pen[i]);
-  if (threadIdx.x == 0) {
-    m.flags[1] = 0;
-    m.flags[2] = 1;
-  }
-  const dw* part = s.part + i * vec;
-  for (int e = threadIdx.x; e < R * n; e += kStepThreads) {
-    dw_acc acc = acc_zero();
-    for (int r = 0; r < nrange; ++r) acc_add(acc, part[(size_t)r * p.B * vec + e]);
-    m.b0[e] = e % R >= rv ? dw_make(e / R == 0 ? 1.f : 0.f) : acc_value(acc);  // ragged padding decoupled
-  }
-  __syncthreads();
-  if (threadIdx.x < 32 * dwsolve::invert_warps(R)) dwsolve::invert_any(m.BB, R, m.gi, m.prow, m.flags + 2);
-  __syncthreads();
-  step_solve(m, R, n);
+  UpdSmem s;
+  upd_carve(s, smem_raw, R, npm, TL, D, per);
+  dw* scr = p.work + (size_t)(i * CL + rank) * upd_cta_dw(BR, R, D, CL);
+  dw* gram = s.gram;                             // [D][R][nlr]: <Q_lr^d, F_i'^d>, own terms lr0.., lr fastest
+  dw* fg = scr;                                  // [D][R][R] F Grams (the same in every CTA of the cluster)
+  dw* w = fg + (size_t)D * RR;                   // [nlr] target weights U(l,i) c_lr of the own terms
+  double* fb = p.qn + (size_t)i * R * nD;
   double* fc = p.qnc + (size_t)i * R;
-  step_weights(m, R, rv, false, fc);
-  step_factor(m, R, n, p.qn + (size_t)i * R * p.nD + p.off[k], p.nD, s.fk + (size_t)i * R * n, n, G + (size_t)k * RR);
-  __syncthreads();
-  if (last) step_renormalise(m, R, D, G, fc);
-  if (threadIdx.x == 0 && m.flags[1]) atomicOr(&p.status[i], 1);
-}
+  const double* qi = p.q + (size_t)i * R * nD;
 
-template <int A>
-void rhs_launch(const UpdParams& p, int k, int n, dim3 grid, int per, cudaStream_t st) {
-  switch ((n + 15) / 16) {
-    case 1: upd_rhs_kernel<A, 1><<<grid, kRhsThreads, 0, st>>>(p, k, per); break;
-    case 2: upd_rhs_kernel<A, 2><<<grid, kRhsThreads, 0, st>>>(p, k, per); break;
-    case 3: upd_rhs_kernel<A, 3><<<grid, kRhsThreads, 0, st>>>(p, k, per); break;
-    default: upd_rhs_kernel<A, 4><<<grid, kRhsThreads, 0, st>>>(p, k, per);
+  // ---- set-up: F = Q_i, target weights, penalty, Grams ----
+  if (rank == 0)
+    for (int e = threadIdx.x; e < R * nD; e += kThreads) fb[e] = qi[e];
+  for (int c = threadIdx.x; c < nlr; c += kThreads) {
+    const int lr = lr0 + c;
+    w[c] = dw_from_double(p.U[lr / R + (size_t)i * B] * p.qc[lr]);
+  }
+  if (threadIdx.x == 0) {
+    double pen = p.qc[(size_t)i * R];
+    for (int r = 1; r < R; ++r) pen = p.qc[(size_t)i * R + r] > pen ? p.qc[(size_t)i * R + r] : pen;
+    s.misc[0] = dw_from_double(pen * p.pen_factor);
+    s.flags[1] = 0;
+    s.flags[2] = 1;
+  }
+  for (int d = 0; d < D; ++d) {
+    const int nd = p.nbas[d], od = p.off[d];
+    const dw* qd = p.qdw + (size_t)od * BR;
+    const dw* fd = p.qdw + (size_t)od * BR + (size_t)i * R * nd;  // F = Q_i: its own terms in the copy
+    for (int e = threadIdx.x; e < R * nlr; e += kThreads) {
+      const int ip = e / nlr, c = e - ip * nlr;
+      dw_acc acc = acc_zero();
+      for (int m = 0; m < nd; ++m) acc_fma(acc, qd[(size_t)(lr0 + c) * nd + m], fd[(size_t)ip * nd + m]);
+      gram[(size_t)d * R * nlr + e] = acc_value(acc);
+    }
+    for (int e = threadIdx.x; e < RR; e += kThreads) {
+      const int a = e % R, c = e / R;
+      dw_acc acc = acc_zero();
+      for (int m = 0; m < nd; ++m) acc_fma(acc, fd[(size_t)a * nd + m], fd[(size_t)c * nd + m]);
+      fg[(size_t)d * RR + e] = acc_value(acc);
+    }
+  }
+  __syncthreads();
+  const dw pen = s.misc[0];
+  const int rv = p.rank_v ? p.rank_v[i] : R;  // ragged: this vector's rank
+
+  int step = 0;
+  for (int sw = 0; sw < p.nals; ++sw) {
+    for (int k = 0; k < D; ++k, ++step) {
+      const int nk = p.nbas[k], ok = p.off[k];
+      const dw* qk = p.qdw + (size_t)ok * BR;
+      dw* bp = s.bpart + (size_t)(step & 1) * R * npm;
+      // -- normal equations --
+      for (int e = threadIdx.x; e < RR; e += kThreads) {
+        dw bb = dw_make(1.f);
+        for (int d = 0; d < D; ++d)
+          if (d != k) bb = dw_mul(bb, fg[(size_t)d * RR + e]);
+        if (e % R == e / R) bb = dw_add(bb, pen);
+        if (e % R >= rv || e / R >= rv) bb = dw_make(e % R == e / R ? 1.f : 0.f);  // ragged: decoupled padding
+        s.BB[e] = bb;
+      }
+      __syncthreads();
+      const int w0 = 32 * dwsolve::invert_warps(R);
+      if (threadIdx.x < w0) {
+        dwsolve::invert_any(s.BB, R, s.gi, s.prow, s.flags + 2);
+      } else {
+        // -- this CTA's part of the right-hand side, tile by tile over its block terms --
+        const int wt = threadIdx.x - w0, nw = kThreads - w0;
+        const int nout = R * nk;
+        const int nsl = nout >= nw ? 1 : nw / nout;  // slices of a tile per output
+        const int items = nout * nsl;
+        for (int it = wt; it < items; it += nw) s.bacc[it] = dw_make(0.f);
+        for (int c0 = 0; c0 < nlr; c0 += TL) {
+          const int tl = min(TL, nlr - c0);
+          for (int e = wt; e < R * tl; e += nw) {
+            const int ip = e / tl, c = e - ip * tl;
+            dw pr = w[c0 + c];
+            for (int d = 0; d < D; ++d)
+              if (d != k) pr = dw_mul(pr, gram[(size_t)d * R * nlr + (size_t)ip * nlr + c0 + c]);
+            s.P[ip * TL + c] = pr;
+          }
+          for (int e = wt; e < tl * nk; e += nw) s.Qt[e] = qk[(size_t)(lr0 + c0) * nk + e];
+          asm volatile("bar.sync 2, %0;" ::"r"(nw) : "memory");
+          for (int it = wt; it < items; it += nw) {
+            const int o = it % nout, sl = it / nout;
+            const int ip = o % R, m = o / R;
+            const int a0 = sl * tl / nsl, a1 = (sl + 1) * tl / nsl;
+            dw_acc acc = acc_zero();
+            for (int c = a0; c < a1; ++c) acc_fma(acc, s.P[ip * TL + c], s.Qt[c * nk + m]);
+            s.bacc[it] = dw_add(s.bacc[it], acc_value(acc));
+          }
+          asm volatile("bar.sync 2, %0;" ::"r"(nw) : "memory");
+        }
+        for (int o = wt; o < nout; o += nw) {
+          dw b = s.bacc[o];
+          for (int sl = 1; sl < nsl; ++sl) b = dw_add(b, s.bacc[sl * nout + o]);
+          const int ip = o % R, m = o / R;
+          bp[ip + m * R] = b;
+        }
+      }
+      // -- the cluster's partial right-hand sides, summed in rank order (a
+      // peer's part of step s is rewritten at step s + 2, after every CTA has
+      // passed the barrier of step s + 1 and so finished its gather of s) --
+      if (CL > 1) {
+        cl_arrive();
+        cl_wait();
+      } else {
+        __syncthreads();
+      }
+      for (int e = threadIdx.x; e < R * nk; e += kThreads) {
+        const int ip = e % R, m = e / R;
+        dw b;
+        if (CL > 1) {
+          const uint32_t local = (uint32_t)__cvta_generic_to_shared(bp + e);
+          dw v[kMaxCl];
+#pragma unroll
+          for (int r = 0; r < kMaxCl; ++r) {
+            v[r] = dw_make(0.f);
+            if (r < CL) {
+              uint32_t remote;
+              asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(r));
+              asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v[r].hi), "=f"(v[r].lo) : "r"(remote)
+                           : "memory");
+            }
+          }
+          b = v[0];
+#pragma unroll
+          for (int r = 1; r < kMaxCl; ++r)
+            if (r < CL) b = dw_add(b, v[r]);
+        } else {
+          b = bp[e];
+        }
+        s.b0[e] = ip >= rv ? dw_make(m == 0 ? 1.f : 0.f) : b;
+      }
+      __syncthreads();
+      // -- solve (as in the power sweep) --
+      bool gj_ok = s.flags[2] != 0;
+      bool solved = false;
+      const int nsw = dwsolve::solve_cols_warps(R, nk);
+      if (gj_ok && R <= 32 && nk <= 16 && nsw <= kWarps) {
+        if (threadIdx.x < nsw * 32) {
+          const bool ok2 = dwsolve::solve_cols_any(s.BB, R, s.b0, s.X, nk, s.gi, s.cf, s.cs);
+          if (threadIdx.x == 0) s.flags[3] = ok2;
+        }
+        __syncthreads();
+        solved = s.flags[3] != 0;
+        gj_ok = false;
+      }
+      if (!solved) {
+        if (!(gj_ok && dwsolve::refine_any<kThreads>(s.BB, R, s.b0, s.X, nk, s.gi, s.res, s.rred))) {
+          if (threadIdx.x < dwsolve::kSolverThreads) {
+            for (int e = threadIdx.x; e < R * nk; e += dwsolve::kSolverThreads) s.X[e] = s.b0[e];
+            const int bad = dwsolve::dw_ldlt(s.BB, R, s.dinv, s.u);
+            dwsolve::dw_ldlt_solve(s.BB, R, s.dinv, s.X, nk);
+            if (threadIdx.x == 0 && bad) s.flags[1] = 1;
+          }
+          __syncthreads();
+        }
+        dwsolve::dw_normalise_rows<kThreads>(s.X, R, nk, s.cf);
+        __syncthreads();
+      }
+      if (threadIdx.x == 0) s.flags[2] = 1;
+      for (int r = rv + threadIdx.x; r < R; r += kThreads) s.cf[r] = dw_make(0.f);  // ragged: weightless padding
+      // -- the new factor: FP64 output (rank 0), its Gram, the own block overlaps of mode k --
+      if (rank == 0)
+        for (int e = threadIdx.x; e < R * nk; e += kThreads) {
+          const int ip = e / nk, m = e % nk;
+          fb[(size_t)ip * nD + ok + m] = dw_to_double(s.X[ip + m * R]);
+        }
+      for (int e = threadIdx.x; e < RR; e += kThreads) {
+        const int a = e % R, c = e / R;
+        if (a > c) continue;
+        dw_acc acc = acc_zero();
+        for (int m = 0; m < nk; ++m) acc_fma(acc, s.X[a + m * R], s.X[c + m * R]);
+        const dw g = acc_value(acc);
+        fg[(size_t)k * RR + a + c * R] = g;
+        fg[(size_t)k * RR + c + a * R] = g;
+      }
+      for (int e = threadIdx.x; e < R * nlr; e += kThreads) {
+        const int ip = e / nlr, c = e - ip * nlr;
+        dw_acc acc = acc_zero();
+        for (int m = 0; m < nk; ++m) acc_fma(acc, qk[(size_t)(lr0 + c) * nk + m], s.X[ip + m * R]);
+        gram[(size_t)k * R * nlr + e] = acc_value(acc);
+      }
+      __syncthreads();
+    }
+  }
+  // ---- weights divided by the norm (src/intertw_lcv.cu:269-273) ----
+  {
+    dw part = dw_make(0.f);
+    for (int e = threadIdx.x; e < RR; e += kThreads) {
+      dw prod = dw_mul(s.cf[e % R], s.cf[e / R]);
+      for (int d = 0; d < D; ++d) prod = dw_mul(prod, fg[(size_t)d * RR + e]);
+      part = dw_add(part, prod);
+    }
+    const dw tot = block_sum(part, s.red);
+    if (threadIdx.x == 0) s.misc[1] = dw_sqrt(dw_abs(tot));
+    __syncthreads();
+    const dw q = s.misc[1];
+    if (rank == 0)
+      for (int r = threadIdx.x; r < R; r += kThreads) fc[r] = dw_to_double(dw_div(s.cf[r], q));
+  }
+  if (threadIdx.x == 0 && rank == 0 && s.flags[1]) atomicOr(&p.status[i], 1);
+  // no CTA leaves while a peer may still read its shared memory
+  if (CL > 1) {
+    cl_arrive();
+    cl_wait();
   }
 }
 
@@ -284,16 +374,26 @@ size_t upd_smem_bytes(int R, int npm) {
   return o;
 }
 
+// Multiply-adds of a right-hand side in one CTA up to which the cluster form is taken.
+// Measured steps (with one of the H application), cluster against grid: 3 modes of 6, 6
+// vectors of rank 8 (0.6 k) 12.5 against 18.5 us; 4 of 20, 12 of rank 8 (3.8 k) 18.7
+// against 28.3; 2 of 10, 30 of rank 10 (7.5 k) 38.6 against 43.4; 6 of 10, 12 of
+// rank 16 (7.7 k) 29.2 against 28.6, 20 of rank 16 (12.8 k) 33.5 against 29.9, 40 (34 k)
+// 53 against 35.
+constexpr double kClusterWork = 9.0e3;
+
 }  // namespace
 
 size_t upd_work_dw(int B, int R, int D, int npm) {
-  UpdScratch s;
-  return upd_scratch(B, R, D, npm, nullptr, &s);
+  size_t most = upd_grid_dw(B, R, D, npm);
+  for (int cl = 1; cl <= kMaxCl; ++cl) most = std::max(most, (size_t)B * cl * upd_cta_dw(B * R, R, D, cl));
+  return most;
 }
 
 size_t upd_qdw_dw(int B, int R, int nD) { return (size_t)B * R * nD; }
 
-int upd_launch(const UpdParams& p, int smem_optin, cudaStream_t st) {
+int upd_launch(const UpdParams& prm, int smem_optin, cudaStream_t st) {
+  UpdParams p = prm;
   if (upd_smem_bytes(p.R, p.npmax) > (size_t)smem_optin) {
     set_error("vector updates: rank %d with %d basis functions needs more shared memory than %d bytes", p.R,
               p.npmax, smem_optin);
@@ -305,37 +405,40 @@ int upd_launch(const UpdParams& p, int smem_optin, cudaStream_t st) {
     MLCP_CUDA_TRY(cudaMemcpyAsync(p.qnc, p.qc, sizeof(double) * BR, cudaMemcpyDeviceToDevice, st));
     return kOk;
   }
-  const long long n = (long long)BR * (p.nD + p.B) + p.B;
+  const long long n = (long long)BR * p.nD;
   upd_prep_kernel<<<(int)std::min<long long>((n + 255) / 256, 4096), 256, 0, st>>>(p);
   MLCP_CUDA_TRY(cudaGetLastError());
-  StepSmem m;
-  const size_t s_solve = step_carve(m, nullptr, R, p.npmax);
-  const size_t s_ov = sizeof(dw) * 2 * (size_t)p.npmax * (kTile + 1);
-  MLCP_CUDA_TRY(cudaFuncSetAttribute(upd_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s_solve));
-  MLCP_CUDA_TRY(cudaFuncSetAttribute(upd_overlap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s_ov));
-  const int tiles = (BR + kTile - 1) / kTile;
-  if (p.D > 1) {  // mode 0 is solved before its overlaps are used
-    upd_overlap_kernel<<<dim3(tiles, tiles, p.D - 1), kOvThreads, s_ov, st>>>(p, 1, 1);
-    MLCP_CUDA_TRY(cudaGetLastError());
+  int dev = 0, nsm = 0;
+  MLCP_CUDA_TRY(cudaGetDevice(&dev));
+  MLCP_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  // CTAs per vector: the most (up to 4) that keeps every cluster of the block
+  // on the SMs at once; the largest tile that fits beside the overlaps
+  int cl = kMaxCl;
+  while (cl > 1 && p.B * cl > nsm) --cl;
+  const int per = upd_per(BR, cl);
+  size_t smem = 0;
+  p.tile = 0;
+  for (int tl = 128; tl >= 16 && !p.tile; tl /= 2) {
+    UpdSmem s;
+    smem = upd_carve(s, nullptr, R, p.npmax, tl, p.D, per);
+    if (smem <= (size_t)smem_optin) p.tile = tl;
   }
-  // ranges of the block terms: whole chunks, about four CTAs for every SM
-  const int rows = R <= 16 ? 1 : (R + 31) / 32, chunks = (BR + kChunk - 1) / kChunk;
-  const int want = std::max(1, std::min(chunks, kRhsCtas / (p.B * rows)));
-  const int per = (chunks + want - 1) / want * kChunk, nrange = (BR + per - 1) / per;
-  for (int sw = 0; sw < p.nals; ++sw)
-    for (int k = 0; k < p.D; ++k) {
-      const dim3 grid(nrange, rows, p.B);
-      if (R <= 16) rhs_launch<2>(p, k, p.h_off[k + 1] - p.h_off[k], grid, per, st);
-      else rhs_launch<4>(p, k, p.h_off[k + 1] - p.h_off[k], grid, per, st);
-      MLCP_CUDA_TRY(cudaGetLastError());
-      const bool last = sw == p.nals - 1 && k == p.D - 1;
-      upd_solve_kernel<<<p.B, kStepThreads, s_solve, st>>>(p, k, nrange, last ? 1 : 0);
-      MLCP_CUDA_TRY(cudaGetLastError());
-      if (!last) {
-        upd_overlap_kernel<<<dim3(tiles, tiles, 1), kOvThreads, s_ov, st>>>(p, k, 0);
-        MLCP_CUDA_TRY(cudaGetLastError());
-      }
-    }
+  if (!p.tile || (double)per * R * p.nD / p.D > kClusterWork) return upd_grid_launch(p, st);
+  p.cl = cl;
+  MLCP_CUDA_TRY(cudaFuncSetAttribute(upd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.B * cl);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cl;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  MLCP_CUDA_TRY(cudaLaunchKernelEx(&cfg, upd_kernel, p));
   return kOk;
 }
 

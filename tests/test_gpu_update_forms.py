@@ -1,6 +1,6 @@
-"""The vector updates (upd.cu: right-hand sides over ranges of the block's terms,
-a solve per vector, overlaps as one matrix product) against the oracle at the
-sizes where their tiles end: block terms around 64 (overlap tiles) and 32
+"""The vector updates (upd_grid.cu: right-hand sides over ranges of the block's terms,
+a solve per vector, overlaps as one matrix product; upd.cu: a cluster per vector, for
+small blocks) against the oracle at the sizes where their tiles end: block terms around 64 (overlap tiles) and 32
 (stages of a right-hand side), ranks around 16 and 32 (rows of a CTA: 16, 32,
 two times 32), bases around 16, 32, 48 and 64 (columns of a thread), more
 ranges than one, two modes, ragged ranks.  npow = 0, one or two sweeps of the
@@ -26,7 +26,9 @@ CASES = [  # nbas, rank, vectors, sweeps
     ([64, 9, 48], 32, 2, 1),
     ([12, 13, 11], 33, 4, 1),
     ([32, 12, 7], 3, 43, 1),
-    ([9, 8], 5, 13, 2),
+    ([9, 8], 5, 13, 2),              # a cluster of four CTAs per vector
+    ([6, 7, 5, 4], 6, 60, 1),        # clusters of two
+    ([6, 5, 7], 3, 100, 2),          # one CTA per vector
 ]
 
 

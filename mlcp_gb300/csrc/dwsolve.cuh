@@ -595,10 +595,11 @@ __device__ inline bool refine_solve_q(const dw* __restrict__ A, int n, const dw*
   return ok;
 }
 
-// refine_solve by threads 0 .. NT-1 for n, nrhs <= 64 (res: [n nrhs] dw).  The
-// Gram-Schmidt of a 3 x 30 node (40 vectors, rank 16, 234 solves of 16 x 30
-// entries) takes 4.57 ms with refine_solve<512>, whose entries are found at run
-// time with an atomic per thread, and 4.00 with refine_solve_q.
+// refine_solve by threads 0 .. NT-1 for n, nrhs <= 64 (res: [n nrhs] dw).  234 solves of
+// 16 x 30 entries on the chain of a Gram-Schmidt took 0.6 ms less with refine_solve_q
+// than with refine_solve<512>, whose entries are found at run time with an atomic per
+// thread; the ALS cluster kernel's solve of 20 x 12 entries by 128 threads takes 7.8 k
+// cycles and took 16.3 k.
 template <int NT>
 __device__ inline bool refine_any(const dw* A, int n, const dw* B, dw* X, int nrhs, const float* inv, dw* res,
                                   float* red) {

@@ -477,7 +477,11 @@ int intertwine_cycle(Context* ctx, double* base, double* coef, const int* nbas, 
     return kOk;
   };
   if (cycle_graph_enabled()) {
-    const unsigned long long key[16] = {(unsigned long long)(uintptr_t)ctx->cyc, bytes,
+    // the sizes per mode, which the launches are planned by (grids, instances by
+    // basis size, shared memory): lists with the same totals may differ in them
+    uint64_t modes = fnv1a(1469598103934665603ull, tab.h_nbas, sizeof(int) * ndof);
+    modes = fnv1a(modes, tab.h_uoff, sizeof(int) * (ndof + 1));
+    const unsigned long long key[17] = {(unsigned long long)(uintptr_t)ctx->cyc, bytes, modes,
                                         (unsigned long long)(uintptr_t)tab.hdw,
                                         (unsigned long long)(uintptr_t)tab.alpha, (unsigned long long)ndof,
                                         (unsigned long long)R, (unsigned long long)B, (unsigned long long)T,

@@ -33,7 +33,6 @@
 // Jacobi rounds are 0.78, the Cholesky 0.28, the three triangular solves 0.21,
 // the rotation replay 0.10 and the twelve matrix products 0.18.
 #include <algorithm>
-#include <cfloat>
 
 #include "common.cuh"
 #include "intertwine.cuh"
@@ -340,22 +339,24 @@ __device__ void phase_jacobi(const GepParams& p, const GepWork& w, unsigned char
   int* pa = reinterpret_cast<int*>(rs + np);  // [np] pair members
   int* pb = pa + np;
   __shared__ float red[2][32];
-  __shared__ double big[32];
-  // scaled by the power of two that brings the largest entry into [0.5, 1): FP32 then holds
-  // the entries and the sums of their squares whatever the unit of H, and the rotations,
-  // which are free of the scale, keep their bits
-  double most = 0.0;
-  for (int e = tid; e < B * B; e += nt) most = fmax(most, fabs(w.C[e]));
-  for (int o = 16; o > 0; o >>= 1) most = fmax(most, __shfl_xor_sync(0xffffffffu, most, o));
+  __shared__ int big[32];
+  // scaled by the power of two that brings the largest entry to about one: FP32 then holds the
+  // entries and the sums of their squares whatever the unit of H, and the rotations, which
+  // are free of the scale, keep their bits.  (High words: they order like the magnitudes, and
+  // the FP64 pipe is left alone.)
+  int most = 0;
+  for (int e = tid; e < B * B; e += nt) most = max(most, __double2hiint(w.C[e]) & 0x7fffffff);
+  most = __reduce_max_sync(0xffffffffu, most);
   if (tid % 32 == 0) big[tid / 32] = most;
   __syncthreads();
-  for (int q = 0; q < nt / 32; ++q) most = fmax(most, big[q]);
-  int ex = 0;
-  if (most > 0.0 && most <= DBL_MAX) frexp(most, &ex);
+  for (int q = 0; q < nt / 32; ++q) most = max(most, big[q]);
+  const int ex = most >> 20;  // biased exponent; 2047: not finite, 0: zero (or nearly)
+  const bool scaled = ex > 0 && ex < 2047;
+  const double half = scaled ? ldexp(0.5, 1023 - max(ex, 24)) : 0.5;
   for (int e = tid; e < Bp * Bp; e += nt) {
     const int r = e % Bp, c = e / Bp;
     C[r + (size_t)c * ld] =
-        r < B && c < B ? (float)ldexp(0.5 * (w.C[r + (size_t)c * B] + w.C[c + (size_t)r * B]), -ex) : 0.f;
+        r < B && c < B ? (float)(half * (w.C[r + (size_t)c * B] + w.C[c + (size_t)r * B])) : 0.f;
   }
   // the blocks of this thread, the same in every round (pairs k <= l)
   constexpr int kItems = 4;

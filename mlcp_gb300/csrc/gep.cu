@@ -10,13 +10,21 @@
 //    parallel cyclic Jacobi in FP32, then refined in FP64 by iterations of
 //    matrix products (Ogita and Aishima, Japan J. Indust. Appl. Math. 35
 //    (2018) 1007-1035): with G = V^T V and S = V^T C V,
-//      lambda_i = S_ii / G_ii,
-//      E_ij = (S_ij - lambda_j G_ij) / (lambda_j - lambda_i),  E_ii = (1 - G_ii) / 2,
+//      lambda_i = S_ii / G_ii,  m = (lambda_i + lambda_j) / 2,
+//      E_ij = (S_ij - m G_ij) / (lambda_j - lambda_i) - G_ij / 2,  E_ii = (1 - G_ii) / 2,
 //      V <- V + V E,
-//    which squares the error of V each time.  Pairs whose |E_ij| would pass
-//    1e-3 (levels nearly degenerate on the scale of the FP32 error) are first
-//    separated by FP64 Jacobi rotations of those pairs alone, so three
-//    iterations end at the rounding level for any spectrum.  The FP64 stage
+//    which squares the error of V each time.  The quotient is antisymmetric to the
+//    last bit, so nearly equal levels cannot cost orthogonality through its rounding.  Pairs
+//    whose quotient would pass a bound (1e-3, 1e-5, 1e-8 in the three iterations) are
+//    rotated apart first, by FP64 Jacobi rotations of those pairs alone: a level close to
+//    another on the scale of the FP32 error in the first iteration, on the scale of the
+//    couplings of second order through third levels, which the iteration before
+//    has left, in the others.  Rotations are orthogonal whatever their angle, so after
+//    the last iteration V is off by the square of 1e-8.  A pair above the bound whose coupling
+//    is below 2^-51 of the largest level is left as it is: that is rounding.  On shells
+//    of equal levels split by 1e-6 to 1e-14, on several scales at once, residuals and
+//    orthogonality end at a few eps (with one separation at 1e-3, in the first
+//    iteration only, they ended at 1e-11).  The FP64 stage
 //    matters: the vector updates combine the block with the eigenvectors,
 //    and for nearly degenerate states (the benchmark block has relative gaps
 //    of 4e-5) FP32 eigenvectors are off by ~1e-7 / gap, which moved the
@@ -33,6 +41,7 @@
 // Jacobi rounds are 0.78, the Cholesky 0.28, the three triangular solves 0.21,
 // the rotation replay 0.10 and the twelve matrix products 0.18.
 #include <algorithm>
+#include <cfloat>
 
 #include "common.cuh"
 #include "intertwine.cuh"
@@ -153,14 +162,20 @@ constexpr int kMaxQ = kMaxB / 32;   // rows per lane of a warp-held column
 constexpr int kJacobiSweeps = 30;
 constexpr int kVRows = 4;           // rows of V per CTA of the rotation replay
 constexpr int kReplay = 8;          // rounds of rotations loaded together
-constexpr double kUnsafe = 1.0e-3;  // pairs with |E_ij| above this are separated by rotations first
+constexpr int kIterations = 3;      // of the refinement
+constexpr int kSeparateSweeps = 40;
+// Pairs whose quotient is above this are separated by rotations first.
+__host__ __device__ constexpr double unsafe_bound(int iteration) {
+  return iteration == 0 ? 1.0e-3 : iteration == 1 ? 1.0e-5 : 1.0e-8;
+}
 
 // Workspace of the phases (doubles): L, L^T, C, W, V, V', G, S, E [B][B];
 // invd [B]; the FP32 Jacobi's rotations; counters.
 struct GepWork {
   double *L, *LT, *C, *W, *V, *V2, *G, *S, *E, *invd;
+  double* floor;  // [1] couplings that are rounding: 2^-51 of the largest level
   float2* rot;  // [sweeps][Bp - 1][Bp / 2] (c, s)
-  int* cnt;     // [0] Jacobi sweeps, [1] unsafe pairs seen
+  int* cnt;     // [0] Jacobi sweeps, [1] unsafe pairs seen in this iteration
 };
 
 __host__ __device__ inline int gep_pad(int B) { return (B + 1) / 2 * 2; }
@@ -183,6 +198,7 @@ __host__ __device__ inline size_t gep_carve(int B, double* base, GepWork* w) {
   w->S = take(bb);
   w->E = take(bb);
   w->invd = take(B);
+  w->floor = take(1);
   w->rot = reinterpret_cast<float2*>(take((size_t)kJacobiSweeps * (Bp - 1) * (Bp / 2)));
   w->cnt = reinterpret_cast<int*>(take(1));
   return o;
@@ -352,7 +368,7 @@ __device__ void phase_jacobi(const GepParams& p, const GepWork& w, unsigned char
   for (int q = 0; q < nt / 32; ++q) most = max(most, big[q]);
   const int ex = most >> 20;  // biased exponent; 2047: not finite, 0: zero (or nearly)
   const bool scaled = ex > 0 && ex < 2047;
-  const double half = scaled ? ldexp(0.5, 1023 - max(ex, 24)) : 0.5;
+  const double half = scaled ? ldexp(0.5, 1023 - max(ex, 24)) : 0.5, unit = scaled ? ldexp(1.0, max(ex, 24) - 1023) : 1.0;
   for (int e = tid; e < Bp * Bp; e += nt) {
     const int r = e % Bp, c = e / Bp;
     C[r + (size_t)c * ld] =
@@ -442,7 +458,17 @@ __device__ void phase_jacobi(const GepParams& p, const GepWork& w, unsigned char
       __syncthreads();
     }
   }
-  if (tid == 0) w.cnt[0] = sweep;
+  float top = 0.f;
+  for (int i = tid; i < B; i += nt) top = fmaxf(top, fabsf(C[i + (size_t)i * ld]));
+  for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+  __syncthreads();
+  if (tid % 32 == 0) red[0][tid / 32] = top;
+  __syncthreads();
+  if (tid == 0) {
+    for (int q = 1; q < nt / 32; ++q) top = fmaxf(top, red[0][q]);
+    *w.floor = (double)top * unit * (2.0 * DBL_EPSILON);
+    w.cnt[0] = sweep;
+  }
 }
 
 // V = the product of the recorded rotations, kVRows rows per CTA in shared
@@ -522,96 +548,143 @@ __device__ void phase_product(const double* X, const double* Y, double* out, int
   }
 }
 
-// E of one iteration; `first` records pairs that need a rotation instead.
-__device__ void phase_correction(const GepWork& w, int B, bool first, int cta, int ncta) {
+// The coupling of levels i and j in the metric G, S_ij - (lambda_i + lambda_j) / 2 G_ij.
+__device__ __forceinline__ double coupling(double sij, double sji, double gij, double li, double lj) {
+  return 0.5 * (sij + sji) - 0.5 * (li + lj) * gij;
+}
+
+// E_ij of one iteration from the coupling and the levels; *unsafe: the pair wants a rotation.
+__device__ __forceinline__ double correction(double num, double gap, double gij, double bound, double floor, bool* unsafe) {
+  double x = -0.5 * gij;
+  *unsafe = false;
+  if (fabs(num) <= bound * fabs(gap) && gap != 0.0) x += num / gap;
+  else if (fabs(num) > floor) *unsafe = true;
+  return x;
+}
+
+// E of iteration `it`; records in cnt[1] that there are pairs to be separated.
+__device__ void phase_correction(const GepWork& w, int B, int it, int cta, int ncta) {
+  const double bound = unsafe_bound(it), floor = *w.floor;
   for (int e = cta * blockDim.x + threadIdx.x; e < B * B; e += ncta * blockDim.x) {
     const int i = e % B, j = e / B;
     const double g = w.G[e];
-    double x = 0.5 * ((i == j ? 1.0 : 0.0) - g);
-    if (i != j) {
-      const double sii = w.S[i + (size_t)i * B], sjj = w.S[j + (size_t)j * B];
-      const double li = sii / w.G[i + (size_t)i * B], lj = sjj / w.G[j + (size_t)j * B];
-      const double num = 0.5 * (w.S[e] + w.S[j + (size_t)i * B]) - lj * g, gap = lj - li;
-      if (fabs(num) <= kUnsafe * fabs(gap) && gap != 0.0) {
-        x = num / gap;
-      } else if (first && fabs(num) > 1e-15 * fmax(fabs(li), fabs(lj))) {
-        w.cnt[1] = 1;
-      }
+    if (i == j) {
+      w.E[e] = 0.5 * (1.0 - g);
+      continue;
     }
-    w.E[e] = x;
+    const double li = w.S[i + (size_t)i * B] / w.G[i + (size_t)i * B], lj = w.S[j + (size_t)j * B] / w.G[j + (size_t)j * B];
+    bool unsafe;
+    w.E[e] = correction(coupling(w.S[e], w.S[j + (size_t)i * B], g, li, lj), lj - li, g, bound, floor, &unsafe);
+    if (unsafe) w.cnt[1] = 1;
   }
 }
 
-// The separation of unsafe pairs (one CTA; nothing to do unless cnt[1]): cyclic
-// Jacobi sweeps in FP64 that rotate only those pairs, S in shared memory,
-// V in global memory; then E from the rotated S (V is orthonormal here, G = I).
-__device__ void phase_separate(const GepWork& w, int B, unsigned char* smem) {
-  if (w.cnt[1] == 0) return;
-  const int Bp = gep_pad(B), np = Bp / 2, tid = threadIdx.x, nt = blockDim.x;
+// The separation of unsafe pairs (one CTA; nothing to do unless cnt[1]): cyclic Jacobi
+// sweeps in FP64 that rotate only those pairs, S and the levels in shared memory, G and V
+// in global memory, until no pair is unsafe; then E from the rotated S and G.  A sweep
+// looks at every pair first and visits only the rounds that hold an unsafe one.
+__device__ void phase_separate(const GepWork& w, int B, int it, unsigned char* smem) {
+  const bool any = w.cnt[1] != 0;
+  __syncthreads();  // read by all before it is cleared
+  if (!any) return;
+  const int Bp = gep_pad(B), np = Bp / 2, m = Bp - 1, tid = threadIdx.x, nt = blockDim.x;
+  const double bound = unsafe_bound(it), floor = *w.floor;
   double* S = reinterpret_cast<double*>(smem);  // [B][B]
-  double* rc = S + (size_t)B * B;               // [np] cosines, then [np] sines
+  double* lev = S + (size_t)B * B;              // [B] the levels S_ii / G_ii
+  double* rc = lev + B;                         // [np] cosines, then [np] sines
   double* rs = rc + np;
+  int* round_hit = reinterpret_cast<int*>(rs + np);  // [Bp] rounds with an unsafe pair
   for (int e = tid; e < B * B; e += nt) {
     const int i = e % B, j = e / B;
     S[e] = 0.5 * (w.S[e] + w.S[j + (size_t)i * B]);
   }
   __syncthreads();
-  for (int sweep = 0; sweep < 12; ++sweep) {
-    bool any = false;
-    for (int round = 0; round < Bp - 1; ++round) {
-      bool mine = false;
+  for (int i = tid; i < B; i += nt) lev[i] = S[i + (size_t)i * B] / w.G[i + (size_t)i * B];
+  for (int sweep = 0; sweep < kSeparateSweeps; ++sweep) {
+    for (int r = tid; r < Bp; r += nt) round_hit[r] = 0;
+    __syncthreads();
+    bool mine = false;
+    for (int e = tid; e < B * B; e += nt) {
+      const int i = e % B, j = e / B;
+      if (i >= j) continue;
+      bool unsafe;
+      correction(coupling(S[e], S[e], w.G[e], lev[i], lev[j]), lev[j] - lev[i], w.G[e], bound, floor, &unsafe);
+      if (!unsafe) continue;
+      mine = true;
+      // the round of robin_pair that holds (i, j): j = m meets i in round i, else the
+      // round's double is i + j modulo the odd m
+      const int sum = i + j;
+      round_hit[j == m ? i : (sum % 2 ? sum + m : sum) / 2 % m] = 1;
+    }
+    if (!__syncthreads_or(mine)) break;
+    for (int round = 0; round < m; ++round) {
+      if (!round_hit[round]) continue;
       for (int k = tid; k < np; k += nt) {
         int a, b;
         robin_pair(Bp, round, k, &a, &b);
         double c = 1.0, s = 0.0;
         if (b < B) {  // index Bp - 1 = B is padding when B is odd
-          const double app = S[a + (size_t)a * B], aqq = S[b + (size_t)b * B], apq = S[a + (size_t)b * B];
-          if (fabs(apq) > kUnsafe * fabs(aqq - app) && fabs(apq) > 1e-16 * fmax(fabs(app), fabs(aqq))) {
-            const double theta = (aqq - app) / (2.0 * apq);
+          const size_t ab = a + (size_t)b * B;
+          const double num = coupling(S[ab], S[ab], w.G[ab], lev[a], lev[b]), gap = lev[b] - lev[a];
+          bool unsafe;
+          correction(num, gap, w.G[ab], bound, floor, &unsafe);
+          if (unsafe) {
+            const double theta = gap / (2.0 * num);
             const double t = copysign(1.0, theta) / (fabs(theta) + sqrt(theta * theta + 1.0));
             c = 1.0 / sqrt(t * t + 1.0);
             s = t * c;
-            mine = true;
           }
         }
         rc[k] = c;
         rs[k] = s;
       }
-      if (!__syncthreads_or(mine)) continue;
-      any = true;
-      for (int e = tid; e < np * B; e += nt) {  // rows: S <- J^T S
+      __syncthreads();
+      auto rotate = [&](double* x, double* y, int k) {
+        const double c = rc[k], s = rs[k], xa = *x, xb = *y;
+        *x = c * xa - s * xb;
+        *y = s * xa + c * xb;
+      };
+      for (int e = tid; e < np * B; e += nt) {  // rows: S <- J^T S, G <- J^T G
         const int k = e / B, col = e % B;
+        if (rs[k] == 0.0) continue;
         int a, b;
         robin_pair(Bp, round, k, &a, &b);
-        const double c = rc[k], s = rs[k];
-        if (b >= B || s == 0.0) continue;
-        const double xa = S[a + (size_t)col * B], xb = S[b + (size_t)col * B];
-        S[a + (size_t)col * B] = c * xa - s * xb;
-        S[b + (size_t)col * B] = s * xa + c * xb;
+        rotate(S + a + (size_t)col * B, S + b + (size_t)col * B, k);
+        rotate(w.G + a + (size_t)col * B, w.G + b + (size_t)col * B, k);
       }
       __syncthreads();
-      for (int e = tid; e < np * B; e += nt) {  // columns: S <- S J, V <- V J
+      for (int e = tid; e < np * B; e += nt) {  // columns: S <- S J, G <- G J, V <- V J
         const int k = e / B, row = e % B;
+        if (rs[k] == 0.0) continue;
         int a, b;
         robin_pair(Bp, round, k, &a, &b);
-        const double c = rc[k], s = rs[k];
-        if (b >= B || s == 0.0) continue;
-        const double xa = S[row + (size_t)a * B], xb = S[row + (size_t)b * B];
-        S[row + (size_t)a * B] = c * xa - s * xb;
-        S[row + (size_t)b * B] = s * xa + c * xb;
-        const double va = w.V[row + (size_t)a * B], vb = w.V[row + (size_t)b * B];
-        w.V[row + (size_t)a * B] = c * va - s * vb;
-        w.V[row + (size_t)b * B] = s * va + c * vb;
+        rotate(S + row + (size_t)a * B, S + row + (size_t)b * B, k);
+        rotate(w.G + row + (size_t)a * B, w.G + row + (size_t)b * B, k);
+        rotate(w.V + row + (size_t)a * B, w.V + row + (size_t)b * B, k);
+      }
+      __syncthreads();
+      for (int k = tid; k < np; k += nt) {
+        if (rs[k] == 0.0) continue;
+        int a, b;
+        robin_pair(Bp, round, k, &a, &b);
+        lev[a] = S[a + (size_t)a * B] / w.G[a + (size_t)a * B];
+        lev[b] = S[b + (size_t)b * B] / w.G[b + (size_t)b * B];
       }
       __syncthreads();
     }
-    if (!any) break;
   }
   for (int e = tid; e < B * B; e += nt) {
-    const int i = e % B, j = e / B;
-    const double gap = S[j + (size_t)j * B] - S[i + (size_t)i * B];
-    w.E[e] = (i != j && fabs(S[e]) <= kUnsafe * fabs(gap) && gap != 0.0) ? S[e] / gap : 0.0;
+    const int i = e % B, j = e / B, f = j + i * B;
+    const double g = 0.5 * (w.G[e] + w.G[f]);  // equal in (i, j) and (j, i), as S is below: E's antisymmetry
+    if (i == j) {
+      w.E[e] = 0.5 * (1.0 - g);
+      w.S[e] = S[e];  // the levels of phase_finish
+      continue;
+    }
+    bool unsafe;
+    w.E[e] = correction(coupling(S[e], S[f], g, lev[i], lev[j]), lev[j] - lev[i], g, bound, floor, &unsafe);
   }
+  if (tid == 0) w.cnt[1] = 0;
 }
 
 // X = L^-T V with unit columns of V; eigenvalues; ascending order; signs.  One
@@ -677,15 +750,15 @@ __device__ void phase_finish(const GepParams& p, const GepWork& w, int cta, int 
   }
 }
 
-// The refinement iterations, in order: G = V^T V and W = C V; S = V^T W; E;
-// (first: the separation); V' = V + V E.  V and V' alternate, starting
+// The refinement iterations, in order: G = V^T V and W = C V; S = V^T W; E; the
+// separation where E asks for it; V' = V + V E.  V and V' alternate, starting
 // from V2 after the Newton step.
 enum Phase : int {
-  kCholesky, kReduce1, kReduce2, kJacobi, kReplayV, kGram0, kNewtonV, kGramApply, kProject, kCorrect1, kSeparate,
-  kCorrect, kUpdate, kFinish
+  kCholesky, kReduce1, kReduce2, kJacobi, kReplayV, kGram0, kNewtonV, kGramApply, kProject, kCorrect, kSeparate,
+  kUpdate, kFinish
 };
 
-__device__ void run_phase(const GepParams& p, const GepWork& w, int ph, unsigned char* smem, int cta, int ncta) {
+__device__ void run_phase(const GepParams& p, const GepWork& w, int ph, int it, unsigned char* smem, int cta, int ncta) {
   const int B = p.nbloc, nb = (B + kTile - 1) / kTile;
   switch (ph) {
     case kCholesky: phase_cholesky(p, w, smem); break;
@@ -701,29 +774,28 @@ __device__ void run_phase(const GepParams& p, const GepWork& w, int ph, unsigned
         phase_product(w.C, w.V, w.W, B, false, kPlain, ncta == 1 ? 0 : cta - nb * nb, ncta == 1 ? 1 : nb * nb, smem);
       break;
     case kProject: phase_product(w.V, w.W, w.S, B, true, kPlain, cta, ncta, smem); break;
-    case kCorrect1: phase_correction(w, B, true, cta, ncta); break;
-    case kSeparate: phase_separate(w, B, smem); break;
-    case kCorrect: phase_correction(w, B, false, cta, ncta); break;
+    case kCorrect: phase_correction(w, B, it, cta, ncta); break;
+    case kSeparate: phase_separate(w, B, it, smem); break;
     case kUpdate: phase_product(w.V, w.E, w.V2, B, false, kAdd, cta, ncta, smem); break;
     case kFinish: phase_finish(p, w, cta, ncta); break;
   }
 }
 
-// The sequence of phases; `swap` after a phase exchanges V and V'.
+// The sequence of phases; `swap` after a phase exchanges V and V'; `it` the iteration.
 struct Step {
   Phase phase;
   bool swap;
+  int it;
 };
-constexpr int kNumSteps = 21;
+constexpr int kBefore = 7, kPerIteration = 5;  // steps before the iterations, and of each
+constexpr int kNumSteps = kBefore + kPerIteration * kIterations + 1;
 __host__ __device__ inline Step step_at(int q) {
-  constexpr Step seq[kNumSteps] = {
-      {kCholesky, false}, {kReduce1, false}, {kReduce2, false}, {kJacobi, false}, {kReplayV, false},
-      {kGram0, false}, {kNewtonV, true},
-      {kGramApply, false}, {kProject, false}, {kCorrect1, false}, {kSeparate, false}, {kUpdate, true},
-      {kGramApply, false}, {kProject, false}, {kCorrect, false}, {kUpdate, true},
-      {kGramApply, false}, {kProject, false}, {kCorrect, false}, {kUpdate, true},
-      {kFinish, false}};
-  return seq[q];
+  constexpr Phase before[kBefore] = {kCholesky, kReduce1, kReduce2, kJacobi, kReplayV, kGram0, kNewtonV};
+  constexpr Phase each[kPerIteration] = {kGramApply, kProject, kCorrect, kSeparate, kUpdate};
+  if (q < kBefore) return Step{before[q], before[q] == kNewtonV, 0};
+  if (q == kNumSteps - 1) return Step{kFinish, false, 0};
+  const Phase ph = each[(q - kBefore) % kPerIteration];
+  return Step{ph, ph == kUpdate, (q - kBefore) / kPerIteration};
 }
 
 __device__ inline void swap_v(GepWork& w) {
@@ -734,14 +806,14 @@ __device__ inline void swap_v(GepWork& w) {
 
 }  // namespace
 
-// One phase per launch (swapped: V and V' exchanged).
+// One phase per launch (swapped: V and V' exchanged; it: the iteration).
 template <int kPhase>
-__global__ void __launch_bounds__(1024) gep_phase_kernel(GepParams p, int swapped) {
+__global__ void __launch_bounds__(1024) gep_phase_kernel(GepParams p, int swapped, int it) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   GepWork w;
   gep_carve(p.nbloc, p.work, &w);
   if (swapped) swap_v(w);
-  run_phase(p, w, kPhase, smem_raw, blockIdx.x, gridDim.x);
+  run_phase(p, w, kPhase, it, smem_raw, blockIdx.x, gridDim.x);
 }
 
 // Every phase in one CTA of 64 threads, for blocks so small that the
@@ -752,7 +824,7 @@ __global__ void __launch_bounds__(64) gep_small_kernel(GepParams p) {
   gep_carve(p.nbloc, p.work, &w);
   for (int q = 0; q < kNumSteps; ++q) {
     const Step st = step_at(q);
-    run_phase(p, w, st.phase, smem_raw, 0, 1);
+    run_phase(p, w, st.phase, st.it, smem_raw, 0, 1);
     __syncthreads();
     if (st.swap) swap_v(w);
   }
@@ -782,11 +854,11 @@ int gep_launch(const GepParams& p, cudaStream_t st) {
 namespace {
 
 template <int kPhase>
-int launch_phase(const GepParams& p, int swapped, int grid, int threads, size_t smem, cudaStream_t st) {
+int launch_phase(const GepParams& p, int swapped, int grid, int threads, size_t smem, cudaStream_t st, int it = 0) {
   if (smem > 48 * 1024)
     MLCP_CUDA_TRY(
         cudaFuncSetAttribute(gep_phase_kernel<kPhase>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  gep_phase_kernel<kPhase><<<grid, threads, smem, st>>>(p, swapped);
+  gep_phase_kernel<kPhase><<<grid, threads, smem, st>>>(p, swapped, it);
   MLCP_CUDA_TRY(cudaGetLastError());
   return kOk;
 }
@@ -802,9 +874,10 @@ constexpr int kSmallBlock = 8;
 int gep_solve_launch(const GepParams& p, cudaStream_t st) {
   const int B = p.nbloc, Bp = gep_pad(B), np = Bp / 2, nb = (B + kTile - 1) / kTile;
   const size_t s_chol = sizeof(double) * ((size_t)B * B + Bp), s_prod = sizeof(double) * 2 * kTile * (kChunk + 1),
-               s_jac = sizeof(float) * ((size_t)Bp * (Bp + 1) + 4 * np), s_rep = sizeof(float) * kVRows * Bp;
+               s_jac = sizeof(float) * ((size_t)Bp * (Bp + 1) + 4 * np), s_rep = sizeof(float) * kVRows * Bp,
+               s_sep = sizeof(double) * ((size_t)B * B + B + 2 * np) + sizeof(int) * Bp;
   if (B <= kSmallBlock) {
-    const size_t smem = std::max(std::max(s_chol, s_prod), std::max(s_jac, s_rep));
+    const size_t smem = std::max(std::max(std::max(s_chol, s_prod), std::max(s_jac, s_rep)), s_sep);
     gep_small_kernel<<<1, 64, smem, st>>>(p);
     MLCP_CUDA_TRY(cudaGetLastError());
     return kOk;
@@ -824,9 +897,8 @@ int gep_solve_launch(const GepParams& p, cudaStream_t st) {
       case kNewtonV: rc = launch_phase<kNewtonV>(p, swapped, nb * nb, 64, s_prod, st); break;
       case kGramApply: rc = launch_phase<kGramApply>(p, swapped, 2 * nb * nb, 64, s_prod, st); break;
       case kProject: rc = launch_phase<kProject>(p, swapped, nb * nb, 64, s_prod, st); break;
-      case kCorrect1: rc = launch_phase<kCorrect1>(p, swapped, (B * B + 127) / 128, 128, 0, st); break;
-      case kSeparate: rc = launch_phase<kSeparate>(p, swapped, 1, 1024, s_chol, st); break;
-      case kCorrect: rc = launch_phase<kCorrect>(p, swapped, (B * B + 127) / 128, 128, 0, st); break;
+      case kCorrect: rc = launch_phase<kCorrect>(p, swapped, (B * B + 127) / 128, 128, 0, st, step.it); break;
+      case kSeparate: rc = launch_phase<kSeparate>(p, swapped, 1, 1024, s_sep, st, step.it); break;
       case kUpdate: rc = launch_phase<kUpdate>(p, swapped, nb * nb, 64, s_prod, st); break;
       case kFinish: rc = launch_phase<kFinish>(p, swapped, B, 32, 0, st); break;
     }

@@ -693,10 +693,11 @@ __device__ void phase_finish(const GepParams& p, const GepWork& w, int cta, int 
   const int B = p.nbloc, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   for (int c = cta * nw + (threadIdx.x >> 5); c < B; c += ncta * nw) {
     const double lam = w.S[c + (size_t)c * B] / w.G[c + (size_t)c * B];
-    int pos = 0;  // place of this eigenvalue, ties by column
+    int pos = 0;  // place of this eigenvalue, ties by column, NaN last: every place is taken once
     for (int k = lane; k < B; k += 32) {
       const double o = w.S[k + (size_t)k * B] / w.G[k + (size_t)k * B];
-      pos += (o < lam) || (o == lam && k < c);
+      const bool same = o == lam || (isnan(o) && isnan(lam));
+      pos += o < lam || (!isnan(o) && isnan(lam)) || (same && k < c);
     }
     for (int o = 16; o > 0; o >>= 1) pos += __shfl_xor_sync(0xffffffffu, pos, o);
     double x[kMaxQ], den = 0.0;

@@ -750,10 +750,11 @@ __device__ __forceinline__ dw lane_sum(dw v) {
   return acc_value(a);
 }
 
-// One correction of correct_inverse: *big = n max |I - Iv A| before it.
+// One correction of correct_inverse: *big = n max |I - Iv A| before it; none when that is
+// above `most`.
 template <int RT, bool kFirst>
 __device__ __forceinline__ bool correct_round(const dw* A, int n_, const float* gi, dw* Iv, float* Ef, float* emax,
-                                              float* big) {
+                                              float most, float* big) {
   constexpr int NE = kRowRank * kRowRank / kSolverThreads;
   const int n = RT ? RT : n_, nn = n * n, t = threadIdx.x, lane = t & 31;
   int i[NE], k[NE];
@@ -783,7 +784,7 @@ __device__ __forceinline__ bool correct_round(const dw* A, int n_, const float* 
   if (lane == 0) emax[t >> 5] = __int_as_float(mx);
   solver_sync();
   *big = n * __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(emax[lane & (kSolverWarps - 1)])));
-  if (!(*big <= (kFirst ? 3e-3f : 1e-5f))) return false;
+  if (!(*big <= most)) return false;
   float d[NE] = {};
 #pragma unroll 4
   for (int l = 0; l < n; ++l)
@@ -801,18 +802,33 @@ __device__ __forceinline__ bool correct_round(const dw* A, int n_, const float* 
 
 // Iv = A^-1 in double-word (threads 0 .. 127, n <= 16; RT: n when known at compile
 // time, else 0): the FP32 inverse gi corrected by Iv += (I - Iv A) Iv (Schulz's iteration, the
-// residual in double-word) until n max |I - Iv A| was at most 1e-5 before a
-// correction, so 1e-10 after it (what refine_solve reaches for its right-hand sides), in
-// two corrections at most; false when that does not suffice.  The left residual is taken
-// so that a solution Iv b has an error of (residual)^2 |x| and (rounding) cond |x|.
-// Ef: [n n], emax: [4] floats.  Ends without a barrier.
+// residual in double-word).  The first correction squares the residual; the product of a
+// correction is FP32, so each later one shrinks it by about the first one's size e0 (the
+// FP32 rounding of gi times the condition of A).  Corrections end when the residual e before
+// the last has e e0 <= 1e-10, which is then about what it leaves; false when kCorrections do
+// not suffice, when the residual does not shrink, or when e0 is above kCorrectable.  The left
+// residual is taken so that a solution Iv b has an error of (residual)^2 |x| and (rounding)
+// cond |x|.  Ef: [n n], emax: [4] floats.  Ends without a barrier.
+//
+// kCorrectable is where these solutions stay as good as those of refine_solve or, where that
+// gives up, of the LDL^T (random systems of 8 and 16 rows with unit diagonal, condition 1e4 to
+// 3e5: errors up to 7e-10 of the solution, at most 2.7 times theirs; 8 times with 2e-2), and it
+// takes as many systems as refine_solve.  With 3e-3 and two corrections most of those of
+// condition 3e4 went to the LDL^T: 28.6 k cycles for 16 rows against 5.9 k with three
+// corrections and 6.8 to 8.5 k with the right-hand sides refined.
+constexpr int kCorrections = 5;
+constexpr float kCorrectable = 1.5e-2f;  // n max |I - gi A| up to which the corrections are tried
 template <int RT>
 __device__ inline bool correct_inverse(const dw* A, int n, const float* gi, dw* Iv, float* Ef, float* emax) {
-  float big;
-  if (!correct_round<RT, true>(A, n, gi, Iv, Ef, emax, &big)) return false;
-  if (big <= 1e-5f) return true;
-  solver_sync();
-  return correct_round<RT, false>(A, n, gi, Iv, Ef, emax, &big);
+  float first;
+  if (!correct_round<RT, true>(A, n, gi, Iv, Ef, emax, kCorrectable, &first)) return false;
+  float big = first;
+  for (int round = 1; first * big > 1e-10f; ++round) {
+    if (round == kCorrections) return false;
+    solver_sync();
+    if (!correct_round<RT, false>(A, n, gi, Iv, Ef, emax, 0.25f * big, &big)) return false;
+  }
+  return true;
 }
 
 // A row of X = Iv B by one warp: iv points at the row (entries ld apart), B is [n][nj].

@@ -36,7 +36,7 @@
 //     soon as eight warps have written it, while the other fifteen refresh the
 //     overlaps (with the next mode's products, and the coefficients <Q_k, F> from
 //     those), form the right-hand side and exchange it;
-//   - the FP32 inverse is then corrected once (twice if need be) by
+//   - the FP32 inverse is then corrected once (more often if need be) by
 //     Inv += (I - Inv BB) Inv with the residual in double-word (Schulz's
 //     iteration), which leaves one product per right-hand side to the solve
 //     instead of refinement rounds on it.  The left residual is used: the error of

@@ -251,8 +251,7 @@ MLCP_API int mlcp_mlp_adam_layers(int count, void *const *t, const int *dims, fl
 /* One forward (backward = 0) or backward pass of the three-layer network
  * X -> H1 -> H2 -> Y (ReLU, ReLU, linear; mean squared error against T), all of
  * its launches from one call.  dims: padded rows, valid rows, padded input, hidden
- * and output widths, output width, row stride of X (the input width for
- * backward).  t: status, X, H1, H1 transposed, H2, H2
+ * and output widths, output width, row stride of X.  t: status, X, H1, H1 transposed, H2, H2
  * transposed, Y, then w and b of the layers 1 to 3 (BF16 weights); for
  * backward also T, loss, X transposed (written), dY, dY transposed, dZ2, dZ2
  * transposed, dZ1, dZ1 transposed, then the transposed weights and the gradients of

@@ -456,8 +456,8 @@ __global__ void __launch_bounds__(kTileThreads) mlp_adam_kernel(MlpAdam p) {
   }
 }
 
-// out[c][r] = in[r][c], BF16 (32 x 32 tiles).
-__global__ void __launch_bounds__(kTileThreads) mlp_transpose_kernel(const __nv_bfloat16* in, int rows, int cols,
+// out[c][r] = in[r][c], BF16, rows of `in` ld apart (32 x 32 tiles).
+__global__ void __launch_bounds__(kTileThreads) mlp_transpose_kernel(const __nv_bfloat16* in, int ld, int rows, int cols,
                                                                      __nv_bfloat16* out) {
   __shared__ __nv_bfloat16 tile[kTileDim][kTileDim + 2];
   const int tx = threadIdx.x % kTileDim, ty = threadIdx.x / kTileDim;
@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(kTileThreads) mlp_transpose_kernel(const __nv_
   const int r0 = blockIdx.x / across * kTileDim, c0 = blockIdx.x % across * kTileDim;
 #pragma unroll
   for (int u = 0; u < kTileDim; u += kTileThreads / kTileDim)
-    if (r0 + ty + u < rows && c0 + tx < cols) tile[ty + u][tx] = in[(size_t)(r0 + ty + u) * cols + c0 + tx];
+    if (r0 + ty + u < rows && c0 + tx < cols) tile[ty + u][tx] = in[(size_t)(r0 + ty + u) * ld + c0 + tx];
   __syncthreads();
 #pragma unroll
   for (int u = 0; u < kTileDim; u += kTileThreads / kTileDim)
@@ -531,7 +531,7 @@ int mlp_backward(const MlpStep& s, cudaStream_t st) {
   const int M = s.rows_p, h = s.h_p, o = s.out_p;
   MLCP_CUDA_TRY(cudaMemsetAsync(s.loss, 0, sizeof(float), st));
   if (int rc = mlp_loss_launch(s.Y, s.T, s.rows, s.out_dim, o, M, s.dY, s.dYt, s.loss, st)) return rc;
-  mlp_transpose_kernel<<<tile_count(M, s.in_p), kTileThreads, 0, st>>>(s.X, M, s.in_p, s.Xt);
+  mlp_transpose_kernel<<<tile_count(M, s.in_p), kTileThreads, 0, st>>>(s.X, s.ldx, M, s.in_p, s.Xt);
   MLCP_CUDA_TRY(cudaGetLastError());
   // layer 3: dW3 = dY^T H2, dZ2 = (dY W3) * (H2 > 0)
   MlpGemm g = gemm_of(s.dYt, M, s.H2t, M, o, h, M, o, s.status);

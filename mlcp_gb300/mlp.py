@@ -119,6 +119,8 @@ class Mlp:
         gw/gb.  Returns the loss (device scalar)."""
         if tuple(Xp.shape) != (self._rows, self.in_p):
             raise RuntimeError(f"inputs of shape {tuple(Xp.shape)}, the last forward's were {(self._rows, self.in_p)}")
+        if Xp.dtype != self.Xt.dtype or Xp.device != self.Xt.device or not Xp.is_contiguous():
+            Xp = Xp.to(device=self.dev, dtype=self.Xt.dtype).contiguous()
         more = [T, self.loss, self.Xt, self.dY, self.dYt, self.dZ2, self.dZ2t, self.dZ1, self.dZ1t]
         for Ly in self.layers:
             more += (Ly["wt"], Ly["gw"], Ly["gb"])

@@ -1,7 +1,7 @@
 """The warm-start network's backward pass on inputs that are not one contiguous BF16
-block: rows further apart than they are long, through mlcp_mlp_step.  The reference is the
-same pass on a packed copy: the values are the same, so the gradients are the same
-bits.
+block: rows further apart than they are long, through mlcp_mlp_step, and tensors of another
+order, type or device, through Mlp.backward.  The reference is the same pass on a packed
+copy: the values are the same, so the gradients are the same bits.
 """
 import ctypes
 
@@ -49,5 +49,21 @@ def test_row_stride_of_the_inputs(rows, extra, cuda_device):
         more += (Ly["wt"], Ly["gw"], Ly["gb"])
     step(net, 0, wide, wide.shape[1], rows)
     step(net, 1, wide, wide.shape[1], rows, *more)
+    for a, b in zip(expected, gradients(net)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["columns first", "FP32", "every other row", "host"])
+def test_backward_takes_any_tensor_of_the_inputs(form, cuda_device):
+    rows = 100
+    net, X, T = network(rows, cuda_device)
+    net.forward(X, rows)
+    net.backward(X, rows, T)
+    expected = gradients(net)
+    other = {"columns first": lambda: X.t().contiguous().t(), "FP32": X.float, "host": X.cpu,
+             "every other row": lambda: X.repeat_interleave(2, 0)[::2]}[form]()
+    assert other.shape == X.shape
+    net.backward(other, rows, T)
     for a, b in zip(expected, gradients(net)):
         assert torch.equal(a, b)

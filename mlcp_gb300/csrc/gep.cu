@@ -833,7 +833,7 @@ __global__ void __launch_bounds__(64) gep_small_kernel(GepParams p) {
 
 size_t gep_work_doubles(int nbloc) {
   GepWork w;
-  return gep_carve(nbloc, nullptr, &w);
+  return nbloc > kMaxB ? 0 : gep_carve(nbloc, nullptr, &w);  // (larger blocks never get here)
 }
 
 int gep_launch(const GepParams& p, cudaStream_t st) {

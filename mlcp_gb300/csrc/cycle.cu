@@ -273,11 +273,12 @@ size_t plan_cycle(const Layout& Ly, const OpTable& t, int R, int B, CycleBuffers
   cb->hqc = (double*)take(sizeof(double) * vec);
   cb->qn = (double*)take(sizeof(double) * vec * Ly.nD);
   cb->qnc = (double*)take(sizeof(double) * vec);
-  cb->mscr = (dw*)take(sizeof(dw) * (size_t)B * t.utot * R * R);
-  cb->wscr = (dw*)take(sizeof(dw) * (size_t)B * t.umax * R * R);
-  cb->zscr = (dw*)take(sizeof(dw) * (size_t)B * t.utot * R * t.npmax);
-  cb->ogscr = (dw*)take(sizeof(dw) * opals_grid_dw(t, B));
-  cb->g64 = (double*)take(sizeof(double) * (size_t)B * Ly.D * R * R);
+  const size_t nv = opals_vectors(t, B);
+  cb->mscr = (dw*)take(sizeof(dw) * nv * t.utot * R * R);
+  cb->wscr = (dw*)take(sizeof(dw) * nv * t.umax * R * R);
+  cb->zscr = (dw*)take(sizeof(dw) * nv * t.utot * R * t.npmax);
+  cb->ogscr = (dw*)take(sizeof(dw) * opals_grid_dw(t, (int)nv));
+  cb->g64 = (double*)take(sizeof(double) * nv * Ly.D * R * R);
   cb->gsw = (double*)take(sizeof(double) * gs_work_doubles(B, R, Ly.nD, Ly.D, Ly.npmax));
   cb->A = (double*)take(sizeof(double) * (size_t)B * B);
   cb->S = (double*)take(sizeof(double) * (size_t)B * B);

@@ -59,17 +59,20 @@ struct OpAlsParams {
   const double* fo_coef;
   double* f_base;         // F output (may alias fo for POW)
   double* f_coef;
-  dw* mscr;               // [nvec][utot][R][R] operator Grams M = Fo^T h F
-  dw* wscr;               // [nvec][umax][R][R] grouped term products W
-  dw* zscr;               // [nvec][utot][R][npmax] h Fo_d
-  double* g64;            // [nvec][D][R][R] FP64 Grams of F
+  // scratch for nv = opals_vectors(ops, nvec) vectors
+  dw* mscr;               // [nv][utot][R][R] operator Grams M = Fo^T h F
+  dw* wscr;               // [nv][umax][R][R] grouped term products W
+  dw* zscr;               // [nv][utot][R][npmax] h Fo_d
+  double* g64;            // [nv][D][R][R] FP64 Grams of F
   int* status;            // [nvec]
-  dw* gscr;               // opals_grid_dw(ops, nvec): scratch of the grid form
+  dw* gscr;               // opals_grid_dw(ops, nv): scratch of the grid form
   int keep;               // one-CTA form: h_u Fo_j of every mode fits (set by opals_launch)
   const int* rank_v;      // [nvec] ranks <= R (terms beyond carry zero weight), or null: all R
 };
 
 int opals_launch(const OpAlsParams& p, cudaStream_t st);
+// Vectors whose scratch is held at once (the launches go over the block in parts of so many).
+int opals_vectors(const OpTable& t, int nvec);
 // Shared-memory footprint that a shape may not exceed.
 size_t opals_smem_bytes(const OpTable& t);
 // The grid form (opals_grid.cu) and its scratch entries.

@@ -31,6 +31,8 @@
 // are rescaled by a power of two after every mode step
 // (rescale_weights_warp), which keeps them in the FP32 exponent range of
 // the double-word values without changing the sweep's result.
+#include <algorithm>
+
 #include "common.cuh"
 #include "dword.cuh"
 #include "dwsolve.cuh"
@@ -333,7 +335,17 @@ size_t opals_smem_bytes(const OpTable& t) {
          sizeof(dw) * ((size_t)2 * t.R * t.nDp + (size_t)t.R * t.npmax + (size_t)t.R);
 }
 
-int opals_launch(const OpAlsParams& p, cudaStream_t st) {
+namespace {
+
+// Scratch that the vectors of one launch may take together.  The operator Grams, term products
+// and h Fo of a vector are 8 (utot (R^2 + R n) + umax R^2) bytes: 48 MB at rank 30 on six
+// modes of 48 functions and 400 operators each, so 16 GB are 360 such vectors, more than fill
+// the GPU.  (Held for a whole block, h Fo of every mode would halve the longest operator list
+// that 160 of them can have.)
+constexpr size_t kScratchBytes = (size_t)16 << 30;
+constexpr int kMaxVectors = 65535;  // gridDim.y and z of the grid form
+
+int launch_vectors(const OpAlsParams& p, cudaStream_t st) {
   int dev = 0, limit = 0;
   MLCP_CUDA_TRY(cudaGetDevice(&dev));
   MLCP_CUDA_TRY(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
@@ -351,6 +363,31 @@ int opals_launch(const OpAlsParams& p, cudaStream_t st) {
   MLCP_CUDA_TRY(cudaFuncSetAttribute(opals_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)res));
   opals_kernel<<<p.nvec, kThreads, res, st>>>(q);
   MLCP_CUDA_TRY(cudaGetLastError());
+  return kOk;
+}
+
+}  // namespace
+
+int opals_vectors(const OpTable& t, int nvec) {
+  const size_t per = sizeof(dw) * ((size_t)(t.utot + t.umax) * t.R * t.R + (size_t)t.utot * t.R * t.npmax);
+  return (int)std::max<size_t>(1, std::min<size_t>(std::min(nvec, kMaxVectors), kScratchBytes / per));
+}
+
+int opals_launch(const OpAlsParams& p, cudaStream_t st) {
+  const int most = opals_vectors(p.ops, p.nvec);
+  const size_t R = p.ops.R;
+  for (int v = 0; v < p.nvec; v += most) {
+    OpAlsParams q = p;
+    q.nvec = std::min(most, p.nvec - v);
+    q.fo_base += v * R * p.nD;
+    q.fo_coef += v * R;
+    q.f_base += v * R * p.nD;
+    q.f_coef += v * R;
+    q.status += v;
+    if (p.eshift_v) q.eshift_v += v;
+    if (p.rank_v) q.rank_v += v;
+    if (int rc = launch_vectors(q, st)) return rc;
+  }
   return kOk;
 }
 

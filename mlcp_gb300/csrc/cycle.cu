@@ -9,10 +9,13 @@
 //
 // Here: the block goes to the device once and comes back once; the operator
 // list is preprocessed once per distinct content (hash) and stays resident;
-// each phase is one launch over the whole block:
+// each phase works on the whole block:
 //   opals (POW_ALS, all vectors)  ->  gs (Gram-Schmidt)  ->
 //   opals (PRODHV_ALS, all vectors) -> gep (inner products, Rayleigh-Ritz) ->
-//   batched ALS with a shared target (vector updates) -> weight normalisation.
+//   upd (vector updates, weights normalised).
+// A small phase is one launch (a CTA or a cluster per vector, one cluster for the
+// Gram-Schmidt); a larger one is a few launches over the whole GPU for every mode step.  The
+// launches of a cycle are captured as a CUDA graph and replayed.
 #include <algorithm>
 #include <cstdio>
 #include <cmath>

@@ -311,8 +311,8 @@ __device__ inline bool gj_inverse_warp(const dw* A, int n, float* inv) {
 // same bits as there.  What it replaces is bound by latency: one warp takes
 // ~15 cycles per row and step (15.7 k cycles for n = 32), four warps through
 // two shared-memory matrices ~1600 cycles per step (100 k for n = 64); this
-// takes ~200 per step with four warps at n = 32 and eight at n = 64.  Writes
-// inv (column-major, ld n); *flag (set by the caller before a barrier) becomes 0
+// takes ~210 per step with four warps (8.3 k for n = 32) and ~500 with eight (33 k for
+// n = 64).  Writes inv (column-major, ld n); *flag (set by the caller before a barrier) becomes 0
 // when a pivot is not positive.  Ends without a barrier.
 template <int NW, int ROWS, int COLS, bool kColumn>
 __device__ inline void team_inverse(const dw* A, int n, float* inv, float* row, int* flag) {

@@ -37,9 +37,13 @@
 // sequential parts (Cholesky, the Jacobi rounds) are chains of barriers.  One
 // CTA that did everything in global memory, with FP64 Jacobi sweeps (and
 // 16-way bank conflicts in the FP32 ones), took 36.0 ms for 144 vectors and
-// 1.36 ms for 40; the phases take 1.6 ms and 0.39 ms.  Of the 1.6 ms the FP32
-// Jacobi rounds are 0.78, the Cholesky 0.28, the three triangular solves 0.21,
-// the rotation replay 0.10 and the twelve matrix products 0.18.
+// 1.36 ms for 40; the phases take 1.6 ms and 0.32 ms.  Of the 1.6 ms the FP32
+// Jacobi rounds are 0.78, the Cholesky 0.28, the three triangular solves 0.22,
+// the rotation replay 0.10 and the matrix products (eleven launches) 0.17; the three
+// separations are launches of 2 us while there is nothing to separate.  Clustered levels pay for
+// theirs: 40 levels in shells split by 1e-6 to 1e-12 0.6 to 1.9 ms more (2.1 to 2.6 ms in all when
+// FP64 sweeps rotated every pair, 1.2 to 2.5 now), 144 levels of two ladders split by 1e-5 to 1e-9
+// 7 to 11 ms more (74 to 84 in all then, 10 to 15 now).
 #include <algorithm>
 #include <cfloat>
 

@@ -656,8 +656,10 @@ int gs_level(const GsParams& p, int cl, int smem_max) {
   return -1;
 }
 
-// Shared memory that a shape may not exceed: its normal equations and inverse, a
-// mode's factor five times and a coefficient per chunk of the overlaps of nkm vectors.
+// Shared memory that a shape may not exceed: what one CTA of the form before these two needed of a
+// mode step (normal equations and two inverses, six right-hand sides, a coefficient per
+// chunk of the overlaps of nkm vectors, its reductions).  Kept as the limit on purpose: what
+// was refused stays refused, and both forms need less.
 size_t gs_core_bytes(int R, int D, int npm, int nkm) {
   const size_t RR = (size_t)R * R, Rn = (size_t)R * npm;
   size_t o = 0;
@@ -717,8 +719,8 @@ int gs_launch(const GsParams& prm, cudaStream_t st) {
 // A larger cluster spreads the earlier vectors over more CTAs but pays a
 // longer gather and cluster barrier at every mode step; which wins depends on
 // the block, and the grid form takes the blocks whose arrays 16 CTAs cannot hold
-// (measured on the 40-vector rank-16 block: 16 CTAs 27.7 ms per
-// cycle, 12 CTAs 28.7, 8 CTAs 31.2).  The first cycle of a block shape runs
+// (measured on the 40-vector rank-16 block, ten sweeps: 16 CTAs 13.7 ms,
+// 12 CTAs 14.1, 8 CTAs 15.5).  The first cycle of a block shape runs
 // one Gram-Schmidt sweep (nals = 1) twice with each candidate size on a
 // scratch copy of the block, times it with CUDA events on the cycle's stream
 // and caches the size of the fastest run for the process, per device and

@@ -33,16 +33,12 @@
 // 79 and 103 us.  Blocks of rank 16 that one cluster can hold are faster there (gs.cu): 5.7 and
 // 13 us for 40 vectors with 10 basis functions in 6 modes; the 250 vectors that it
 // cannot hold take 11.0 us (10.9 over several clusters).
-#include <cooperative_groups.h>
-
 #include <algorithm>
 
 #include "common.cuh"
 #include "dword.cuh"
 #include "dwsolve.cuh"
 #include "intertwine.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace mlcp {
 

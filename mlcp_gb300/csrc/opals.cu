@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(kThreads, 1) opals_kernel(OpAlsParams p) {
 }
 
 // F, Fo and one mode step: what both forms' callers check against the
-// device's limit (the grid form alone would need less).
+// device's limit.  (The grid form alone would need less; shapes beyond stay refused.)
 size_t opals_smem_bytes(const OpTable& t) {
   StepSmem m;
   return step_carve(m, nullptr, t.R, t.npmax) +

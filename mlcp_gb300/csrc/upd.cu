@@ -362,8 +362,10 @@ __global__ void __launch_bounds__(kThreads, 1) upd_kernel(UpdParams p) {
   }
 }
 
-// Shared memory that a shape may not exceed: the step's arrays, seven right-hand sides in
-// all, and the products and factors of sixteen block terms.
+// Shared memory that a shape may not exceed: what a CTA of the form before these two needed at
+// least (the step's arrays, six right-hand sides among them, and the products and factors of
+// sixteen block terms).  Kept as the limit on purpose: what was refused stays refused, and the
+// grid form needs less.
 size_t upd_smem_bytes(int R, int npm) {
   const size_t Rn = (size_t)R * npm, RR = (size_t)R * R;
   size_t o = 0;
